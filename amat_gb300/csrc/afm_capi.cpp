@@ -246,6 +246,11 @@ void free_device(afm_operator* op) {
     dfree(op, op->d_bc_val);
     dfree(op, op->d_bcmask);
     dfree(op, op->d_gbar);
+    dfree(op, op->d_gather_off);
+    dfree(op, op->d_gather_idx);
+    dfree(op, op->d_ve);
+    op->gather_b = 0;
+    op->ve_stream = nullptr;
     op->fused_ok = false;
     dfree(op, op->d_work);
     dfree(op, op->d_work32);
@@ -635,12 +640,109 @@ void build_segments(afm_operator* op, int prec) {
         s.map_offset = map_off;
         ke_off += s.unit_bytes * s.units;
         map_off += (uint64_t)s.units * (s.regime == REG_TPE ? kTpeWidth : 1) * s.n;
-        map_off = (map_off + 3) / 4 * 4;  // keep 16-byte alignment of each segment's map
+        // (maps are read word by word: no padding between segments, so the elements of a plan of one size are one
+        // contiguous range)
         op->segs.push_back(s);
         p = q;
     }
     op->ke_bytes = ke_off;
     op->map_bytes = map_off * sizeof(uint32_t);
+}
+
+// Whether one launch for every element plus the gather pass beats a launch
+// per colour. The gather pass costs its traffic (element products written and
+// read, lists read), a colour launch its ramp and tail, so the line is a
+// number of entries (elements x DoFs) per colour; and the products
+// (ve_bytes each) must stay in the 126 MB L2. Measured, colours -> gather:
+// 8-byte staged u (FP64, split): hex20 elasticity 12^3 27 -> 20 us, 32^3 188 ->
+// 172 (0.25 M entries per colour), 42^3 389 -> 377 (0.56 M), 48^3 556 -> 561
+// (0.83 M), 56^3 885 -> 897 (1.3 M); hex8 elasticity 16^3 45 -> 14 us, 48^3
+// 146 -> 123 (0.33 M), 56^3 211 -> 192 (0.53 M); tet10 elasticity 16^3 x 6 136
+// -> 49 us, 32^3 x 6 392 -> 320. FP32 products and inner formats, whose
+// element launches are shorter: hex8 elasticity 72^3 164 -> 142 us (1.1 M),
+// hex20 42^3 (format 4) 231 -> 204 (0.56 M), 56^3 (FP32) 305 -> 309 (1.3 M);
+// tet10 elasticity 44^3 x 6: FP32 349 -> 287 (61 MB of products), format 4
+// 618 -> 635 (123 MB).
+bool gather_pays(const afm_operator* op, bool wide, uint32_t ve_bytes) {
+    const uint64_t entries = (uint64_t)op->n_elem * op->nmax;
+    return entries / std::max<uint32_t>(op->n_colors, 1) <= (wide ? 700000u : 1200000u) &&
+           entries * ve_bytes <= 100000000u;
+}
+
+// Lists of the gather pass (launch_gather_sum) for a plan whose elements all
+// have n DoFs and no DoF twice: per DoF, or per node where the map lists whole
+// nodes of three consecutive DoFs, its entries in the element-product buffer
+// (position in the colour-sorted order x n + row) in ascending order, i.e. in
+// colour order: the order in which a launch per colour adds them to v, hence
+// the same bits. color_first: offsets of the colours in that order.
+int build_gather(afm_operator* op, uint32_t n, const std::vector<uint32_t>& color_first) {
+    const uint64_t entries = (uint64_t)op->n_elem * n;
+    if (entries == 0 || !gather_pays(op, false, 4)) return AFM_SUCCESS;
+    int nodes3 = n % 3 == 0 && op->n_dofs % 3 == 0;
+    if (nodes3) {
+#pragma omp parallel for schedule(static) reduction(&& : nodes3)
+        for (int64_t k = 0; k < (int64_t)(entries / 3); k++) {
+            const uint32_t* m = op->map.data() + 3 * k;
+            nodes3 = nodes3 && m[0] % 3 == 0 && m[1] == m[0] + 1 && m[2] == m[0] + 2;
+        }
+    }
+    const uint32_t b = nodes3 ? 3 : 1, lists = op->n_dofs / b, per = n / b;
+    std::vector<uint32_t> off((size_t)lists + 1, 0), idx(entries / b);
+    for (uint64_t k = 0; k < entries; k += b) off[op->map[k] / b + 1]++;
+    for (uint32_t m = 0; m < lists; m++) off[m + 1] += off[m];
+    std::vector<uint32_t> fill(off.begin(), off.end() - 1);
+    for (size_t c = 0; c + 1 < color_first.size(); c++) {
+        // elements of one colour share no DoF: their lists are filled side by side
+#pragma omp parallel for schedule(static)
+        for (int64_t p = color_first[c]; p < (int64_t)color_first[c + 1]; p++) {
+            const uint32_t* m = op->map.data() + op->offsets[op->perm[p]];
+            for (uint32_t j = 0; j < per; j++) idx[fill[m[j * b] / b]++] = (uint32_t)p * n + j * b;
+        }
+    }
+    AFM_CUDA(dalloc(op, &op->d_gather_off, sizeof(uint32_t) * off.size()));
+    AFM_CUDA(dalloc(op, &op->d_gather_idx, sizeof(uint32_t) * idx.size()));
+    AFM_CUDA(dalloc(op, &op->d_ve, (gather_pays(op, false, 8) ? 8 : 4) * entries));
+    AFM_CUDA(cudaMemcpyAsync(op->d_gather_off, off.data(), sizeof(uint32_t) * off.size(), cudaMemcpyHostToDevice,
+                             op->stream));
+    AFM_CUDA(cudaMemcpyAsync(op->d_gather_idx, idx.data(), sizeof(uint32_t) * idx.size(), cudaMemcpyHostToDevice,
+                             op->stream));
+    AFM_CUDA(cudaStreamSynchronize(op->stream));
+    op->gather_b = b;
+    return AFM_SUCCESS;
+}
+
+// Whether a product (wide: 8-byte staged u) enqueued on st may use the element-product buffer, which
+// the operator's products share. A product on another stream than the one
+// before waits for that one's end; inside a caller's own capture, whose graph
+// may be replayed beside other products, the colour launches (no shared
+// buffer) run instead.
+int gather_ready(afm_operator* op, bool wide, uint32_t ve_bytes, cudaStream_t st, bool* use) {
+    *use = false;
+    if (!op->gather_b || !gather_pays(op, wide, ve_bytes)) return AFM_SUCCESS;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    AFM_CUDA(cudaStreamIsCapturing(st, &cap));
+    const bool own = op->own_capture && st == op->stream;  // after a product of the same solve on this stream
+    if (cap != cudaStreamCaptureStatusNone && !own) return AFM_SUCCESS;
+    if (st != op->ve_stream && op->ve_stream && !own) {
+        if (op->ve_stream == op->stream) {
+            // (a caller's stream may be gone by now: its event was recorded after its product)
+            if (!op->ve_event) AFM_CUDA(cudaEventCreateWithFlags(&op->ve_event, cudaEventDisableTiming));
+            AFM_CUDA(cudaStreamIsCapturing(op->stream, &cap));
+            if (cap != cudaStreamCaptureStatusNone) return AFM_SUCCESS;
+            AFM_CUDA(cudaEventRecord(op->ve_event, op->stream));
+        }
+        AFM_CUDA(cudaStreamWaitEvent(st, op->ve_event, 0));
+    }
+    op->ve_stream = st;
+    *use = true;
+    return AFM_SUCCESS;
+}
+
+int gather_done(afm_operator* op, cudaStream_t st) {
+    if (st == op->stream) return AFM_SUCCESS;
+    if (!op->ve_event) AFM_CUDA(cudaEventCreateWithFlags(&op->ve_event, cudaEventDisableTiming));
+    AFM_CUDA(cudaEventRecord(op->ve_event, st));
+    return AFM_SUCCESS;
 }
 
 // True when every element matrix is symmetric to within 1e-6 of its largest
@@ -848,9 +950,11 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
     return AFM_SUCCESS;
 }
 
+// bc_done (MatMult_mf callers, bc_mode 1): set where the product also wrote v_c = u_c.
 int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32 = false,
-                   bool inner64 = false) {
+                   bool inner64 = false, bool* bc_done = nullptr) {
     if (op->matfree_type == 2) return enqueue_free(op, d_v, d_u, bc_mode, st, f32);
+    const void* const d_u_in = d_u;
     // f32: FP32 product on float vectors, from the symmetric inner arena once
     // built, else from an FP32 arena or the hi plane of a split arena (half of
     // each unit is copied). inner64: FP64 vectors on the corrected symmetric
@@ -877,6 +981,43 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     // split arithmetic: max|u| for the launches' power-of-two u scale (and v = 0) in one launch, before
     // the first element launch, which waits for it in full; other arithmetic: v = 0
     const bool scaled = kprec == AFM_PREC_FP64_SPLIT || kprec == kPrecSplitSymX;
+    // one launch for every element plus the gather pass, which writes every entry of v
+    bool gather = false;
+    const bool fused = op->fused && op->fused_ok && kprec == AFM_PREC_FP64_SPLIT && !sym && !f32;
+    const int ve_bytes = (f32 || kprec == AFM_PREC_FP32) && !symx ? 4 : 8;
+    if (!fused)
+        if (int s = gather_ready(op, scaled || kprec == AFM_PREC_FP64, ve_bytes, st, &gather)) return s;
+    if (gather) {
+        if (scaled)
+            AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs, nullptr,
+                                 0, op->d_usc, st));
+        Segment s = op->segs[0];
+        s.count = s.units = op->n_elem;
+        SegArgs a;
+        a.ke = sym ? op->d_sym : op->d_ke;
+        a.map = op->d_map;
+        a.u = d_u;
+        a.v = nullptr;
+        a.ve = op->d_ve;
+        a.units = a.count = op->n_elem;
+        a.unit_bytes = sym ? s.sym_unit_bytes : s.unit_bytes;
+        a.copy_bytes = (uint32_t)a.unit_bytes;
+        a.plane = sym ? s.sym_plane : s.plane;
+        if (f32 && !sym && op->precision == AFM_PREC_FP64_SPLIT) a.copy_bytes = s.plane * 4;
+        a.bc_mode = bc_mode;
+        a.err = op->d_err;
+        a.umax = op->d_usc;
+        a.wait_ns = op->wait_ns;
+        a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
+        AFM_CUDA(launch_segment(s, kprec, a, op->sm_count, false, false, st));
+        const int vt_bytes = f32 || kprec == AFM_PREC_FP32 ? 4 : 8;
+        const bool set_rows = bc_mode && bc_done;
+        AFM_CUDA(launch_gather_sum(ve_bytes, vt_bytes, op->gather_b, via_vx ? (void*)d_v32 : d_v, op->d_ve,
+                                   op->d_gather_off, op->d_gather_idx, op->n_dofs, d_u_in,
+                                   set_rows ? op->d_bcmask : nullptr, st));
+        if (set_rows) *bc_done = true;
+        return gather_done(op, st);
+    }
     if (scaled)
         AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
                              static_cast<double*>(d_v), op->n_dofs, op->d_usc, st));
@@ -918,8 +1059,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     // split products of a plan with one element size: every colour in one cooperative launch (outside
     // stream capture: captured solve iterations keep the colour launches)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (op->fused && op->fused_ok && kprec == AFM_PREC_FP64_SPLIT && !sym && !f32 &&
-        cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    if (fused && cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
         const Segment& s0 = op->segs[0];
         SegArgs a;
         a.ke = op->d_ke;
@@ -963,6 +1103,17 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         first = false;
     }
     if (via_vx) AFM_CUDA(launch_to_f32(d_v32, op->d_vx, op->n_dofs, st));
+    return AFM_SUCCESS;
+}
+
+// MatMult_mf: the product with constrained columns read as zero, then v_c = u_c.
+// T = float: the FP32 product. inner64: the FP64 product of symmetric inner formats 3 to 5.
+template <typename T>
+int enqueue_matmult(afm_operator* op, T* d_v, const T* d_u, cudaStream_t st, bool inner64 = false) {
+    bool bc_done = false;
+    const int s = enqueue_matvec(op, d_v, d_u, 1, st, std::is_same<T, float>::value, inner64, &bc_done);
+    if (s) return s;
+    if (!bc_done) AFM_CUDA(launch_set_constrained(d_v, d_u, op->d_bc_idx, op->n_bc, st));
     return AFM_SUCCESS;
 }
 
@@ -1251,9 +1402,7 @@ template <typename T>
 int cg_step(afm_operator* op, const CgVectors<T>& V, cudaStream_t st);
 template <>
 int cg_step<double>(afm_operator* op, const CgVectors<double>& V, cudaStream_t st) {
-    int s = enqueue_matvec(op, V.q, V.p, 1, st);
-    if (s) return s;
-    AFM_CUDA(launch_set_constrained(V.q, V.p, op->d_bc_idx, op->n_bc, st));
+    if (int s = enqueue_matmult(op, V.q, V.p, st)) return s;
     double* sc = op->d_scalars;
     double* part = sc + kScalarSlots;
     AFM_CUDA(launch_cg_alpha(V.p, V.q, op->n_dofs, sc, part, st));
@@ -1262,9 +1411,7 @@ int cg_step<double>(afm_operator* op, const CgVectors<double>& V, cudaStream_t s
 }
 template <>
 int cg_step<float>(afm_operator* op, const CgVectors<float>& V, cudaStream_t st) {
-    int s = enqueue_matvec(op, V.q, V.p, 1, st, true);
-    if (s) return s;
-    AFM_CUDA(launch_set_constrained(V.q, V.p, op->d_bc_idx, op->n_bc, st));
+    if (int s = enqueue_matmult(op, V.q, V.p, st)) return s;
     double* sc = op->d_scalars;
     double* part = sc + kScalarSlots;
     AFM_CUDA(launch_cg_alpha(V.p, V.q, op->n_dofs, sc, part, st));
@@ -1275,9 +1422,7 @@ int cg_step<float>(afm_operator* op, const CgVectors<float>& V, cudaStream_t st)
 // One iteration of the FP64-vector inner recursion (symmetric inner format
 // 3): the double-float product of the corrected symmetric arena.
 int cg_step_inner64(afm_operator* op, const CgVectors<double>& V, cudaStream_t st) {
-    int s = enqueue_matvec(op, V.q, V.p, 1, st, false, true);
-    if (s) return s;
-    AFM_CUDA(launch_set_constrained(V.q, V.p, op->d_bc_idx, op->n_bc, st));
+    if (int s = enqueue_matmult(op, V.q, V.p, st, true)) return s;
     double* sc = op->d_scalars;
     double* part = sc + kScalarSlots;
     AFM_CUDA(launch_cg_alpha(V.p, V.q, op->n_dofs, sc, part, st));
@@ -1313,12 +1458,14 @@ int ensure_cg_graph(afm_operator* op, afm_operator::CgGraph& gc, const CgVectors
     AFM_CUDA(cudaStreamSynchronize(st));
     AFM_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int s = AFM_SUCCESS;
+    op->own_capture = true;
     for (int i = 0; i < batch && s == AFM_SUCCESS; i++) {
         if constexpr (std::is_same<T, double>::value)
             s = inner64 ? cg_step_inner64(op, V, st) : cg_step<T>(op, V, st);
         else
             s = cg_step<T>(op, V, st);
     }
+    op->own_capture = false;
     if (s == AFM_SUCCESS &&
         cudaMemcpyAsync(h, op->d_scalars, sizeof(double) * kScalarSlots, cudaMemcpyDeviceToHost, st) != cudaSuccess)
         s = fail(AFM_ERR_CUDA, "capture: scalar copy");
@@ -1683,6 +1830,7 @@ int afm::set_stream_priority(afm_operator* op, int priority) {
     }
     cudaStreamDestroy(op->stream);
     op->stream = st;
+    op->ve_stream = nullptr;  // (its work has finished)
     drop_graph(op->cg64);  // no captured iteration keeps the old stream's work order
     drop_graph(op->cg32);
     drop_graph(op->cg64i);
@@ -1777,6 +1925,7 @@ int afm_destroy(afm_operator* op) {
         }
         if (op->h_scalars) cudaFreeHost(op->h_scalars);
         if (op->h_bremain) cudaFreeHost(op->h_bremain);
+        if (op->ve_event) cudaEventDestroy(op->ve_event);
         if (op->stream) cudaStreamDestroy(op->stream);
     }
     delete op;
@@ -2307,6 +2456,17 @@ int afm_finalize(afm_operator* op) {
     AFM_CUDA(cudaStreamSynchronize(op->stream));
     int st = upload_arena(op);
     if (st != AFM_SUCCESS) return st;
+    if (!op->use_patches && !op->dup_in_element && !op->segs.empty()) {
+        bool same = true;
+        for (const Segment& s : op->segs) same = same && s.regime == REG_WPE && s.n == op->segs[0].n;
+        if (same) {
+            std::vector<uint32_t> first;
+            for (const Segment& s : op->segs) first.push_back((uint32_t)s.first_pos);
+            first.push_back(op->n_elem);
+            st = build_gather(op, op->segs[0].n, first);
+            if (st != AFM_SUCCESS) return st;
+        }
+    }
 
     // symmetric inner arena (built on the first FP32 product): split arena,
     // symmetric Ke, and elements that run as patches or on the warp-group kernel
@@ -2395,10 +2555,8 @@ int afm_matmult_bc_device(afm_operator* op, double* d_v, const double* d_u, void
     if (!d_v || !d_u || d_v == (double*)d_u) return fail(AFM_ERR_INVALID_ARG, "bad vectors");
     DeviceGuard g(op->device);
     cudaStream_t st = pick_stream(op, stream);
-    int s = enqueue_matvec(op, d_v, d_u, 1, st);
-    if (s) return s;
-    AFM_CUDA(launch_set_constrained(d_v, d_u, op->d_bc_idx, op->n_bc, st));
-    return ok();
+    const int s = enqueue_matmult(op, d_v, d_u, st);
+    return s == AFM_SUCCESS ? ok() : s;
 }
 
 int afm_matmult_bc(afm_operator* op, double* v, const double* u) {
@@ -2429,10 +2587,8 @@ int afm_matmult_bc_device_f32(afm_operator* op, float* d_v, const float* d_u, vo
     cudaStream_t st = pick_stream(op, stream);
     int s = ensure_sym(op, st);
     if (s) return s;
-    s = enqueue_matvec(op, d_v, d_u, 1, st, true);
-    if (s) return s;
-    AFM_CUDA(launch_set_constrained(d_v, d_u, op->d_bc_idx, op->n_bc, st));
-    return ok();
+    s = enqueue_matmult(op, d_v, d_u, st);
+    return s == AFM_SUCCESS ? ok() : s;
 }
 
 int afm_get_diagonal(afm_operator* op, double* diag) {
@@ -3022,8 +3178,11 @@ int afm_get_info(afm_operator* op, afm_info* info) {
     } else if (op->use_patches) {
         launches += op->patch_one_launch ? 1u + (op->n_shared ? 1u : 0u) : (uint32_t)op->patch_color_first.size() - 1;
     } else {
-        for (const Segment& s : op->segs)
-            if (s.units) launches++;
+        if (op->gather_b && gather_pays(op, op->precision != AFM_PREC_FP32, op->precision == AFM_PREC_FP32 ? 4 : 8) && !(op->fused && op->fused_ok))
+            launches += 2;  // one launch for every element and the gather pass
+        else
+            for (const Segment& s : op->segs)
+                if (s.units) launches++;
     }
     info->n_launches = launches;
     info->n_patches = op->n_patches;

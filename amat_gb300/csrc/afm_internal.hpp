@@ -71,6 +71,8 @@ struct SegArgs {
     const unsigned long long* umax;  // split arithmetic: max|u| (bits of a non-negative double)
     unsigned long long wait_ns;  // limit of each pipeline wait (afm_set_wait_limit)
     const int* probe;         // test hook: a flag nothing sets, or null (afm_set_wait_probe)
+    void* ve = nullptr;       // warp-group kernel: element products go here (VO, n per element in arena order)
+                              // for the gather pass (launch_gather_sum); null: added to v, one launch per colour
 };
 
 // Arguments of one batched (multi right-hand side) segment launch.
@@ -165,6 +167,15 @@ cudaError_t launch_patches(int prec, const PatchPlanGeom& pg, const PatchArgs& a
 // Launched with programmatic dependence on the patch launch.
 cudaError_t launch_patch_combine(int vo_bytes, void* v, const void* pv, const uint32_t* dof, const uint32_t* off,
                                  const uint32_t* idx, uint32_t nb, cudaStream_t st);
+// The gather pass of a plan whose elements run in one launch: v[d] = sum over
+// k in [off[m], off[m + 1]) of ve[idx[k] + d - b m], in order, m = d / b (b =
+// 3: the map lists whole nodes of three consecutive DoFs; b = 1: one list per
+// DoF); where mask is not null and mask[d] != 0, v[d] = u[d] instead. ve holds
+// ve_bytes-wide entries, v and u vt_bytes-wide ones (8 and 8, 8 and 4, 4 and
+// 4). Launched with programmatic dependence on the element launch.
+cudaError_t launch_gather_sum(int ve_bytes, int vt_bytes, uint32_t b, void* v, const void* ve, const uint32_t* off,
+                              const uint32_t* idx, uint32_t n_dofs, const void* u, const uint8_t* mask,
+                              cudaStream_t st);
 // Shared memory of a patch launch (0 if it does not fit).
 size_t patch_smem_bytes(int prec, const PatchPlanGeom& pg, uint32_t copy_bytes);
 
@@ -379,6 +390,16 @@ struct afm_operator {
     uint32_t* d_shared_dof = nullptr;
     uint32_t* d_shared_off = nullptr;
     uint32_t* d_shared_idx = nullptr;
+
+    // one launch for every element (plans of one element size): the element products go to d_ve and a gather
+    // pass sums each DoF's entries in arena (colour) order
+    uint32_t gather_b = 0;          // DoFs per list of the gather pass (0: the plan has none)
+    uint32_t* d_gather_off = nullptr;
+    uint32_t* d_gather_idx = nullptr;
+    double* d_ve = nullptr;
+    cudaStream_t ve_stream = nullptr;  // stream of the last product that used d_ve
+    cudaEvent_t ve_event = nullptr;    // its end, where that stream is not the operator's own
+    bool own_capture = false;          // the operator's solver is capturing its iterations on `stream`
 
     // batched (multi right-hand side) state
     double* d_bwork = nullptr;

@@ -855,7 +855,9 @@ __device__ __forceinline__ void grid_barrier(unsigned* ctr, uint32_t threads, vo
 // FU: the colours of T in one cooperative launch, a grid barrier between
 // them (every colour's CTA split as a colour launch of its own would have);
 // without it one segment, a.units units from a.ke and a.map.
-template <int NT, typename A, bool CH, bool FU>
+// VE: the element products go to a.ve instead of v (a template argument: as a
+// run-time test it cost the colour launches of hex20 42^3 2.7%).
+template <int NT, typename A, bool CH, bool FU, bool VE = false>
 __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, const GroupGeom& G, uint32_t n_rt,
                                         const ColourTable* T) {
     using KT = typename A::KT;
@@ -944,6 +946,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
     const uint32_t bar_id = 1 + grp, bar_threads = G.g * 32;
     const VT* __restrict__ u = static_cast<const VT*>(a.u);
     VO* __restrict__ v = static_cast<VO*>(a.v);
+    VO* __restrict__ ve = static_cast<VO*>(a.ve);
     // the scale was written by a launch that completed before this segment's first launch
     const int usk = load_uscale<A>(a.umax);
     unsigned char* ubuf0 = ubase + (size_t)(grp * 2) * ub;
@@ -993,7 +996,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
             wait_prior_grid();
         else  // every CTA has written the previous colour's sums to v
             grid_barrier(T->gbar + (col - 1), consumer_threads, abort, a.wait_ns);
-        if (gatherer && i < cnt && rvalid) vold_c = v_load(v + (dof_c & kDofMask));
+        if (!VE && gatherer && i < cnt && rvalid) vold_c = v_load(v + (dof_c & kDofMask));
         group_sync(bar_id, bar_threads);
         bool ok = false;  // the current chunk's slot has landed (one verdict per warp and chunk)
         uint32_t s = 0;   // the current chunk's ring slot
@@ -1005,7 +1008,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
             if (gatherer && rvalid) {
                 if (inext < cnt) {
                     u_n = load_u_hint(u, dof_n, a.bc_mode, keep);
-                    vold_n = v_load(v + (dof_n & kDofMask));
+                    if (!VE) vold_n = v_load(v + (dof_n & kDofMask));
                 }
                 if (inn < cnt) dof_nn = map_at(inn);
             }
@@ -1094,7 +1097,13 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
                 for (uint32_t c2 = 1; c2 < G.gc; c2++) {
                     if (rvalid) A::combine(acc, pbuf(par)[(c2 - 1) * n + r]);
                 }
-                if (rvalid && !*abort) st_hint(v + (dof_c & kDofMask), vold_c + finish_s<A>(acc, usk), keep);
+                if (rvalid && !*abort) {
+                    const VO x = finish_s<A>(acc, usk);
+                    if constexpr (VE)
+                        ve[(size_t)(begin + i) * n + r] = x;  // read once: no L2 policy (evict_last: 2% slower at 35 MB)
+                    else
+                        st_hint(v + (dof_c & kDofMask), vold_c + x, keep);
+                }
                 dof_c = dof_n;
                 vold_c = vold_n;
                 dof_n = dof_nn;
@@ -1111,10 +1120,10 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
     if (lane == 0 && *abort) atomicOr(a.err, kErrTimeout);
 }
 
-template <int NT, typename A, bool CH>
+template <int NT, typename A, bool CH, bool VE>
 __global__ void __launch_bounds__((A::kWpgWarps + 1) * 32, 1)
     afm_wpg_kernel(SegArgs a, RingLayout L, GroupGeom G, uint32_t n_rt) {
-    wpg_run<NT, A, CH, false>(a, L, G, n_rt, nullptr);
+    wpg_run<NT, A, CH, false, VE>(a, L, G, n_rt, nullptr);
 }
 
 // All colours of a segment plan with one element size in one cooperative

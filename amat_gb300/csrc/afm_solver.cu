@@ -470,6 +470,48 @@ __global__ void __launch_bounds__(kRedThreads) k_patch_combine(VO* __restrict__ 
     }
 }
 
+// Gather pass of a plan whose elements run in one launch (launch_gather_sum):
+// one thread per DoF; lists and mask are constant, so they load before the
+// wait for the element launch.
+template <typename VO, typename VT, uint32_t B>
+__global__ void __launch_bounds__(kRedThreads) k_gather_sum(VT* __restrict__ v, const VO* __restrict__ ve,
+                                                            const uint32_t* __restrict__ off,
+                                                            const uint32_t* __restrict__ idx, uint32_t n,
+                                                            const VT* __restrict__ u, const uint8_t* __restrict__ mask) {
+    constexpr int kAhead = 8;  // entries in flight per thread
+    const uint32_t d = blockIdx.x * kRedThreads + threadIdx.x;
+    const uint32_t m = d / B, c = d - m * B;
+    const bool live = d < n;
+    const uint32_t k0 = live ? __ldg(off + m) : 0u, k1 = live ? __ldg(off + m + 1) : 0u;
+    const bool fixed = live && mask && mask[d];
+    uint32_t at[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; q++) at[q] = k0 + q < k1 ? __ldg(idx + k0 + q) : 0u;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!live) return;
+    if (fixed) {
+        v[d] = u[d];
+        return;
+    }
+    VO s = VO(0);
+    VO x[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; q++) x[q] = k0 + q < k1 ? __ldcg(ve + at[q] + c) : VO(0);
+#pragma unroll
+    for (int q = 0; q < kAhead; q++)
+        if (k0 + q < k1) s += x[q];
+    for (uint32_t k = k0 + kAhead; k < k1; k += kAhead) {
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) at[q] = k + q < k1 ? __ldg(idx + k + q) : 0u;
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) x[q] = k + q < k1 ? __ldcg(ve + at[q] + c) : VO(0);
+#pragma unroll
+        for (int q = 0; q < kAhead; q++)
+            if (k + q < k1) s += x[q];
+    }
+    v[d] = (VT)s;
+}
+
 inline unsigned grid_for(size_t n) {
     size_t g = (n + kRedThreads - 1) / kRedThreads;
     if (g > 4096) g = 4096;
@@ -583,6 +625,33 @@ cudaError_t launch_patch_combine(int vo_bytes, void* v, const void* pv, const ui
                                   static_cast<const double*>(pv), dof, off, idx, nb);
     return cudaLaunchKernelEx(&cfg, k_patch_combine<float>, static_cast<float*>(v), static_cast<const float*>(pv),
                               dof, off, idx, nb);
+}
+
+namespace {
+template <typename VO, typename VT>
+cudaError_t gather_sum(uint32_t b, void* v, const void* ve, const uint32_t* off, const uint32_t* idx, uint32_t n,
+                       const void* u, const uint8_t* mask, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((n + kRedThreads - 1) / kRedThreads);
+    cfg.blockDim = dim3(kRedThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, b == 3 ? k_gather_sum<VO, VT, 3> : k_gather_sum<VO, VT, 1>, static_cast<VT*>(v),
+                              static_cast<const VO*>(ve), off, idx, n, static_cast<const VT*>(u), mask);
+}
+}  // namespace
+
+cudaError_t launch_gather_sum(int ve_bytes, int vt_bytes, uint32_t b, void* v, const void* ve, const uint32_t* off,
+                              const uint32_t* idx, uint32_t n_dofs, const void* u, const uint8_t* mask,
+                              cudaStream_t st) {
+    if (n_dofs == 0) return cudaSuccess;
+    if (ve_bytes == 8 && vt_bytes == 8) return gather_sum<double, double>(b, v, ve, off, idx, n_dofs, u, mask, st);
+    if (ve_bytes == 8) return gather_sum<double, float>(b, v, ve, off, idx, n_dofs, u, mask, st);
+    return gather_sum<float, float>(b, v, ve, off, idx, n_dofs, u, mask, st);
 }
 
 cudaError_t launch_umax(const double* u, const uint8_t* mask, size_t n, double* vz, size_t nv,
