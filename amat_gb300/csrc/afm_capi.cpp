@@ -926,11 +926,8 @@ int check_device_error(afm_operator* op) {
     return AFM_SUCCESS;
 }
 
-// v = K u (bc_mode 0) or the product of MatMult_mf without the final v_c = u_c
-// (bc_mode 1: constrained columns of u read as zero), device arrays.
-// Matrix-free product (method 2): one launch per colour.
-int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32) {
-    AFM_CUDA(cudaMemsetAsync(d_v, 0, (size_t)op->n_dofs * (f32 ? 4 : 8), st));
+// Matrix-free product (method 2): one launch and the gather pass, or one launch per colour.
+int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32, bool* bc_done) {
     const double E = op->elem_E, nu = op->elem_nu;
     FreeArgs a;
     a.xe = f32 ? (const void*)op->d_free_xe32 : (const void*)op->d_free_xe64;
@@ -942,6 +939,21 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
     a.bc_mode = bc_mode;
     a.lam = E * nu / (1.0 + nu) / (1.0 - 2.0 * nu);
     a.mu = 0.5 * E / (1.0 + nu);
+    bool gather = false;
+    const int vb = f32 ? 4 : 8;
+    if (int s = gather_ready(op, false, vb, st, &gather)) return s;
+    if (gather) {
+        a.ve = op->d_ve;
+        a.first = 0;
+        a.count = op->n_elem;
+        AFM_CUDA(launch_free(op->elem_kind, f32, a, op->sm_count, st));
+        const bool set_rows = bc_mode && bc_done;
+        AFM_CUDA(launch_gather_sum(vb, vb, op->gather_b, d_v, op->d_ve, op->d_gather_off, op->d_gather_idx, op->n_dofs,
+                                   d_u, set_rows ? op->d_bcmask : nullptr, st));
+        if (set_rows) *bc_done = true;
+        return gather_done(op, st);
+    }
+    AFM_CUDA(cudaMemsetAsync(d_v, 0, (size_t)op->n_dofs * vb, st));
     for (size_t c = 0; c + 1 < op->free_color_first.size(); c++) {
         a.first = op->free_color_first[c];
         a.count = op->free_color_first[c + 1] - a.first;
@@ -950,10 +962,12 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
     return AFM_SUCCESS;
 }
 
+// v = K u (bc_mode 0) or the product of MatMult_mf without the final v_c = u_c
+// (bc_mode 1: constrained columns of u read as zero), device arrays.
 // bc_done (MatMult_mf callers, bc_mode 1): set where the product also wrote v_c = u_c.
 int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32 = false,
                    bool inner64 = false, bool* bc_done = nullptr) {
-    if (op->matfree_type == 2) return enqueue_free(op, d_v, d_u, bc_mode, st, f32);
+    if (op->matfree_type == 2) return enqueue_free(op, d_v, d_u, bc_mode, st, f32, bc_done);
     const void* const d_u_in = d_u;
     // f32: FP32 product on float vectors, from the symmetric inner arena once
     // built, else from an FP32 arena or the hi plane of a split arena (half of
@@ -2168,14 +2182,15 @@ int finalize_free(afm_operator* op) {
             x32[(size_t)p * nn * 3 + k] = (float)op->xe[(size_t)e * nn * 3 + k];
         }
     }
-    // reference tables: dN of every node at every quadrature point, then the weights
+    // reference tables: dN of every node at every quadrature point, the weights, the points
     std::vector<double> q;
     afm_shape::quadrature(K.tet, op->elem_ngt, q);
     const uint32_t nq = (uint32_t)(q.size() / 4);
-    std::vector<double> r64((size_t)nq * (nn * 3 + 1));
+    std::vector<double> r64((size_t)nq * (nn * 3 + 4));
     for (uint32_t t = 0; t < nq; t++) {
         K.shape(&q[4 * t], nullptr, &r64[(size_t)t * nn * 3]);
         r64[(size_t)nq * nn * 3 + t] = q[4 * t + 3];
+        for (int p = 0; p < 3; p++) r64[(size_t)nq * (nn * 3 + 1) + 3 * t + p] = q[4 * t + p];
     }
     std::vector<float> r32(r64.begin(), r64.end());
     op->free_nq = nq;
@@ -2243,11 +2258,17 @@ int finalize_free(afm_operator* op) {
         AFM_CUDA(cudaMemcpyAsync(op->d_bc_val, op->values.data(), sizeof(double) * op->n_bc, cudaMemcpyHostToDevice,
                                  st));
     }
+    if (!op->bc_unique.empty()) {
+        AFM_CUDA(dalloc(op, &op->d_bcmask, std::max<uint32_t>(op->n_dofs, 1)));
+        AFM_CUDA(cudaMemcpyAsync(op->d_bcmask, is_bc.data(), op->n_dofs, cudaMemcpyHostToDevice, st));
+    }
     AFM_CUDA(cudaMemcpyAsync(op->d_free_xe64, x64.data(), sizeof(double) * x64.size(), cudaMemcpyHostToDevice, st));
     AFM_CUDA(cudaMemcpyAsync(op->d_free_xe32, x32.data(), sizeof(float) * x32.size(), cudaMemcpyHostToDevice, st));
     AFM_CUDA(cudaMemcpyAsync(op->d_free_ref64, r64.data(), sizeof(double) * r64.size(), cudaMemcpyHostToDevice, st));
     AFM_CUDA(cudaMemcpyAsync(op->d_free_ref32, r32.data(), sizeof(float) * r32.size(), cudaMemcpyHostToDevice, st));
     AFM_CUDA(cudaStreamSynchronize(st));
+    if (!op->dup_in_element)
+        if (int s = build_gather(op, n, op->free_color_first)) return s;
     op->ke_dirty = false;
     op->finalized = true;
     return ok();
@@ -3174,7 +3195,7 @@ int afm_get_info(afm_operator* op, afm_info* info) {
         // matrix-free: node coordinates and the map per element instead of Ke
         info->algorithmic_bytes = (uint64_t)op->n_elem * (op->elem_nodes * 3 * 8 + (uint64_t)op->nmax * 4) +
                                   16 * (uint64_t)op->n_dofs;
-        launches += (uint32_t)op->free_color_first.size() - 1;
+        launches += op->gather_b && gather_pays(op, false, 8) ? 1u : (uint32_t)op->free_color_first.size() - 1;
     } else if (op->use_patches) {
         launches += op->patch_one_launch ? 1u + (op->n_shared ? 1u : 0u) : (uint32_t)op->patch_color_first.size() - 1;
     } else {

@@ -184,12 +184,13 @@ size_t patch_smem_bytes(int prec, const PatchPlanGeom& pg, uint32_t copy_bytes);
 struct FreeArgs {
     const void* xe;        // node coordinates, element-major (nodes x 3), double or float
     const uint32_t* map;   // n DoFs per element (kBcFlag on constrained DoFs)
-    const void* ref;       // dN of every node at every quadrature point ([q][node][3]), then the q weights
+    const void* ref;       // dN of every node at every quadrature point ([q][node][3]), the q weights, the q points
     const void* u;
     void* v;
     uint32_t first, count, nq;
     int bc_mode;
     double lam, mu;        // Lame parameters (elasticity)
+    void* ve = nullptr;    // element products go here for the gather pass; null: added to v, one launch per colour
 };
 cudaError_t launch_free(int kind, bool f32, const FreeArgs& a, int sm_count, cudaStream_t st);
 
