@@ -992,8 +992,6 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     const bool via_vx = symx && !inner64;
     float* const d_v32 = static_cast<float*>(d_v);
     if (via_vx) d_v = op->d_vx;
-    // split arithmetic: max|u| for the launches' power-of-two u scale (and v = 0) in one launch, before
-    // the first element launch, which waits for it in full; other arithmetic: v = 0
     const bool scaled = kprec == AFM_PREC_FP64_SPLIT || kprec == kPrecSplitSymX;
     // one launch for every element plus the gather pass, which writes every entry of v
     bool gather = false;
@@ -1032,22 +1030,30 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         if (set_rows) *bc_done = true;
         return gather_done(op, st);
     }
-    if (scaled)
+    // one launch over every patch and its combine pass write every DoF that an element lists; else v = 0, and
+    // for a segment plan max|u| for the launches' power-of-two u scale, in one launch before the first element
+    // launch, which waits for it in full
+    const bool one_patch = op->use_patches && op->patch_one_launch;
+    if (scaled && !op->use_patches)
         AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
                              static_cast<double*>(d_v), op->n_dofs, op->d_usc, st));
-    else
+    else if (!one_patch || op->n_unlisted)
         AFM_CUDA(cudaMemsetAsync(d_v, 0, via_vx ? (size_t)op->n_dofs * 8 : vbytes, st));
     bool first = true;
     if (op->use_patches) {
         const Segment& s = op->segs[0];
         // one launch over every patch plus the combine pass, or one launch per patch colour
-        const bool one = op->patch_one_launch;
+        const bool one = one_patch;
+        // v_c = u_c on the way, where every constrained DoF is in a patch and v has u's type
+        const bool set_rows = one && bc_mode && bc_done && !op->n_unlisted && !via_vx && op->n_bc;
         const size_t launches = one ? 1 : op->patch_color_first.size() - 1;
         for (size_t c = 0; c < launches; c++) {
             PatchArgs a;
             a.desc = op->d_patch_desc + (one ? 0 : op->patch_color_first[c]);
             a.count = one ? op->n_patches : op->patch_color_first[c + 1] - op->patch_color_first[c];
             a.pv = one ? (void*)op->d_pv : nullptr;
+            a.set_rows = set_rows;
+            a.u_rows = d_u_in;
             a.ke = sym ? op->d_sym : op->d_ke;
             a.idx = op->d_patch_idx;
             a.u = d_u;
@@ -1058,7 +1064,6 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
             if (f32 && !sym && op->precision == AFM_PREC_FP64_SPLIT) a.copy_bytes = s.plane * 4;
             a.bc_mode = bc_mode;
             a.err = op->d_err;
-            a.umax = op->d_usc;
             a.wait_ns = op->wait_ns;
             a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
             AFM_CUDA(launch_patches(kprec, op->patch_geom, a, op->sm_count, !first, st));
@@ -1066,7 +1071,9 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         }
         if (one)
             AFM_CUDA(launch_patch_combine((f32 && !symx) ? 4 : 8, d_v, op->d_pv, op->d_shared_dof,
-                                          op->d_shared_off, op->d_shared_idx, op->n_shared, st));
+                                          op->d_shared_off, op->d_shared_idx, op->n_shared,
+                                          set_rows ? d_u_in : nullptr, st));
+        if (set_rows) *bc_done = true;
         if (via_vx) AFM_CUDA(launch_to_f32(d_v32, op->d_vx, op->n_dofs, st));
         return AFM_SUCCESS;
     }
@@ -2454,12 +2461,20 @@ int afm_finalize(afm_operator* op) {
         const bool small = op->n_patches / ncol < 16ull * (uint64_t)std::max(op->sm_count, 1);
         op->patch_one_launch = op->patch_mode == 3 || (op->patch_mode == 1 && small);
     }
+    std::vector<uint32_t> sdof(op->shared_dof);  // constrained ones flagged
+    for (uint32_t& d : sdof)
+        if (is_bc[d]) d |= kBcFlag;
+    {
+        std::vector<uint8_t> listed(op->n_dofs, 0);
+        for (uint32_t d : op->map) listed[d] = 1;
+        op->n_unlisted = op->n_dofs - (uint32_t)std::count(listed.begin(), listed.end(), (uint8_t)1);
+    }
     if (op->patch_one_launch) {
         AFM_CUDA(dalloc(op, &op->d_pv, sizeof(double) * std::max<size_t>(op->pv_count, 1)));
         AFM_CUDA(dalloc(op, &op->d_shared_dof, sizeof(uint32_t) * std::max<size_t>(op->shared_dof.size(), 1)));
         AFM_CUDA(dalloc(op, &op->d_shared_off, sizeof(uint32_t) * op->shared_off.size()));
         AFM_CUDA(dalloc(op, &op->d_shared_idx, sizeof(uint32_t) * std::max<size_t>(op->shared_idx.size(), 1)));
-        AFM_CUDA(cudaMemcpyAsync(op->d_shared_dof, op->shared_dof.data(), sizeof(uint32_t) * op->shared_dof.size(),
+        AFM_CUDA(cudaMemcpyAsync(op->d_shared_dof, sdof.data(), sizeof(uint32_t) * sdof.size(),
                                  cudaMemcpyHostToDevice, op->stream));
         AFM_CUDA(cudaMemcpyAsync(op->d_shared_off, op->shared_off.data(), sizeof(uint32_t) * op->shared_off.size(),
                                  cudaMemcpyHostToDevice, op->stream));
@@ -3190,7 +3205,7 @@ int afm_get_info(afm_operator* op, afm_info* info) {
     }
     info->algorithmic_bytes = alg + 2 * vb * (uint64_t)op->n_dofs;
     info->algorithmic_flops = fl;
-    uint32_t launches = 1;  // the zero fill of v
+    uint32_t launches = 1;  // the zero fill of v, where there is one
     if (op->matfree_type == 2 && op->finalized) {
         // matrix-free: node coordinates and the map per element instead of Ke
         info->algorithmic_bytes = (uint64_t)op->n_elem * (op->elem_nodes * 3 * 8 + (uint64_t)op->nmax * 4) +

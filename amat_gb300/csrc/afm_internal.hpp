@@ -147,7 +147,8 @@ struct PatchArgs {
     int* err;
     void* pv;                 // one launch for every colour: sums of shared DoFs go here (VO), others to v;
                               // null: one launch per colour, every sum added to v
-    const unsigned long long* umax;  // split arithmetic: max|u| (double bits)
+    int set_rows;             // one launch: v_c = u_c on constrained DoFs of one patch (u_rows has v's entry type)
+    const void* u_rows;
     unsigned long long wait_ns;  // limit of each pipeline wait
     const int* probe;         // test hook: a flag nothing sets, or null (afm_set_wait_probe)
 };
@@ -163,10 +164,11 @@ struct PatchPlanGeom {
 cudaError_t launch_patches(int prec, const PatchPlanGeom& pg, const PatchArgs& a, int sm_count, bool pdl,
                            cudaStream_t stream);
 // The combine pass of one-launch patches: v[dof[i]] = sum over k in
-// [off[i], off[i+1]) of pv[idx[k]], in order (vo_bytes 8: double, 4: float).
+// [off[i], off[i+1]) of pv[idx[k]], in order (vo_bytes 8: double, 4: float);
+// where dof[i] carries kBcFlag and u_rows is not null, v = u_rows instead.
 // Launched with programmatic dependence on the patch launch.
 cudaError_t launch_patch_combine(int vo_bytes, void* v, const void* pv, const uint32_t* dof, const uint32_t* off,
-                                 const uint32_t* idx, uint32_t nb, cudaStream_t st);
+                                 const uint32_t* idx, uint32_t nb, const void* u_rows, cudaStream_t st);
 // The gather pass of a plan whose elements run in one launch: v[d] = sum over
 // k in [off[m], off[m + 1]) of ve[idx[k] + d - b m], in order, m = d / b (b =
 // 3: the map lists whole nodes of three consecutive DoFs; b = 1: one list per
@@ -281,6 +283,7 @@ struct afm_operator {
     std::vector<uint32_t> offsets;  // n_elem + 1
     std::vector<uint32_t> map;      // global DoF ids
     bool dup_in_element = false;    // some element lists a DoF twice
+    uint32_t n_unlisted = 0;        // DoFs that no element lists (decided at finalize)
     int patch_mode = 1;             // small elements: patches, 1 one launch + combine pass when the patch colours
                                     // are small, else one launch per colour; 2 always per colour; 3 always one
                                     // launch; 0 colour segments

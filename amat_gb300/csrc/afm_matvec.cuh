@@ -393,9 +393,14 @@ struct ArithSplitSymX {
 
 // Range guard of the double-float arithmetic. Its u pairs and products live in
 // FP32's exponent range: unscaled, |u| above 3.4e38 would overflow and small
-// entries would fall into FP32 subnormals and lose their low bits. So every
-// launch scales u by 2^k with k = -eu, max|u| = f 2^eu (f in [0.5, 1)), over
-// the DoFs the product reads: the largest scaled entry lies in [0.5, 1), and
+// entries would fall into FP32 subnormals and lose their low bits. So u is
+// scaled by 2^k with k = -eu, max|u| = f 2^eu (f in [0.5, 1)), over the DoFs
+// the product reads (one k per product, from a pass over u before the element
+// launches: launch_umax) or, in the patch kernel, over the patch's DoFs (one k
+// per patch, from the entries it has gathered anyway: the pass over u took 2 of
+// the 8 us of a product on 8^3 elements. The warp-group kernel keeps one k per
+// product: finding it per element cost its loop 25 registers, hex20 42^3 377 ->
+// 482 us). The largest scaled entry lies in [0.5, 1), and
 // with each element's max|Ke| in [1e-30, 1e30] (checked at finalize) the
 // products of a scaled u entry and the element's leading entries stay within
 // FP32's normal range (smaller entries may reach FP32 subnormals, whose
@@ -415,6 +420,14 @@ __device__ __forceinline__ int uscale_of(unsigned long long mbits) {
     if (e == 0) eu = -1022;            // a subnormal maximum: scale as the smallest normal
     return eu > 1000 ? -1000 : (eu < -1000 ? 1000 : -eu);
 }
+
+// The same from the largest biased exponent of the entries (0: all zero or subnormal).
+__device__ __forceinline__ int uscale_of_exp(unsigned e) {
+    if (e >= 0x7ffu) return 0;
+    const int eu = e ? (int)e - 1022 : -1022;
+    return eu > 1000 ? -1000 : (eu < -1000 ? 1000 : -eu);
+}
+__device__ __forceinline__ unsigned biased_exp(double x) { return ((unsigned)__double2hiint(x) >> 20) & 0x7ffu; }
 
 // u scale exponent k of a launch: from the max|u| word for a scaled
 // arithmetic, 0 otherwise.

@@ -272,7 +272,7 @@ PatchLayout patch_layout_g(const PatchPlanGeom& pg, uint32_t copy_bytes, uint32_
     L.groups = groups;
     L.slot_bytes = (copy_bytes + kSlotAlign - 1) / kSlotAlign * kSlotAlign;
     L.idx_bytes = patch_r16(pg.max_idx);
-    L.us_bytes = patch_r16(pg.max_ndof * (uint32_t)sizeof(typename ARITH::UT));
+    L.us_bytes = patch_r16(pg.max_ndof * (uint32_t)sizeof(typename ARITH::UT)) + (ARITH::kScaled ? 16u : 0u);
     L.ve_bytes = patch_r16(pg.n * pg.max_slots * (uint32_t)sizeof(typename ARITH::Acc));
     const uint32_t fixed = 16 * kPatchMaxGroups + 16 + 16 + L.groups * L.group_bytes();
     L.stages = 0;

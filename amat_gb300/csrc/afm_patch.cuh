@@ -173,8 +173,7 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
     VO* __restrict__ v = static_cast<VO*>(a.v);
     VO* __restrict__ pv = static_cast<VO*>(a.pv);
     const uint64_t keep = l2_evict_last_policy();
-    // the scale was written by a launch that completed before this matvec's first launch
-    const int usk = load_uscale<A>(a.umax);
+    unsigned* emax = reinterpret_cast<unsigned*>(gbase + L.idx_bytes + L.us_bytes - 16);  // scaled arithmetic
 
     // ring index of this group's first unit: units of the patches before it
     uint32_t base = 0;
@@ -190,6 +189,7 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
         const uint16_t* slot = reinterpret_cast<const uint16_t*>(gbase + patch_slot_off(d.ndof, d.units, n));
         const uint32_t cap = d.units * 32u;
 
+        unsigned ue = 0;  // largest exponent of this thread's entries (scaled arithmetic)
         // u of the patch's DoFs, once; kBatch independent loads in flight per
         // thread before any of them is used (in-order issue would otherwise
         // pay one memory latency per DoF)
@@ -206,9 +206,30 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
 #pragma unroll
                 for (int q = 0; q < kBatch; q++) {
                     const uint32_t i = i0 + q * kPatchGroupThreads;
-                    if (i < d.ndof) us[i] = stage_s<A>((a.bc_mode && (m[q] & kBcFlag)) ? VT(0) : x[q], usk);
+                    if (i < d.ndof) {
+                        const VT y = (a.bc_mode && (m[q] & kBcFlag)) ? VT(0) : x[q];
+                        if constexpr (A::kScaled) {
+                            static_assert(sizeof(VT) == sizeof(UT), "staged in place");
+                            reinterpret_cast<VT*>(us)[i] = y;  // split below, once the patch's scale is known
+                            ue = max(ue, biased_exp(y));
+                        } else {
+                            us[i] = A::stage(y);
+                        }
+                    }
                 }
             }
+        int usk = 0;
+        if constexpr (A::kScaled) {
+            ue = __reduce_max_sync(0xffffffffu, ue);
+            if (lane == 0) emax[wg] = ue;
+            named_barrier(bar_id, kPatchGroupThreads);
+#pragma unroll
+            for (uint32_t w = 0; w < kPatchGroupWarps; w++) ue = max(ue, emax[w]);
+            usk = uscale_of_exp(ue);
+            if (iok)
+                for (uint32_t i = t; i < d.ndof; i += kPatchGroupThreads)  // (each thread's own entries)
+                    us[i] = split_scaled(reinterpret_cast<const VT*>(us)[i], usk);
+        }
         named_barrier(bar_id, kPatchGroupThreads);
 
         // element products: lane l of warp w takes slot (unit w + W i, lane l)
@@ -253,13 +274,15 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
                 const uint32_t q1 = coff[i + 1];
                 for (uint32_t c = coff[i]; c < q1; c++) A::combine(sum, ve[slot[c]]);
                 const VO val = finish_s<A>(sum, usk);
-                const uint32_t g = glob[i];
+                const uint32_t g = glob[i], dof = g & kPatchDofMask;
                 if (pv == nullptr)
-                    red_add(v + (g & kPatchDofMask), val);
+                    red_add(v + dof, val);
                 else if (g & kSharedFlag)
                     pv[d.pv_off + i] = val;  // added to v by the combine pass, in patch order
+                else if (a.set_rows && (g & kBcFlag))
+                    v[dof] = static_cast<const VO*>(a.u_rows)[dof];  // MatMult_mf's v_c = u_c
                 else
-                    v[g & kPatchDofMask] = val;  // the only patch that lists this DoF
+                    v[dof] = val;  // the only patch that lists this DoF
             }
         named_barrier(bar_id, kPatchGroupThreads);
         if (t == 0) mbar_arrive(&idx_empty[g]);

@@ -459,14 +459,20 @@ template <typename VO>
 __global__ void __launch_bounds__(kRedThreads) k_patch_combine(VO* __restrict__ v, const VO* __restrict__ pv,
                                                                const uint32_t* __restrict__ dof,
                                                                const uint32_t* __restrict__ off,
-                                                               const uint32_t* __restrict__ idx, uint32_t nb) {
+                                                               const uint32_t* __restrict__ idx, uint32_t nb,
+                                                               const VO* __restrict__ u_rows) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += stride) {
+        const uint32_t d = dof[i] & kDofMask;
+        if (u_rows && (dof[i] & kBcFlag)) {
+            v[d] = u_rows[d];
+            continue;
+        }
         const uint32_t k0 = off[i], k1 = off[i + 1];
         VO s = pv[idx[k0]];
         for (uint32_t k = k0 + 1; k < k1; k++) s += pv[idx[k]];
-        v[dof[i]] = s;
+        v[d] = s;
     }
 }
 
@@ -609,7 +615,7 @@ cudaError_t launch_add_f32(double* x, double* d, size_t n, cudaStream_t st, doub
 }
 
 cudaError_t launch_patch_combine(int vo_bytes, void* v, const void* pv, const uint32_t* dof, const uint32_t* off,
-                                 const uint32_t* idx, uint32_t nb, cudaStream_t st) {
+                                 const uint32_t* idx, uint32_t nb, const void* u_rows, cudaStream_t st) {
     if (nb == 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid_for(nb));
@@ -622,9 +628,10 @@ cudaError_t launch_patch_combine(int vo_bytes, void* v, const void* pv, const ui
     cfg.numAttrs = 1;
     if (vo_bytes == 8)
         return cudaLaunchKernelEx(&cfg, k_patch_combine<double>, static_cast<double*>(v),
-                                  static_cast<const double*>(pv), dof, off, idx, nb);
+                                  static_cast<const double*>(pv), dof, off, idx, nb,
+                                  static_cast<const double*>(u_rows));
     return cudaLaunchKernelEx(&cfg, k_patch_combine<float>, static_cast<float*>(v), static_cast<const float*>(pv),
-                              dof, off, idx, nb);
+                              dof, off, idx, nb, static_cast<const float*>(u_rows));
 }
 
 namespace {
