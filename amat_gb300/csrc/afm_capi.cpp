@@ -261,6 +261,7 @@ void free_device(afm_operator* op) {
     dfree(op, op->d_shared_dof);
     dfree(op, op->d_shared_off);
     dfree(op, op->d_shared_idx);
+    dfree(op, op->d_shared_pos);
     dfree(op, op->d_sym);
     dfree(op, op->d_vx);
     dfree(op, op->d_csr_rp);
@@ -926,8 +927,16 @@ int check_device_error(afm_operator* op) {
     return AFM_SUCCESS;
 }
 
+// What a product's last pass may do beside v for a MatMult_mf caller, and whether it did.
+struct ProductTail {
+    bool bc_done = false;      // v_c = u_c was written
+    double* part = nullptr;    // wanted: the partials of v.u (null: not)
+    uint32_t nb = 0;           // ... and how many were written (0: none)
+};
+
 // Matrix-free product (method 2): one launch and the gather pass, or one launch per colour.
-int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32, bool* bc_done) {
+int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32,
+                 ProductTail* tail) {
     const double E = op->elem_E, nu = op->elem_nu;
     FreeArgs a;
     a.xe = f32 ? (const void*)op->d_free_xe32 : (const void*)op->d_free_xe64;
@@ -947,10 +956,10 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
         a.first = 0;
         a.count = op->n_elem;
         AFM_CUDA(launch_free(op->elem_kind, f32, a, op->sm_count, st));
-        const bool set_rows = bc_mode && bc_done;
+        double* part = tail && op->n_dofs <= kFusedDotDofs ? tail->part : nullptr;
         AFM_CUDA(launch_gather_sum(vb, vb, op->gather_b, d_v, op->d_ve, op->d_gather_off, op->d_gather_idx, op->n_dofs,
-                                   d_u, set_rows ? op->d_bcmask : nullptr, st));
-        if (set_rows) *bc_done = true;
+                                   d_u, tail ? op->d_bcmask : nullptr, part, tail ? &tail->nb : nullptr, st));
+        if (tail) tail->bc_done = true;
         return gather_done(op, st);
     }
     AFM_CUDA(cudaMemsetAsync(d_v, 0, (size_t)op->n_dofs * vb, st));
@@ -964,10 +973,10 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
 
 // v = K u (bc_mode 0) or the product of MatMult_mf without the final v_c = u_c
 // (bc_mode 1: constrained columns of u read as zero), device arrays.
-// bc_done (MatMult_mf callers, bc_mode 1): set where the product also wrote v_c = u_c.
+// tail: MatMult_mf callers (bc_mode 1).
 int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32 = false,
-                   bool inner64 = false, bool* bc_done = nullptr) {
-    if (op->matfree_type == 2) return enqueue_free(op, d_v, d_u, bc_mode, st, f32, bc_done);
+                   bool inner64 = false, ProductTail* tail = nullptr) {
+    if (op->matfree_type == 2) return enqueue_free(op, d_v, d_u, bc_mode, st, f32, tail);
     const void* const d_u_in = d_u;
     // f32: FP32 product on float vectors, from the symmetric inner arena once
     // built, else from an FP32 arena or the hi plane of a split arena (half of
@@ -1002,7 +1011,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     if (gather) {
         if (scaled)
             AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs, nullptr,
-                                 0, op->d_usc, st));
+                                 0, op->d_usc, op->own_capture && !inner_f32u, st));
         Segment s = op->segs[0];
         s.count = s.units = op->n_elem;
         SegArgs a;
@@ -1023,11 +1032,11 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
         AFM_CUDA(launch_segment(s, kprec, a, op->sm_count, false, false, st));
         const int vt_bytes = f32 || kprec == AFM_PREC_FP32 ? 4 : 8;
-        const bool set_rows = bc_mode && bc_done;
+        double* part = tail && op->n_dofs <= kFusedDotDofs ? tail->part : nullptr;
         AFM_CUDA(launch_gather_sum(ve_bytes, vt_bytes, op->gather_b, via_vx ? (void*)d_v32 : d_v, op->d_ve,
                                    op->d_gather_off, op->d_gather_idx, op->n_dofs, d_u_in,
-                                   set_rows ? op->d_bcmask : nullptr, st));
-        if (set_rows) *bc_done = true;
+                                   tail ? op->d_bcmask : nullptr, part, tail ? &tail->nb : nullptr, st));
+        if (tail) tail->bc_done = true;
         return gather_done(op, st);
     }
     // one launch over every patch and its combine pass write every DoF that an element lists; else v = 0, and
@@ -1036,7 +1045,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     const bool one_patch = op->use_patches && op->patch_one_launch;
     if (scaled && !op->use_patches)
         AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
-                             static_cast<double*>(d_v), op->n_dofs, op->d_usc, st));
+                             static_cast<double*>(d_v), op->n_dofs, op->d_usc, false, st));
     else if (!one_patch || op->n_unlisted)
         AFM_CUDA(cudaMemsetAsync(d_v, 0, via_vx ? (size_t)op->n_dofs * 8 : vbytes, st));
     bool first = true;
@@ -1045,13 +1054,15 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         // one launch over every patch plus the combine pass, or one launch per patch colour
         const bool one = one_patch;
         // v_c = u_c on the way, where every constrained DoF is in a patch and v has u's type
-        const bool set_rows = one && bc_mode && bc_done && !op->n_unlisted && !via_vx && op->n_bc;
+        const bool set_rows = one && tail && !op->n_unlisted && !via_vx;
         const size_t launches = one ? 1 : op->patch_color_first.size() - 1;
         for (size_t c = 0; c < launches; c++) {
             PatchArgs a;
             a.desc = op->d_patch_desc + (one ? 0 : op->patch_color_first[c]);
             a.count = one ? op->n_patches : op->patch_color_first[c + 1] - op->patch_color_first[c];
             a.pv = one ? (void*)op->d_pv : nullptr;
+            // the solver's last launch wrote u: one launch may be on the SMs (and loading element matrices) before
+            a.u_dep = one && op->own_capture && !op->n_unlisted && !inner_f32u;
             a.set_rows = set_rows;
             a.u_rows = d_u_in;
             a.ke = sym ? op->d_sym : op->d_ke;
@@ -1066,14 +1077,18 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
             a.err = op->d_err;
             a.wait_ns = op->wait_ns;
             a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
-            AFM_CUDA(launch_patches(kprec, op->patch_geom, a, op->sm_count, !first, st));
+            AFM_CUDA(launch_patches(kprec, op->patch_geom, a, op->sm_count, !first || a.u_dep, st));
             first = false;
         }
-        if (one)
-            AFM_CUDA(launch_patch_combine((f32 && !symx) ? 4 : 8, d_v, op->d_pv, op->d_shared_dof,
-                                          op->d_shared_off, op->d_shared_idx, op->n_shared,
-                                          set_rows ? d_u_in : nullptr, st));
-        if (set_rows) *bc_done = true;
+        const int vo_bytes = (f32 || kprec == AFM_PREC_FP32) && !symx ? 4 : 8;
+        if (one && set_rows && tail->part && op->n_dofs <= kFusedDotDofs)
+            AFM_CUDA(launch_patch_combine_dot(vo_bytes, d_v, op->d_pv, op->d_shared_pos, op->d_shared_dof,
+                                              op->d_shared_off, op->d_shared_idx, op->n_dofs, d_u_in, tail->part,
+                                              &tail->nb, st));
+        else if (one)
+            AFM_CUDA(launch_patch_combine(vo_bytes, d_v, op->d_pv, op->d_shared_dof, op->d_shared_off,
+                                          op->d_shared_idx, op->n_shared, set_rows ? d_u_in : nullptr, st));
+        if (set_rows) tail->bc_done = true;
         if (via_vx) AFM_CUDA(launch_to_f32(d_v32, op->d_vx, op->n_dofs, st));
         return AFM_SUCCESS;
     }
@@ -1129,12 +1144,16 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
 
 // MatMult_mf: the product with constrained columns read as zero, then v_c = u_c.
 // T = float: the FP32 product. inner64: the FP64 product of symmetric inner formats 3 to 5.
+// part not null: the partials of v.u too (*nb of them, or 0: not computed).
 template <typename T>
-int enqueue_matmult(afm_operator* op, T* d_v, const T* d_u, cudaStream_t st, bool inner64 = false) {
-    bool bc_done = false;
-    const int s = enqueue_matvec(op, d_v, d_u, 1, st, std::is_same<T, float>::value, inner64, &bc_done);
+int enqueue_matmult(afm_operator* op, T* d_v, const T* d_u, cudaStream_t st, bool inner64 = false,
+                    double* part = nullptr, uint32_t* nb = nullptr) {
+    ProductTail tail;
+    tail.part = part;
+    const int s = enqueue_matvec(op, d_v, d_u, 1, st, std::is_same<T, float>::value, inner64, &tail);
     if (s) return s;
-    if (!bc_done) AFM_CUDA(launch_set_constrained(d_v, d_u, op->d_bc_idx, op->n_bc, st));
+    if (nb) *nb = tail.nb;
+    if (!tail.bc_done) AFM_CUDA(launch_set_constrained(d_v, d_u, op->d_bc_idx, op->n_bc, st));
     return AFM_SUCCESS;
 }
 
@@ -1419,35 +1438,17 @@ struct CgVectors {
     T *r, *z, *p, *q, *dinv, *x;
 };
 
+// Iteration k of a captured batch. inner64: the FP64-vector inner recursion
+// (symmetric inner formats 3 to 5).
 template <typename T>
-int cg_step(afm_operator* op, const CgVectors<T>& V, cudaStream_t st);
-template <>
-int cg_step<double>(afm_operator* op, const CgVectors<double>& V, cudaStream_t st) {
-    if (int s = enqueue_matmult(op, V.q, V.p, st)) return s;
-    double* sc = op->d_scalars;
-    double* part = sc + kScalarSlots;
-    AFM_CUDA(launch_cg_alpha(V.p, V.q, op->n_dofs, sc, part, st));
-    AFM_CUDA(launch_cg_update(V.x, V.r, V.z, V.p, V.q, V.dinv, op->n_dofs, sc, part, st));
-    return AFM_SUCCESS;
-}
-template <>
-int cg_step<float>(afm_operator* op, const CgVectors<float>& V, cudaStream_t st) {
-    if (int s = enqueue_matmult(op, V.q, V.p, st)) return s;
-    double* sc = op->d_scalars;
-    double* part = sc + kScalarSlots;
-    AFM_CUDA(launch_cg_alpha(V.p, V.q, op->n_dofs, sc, part, st));
-    AFM_CUDA(launch_cg_update(V.x, V.r, V.z, V.p, V.q, V.dinv, op->n_dofs, sc, part, st));
-    return AFM_SUCCESS;
-}
-
-// One iteration of the FP64-vector inner recursion (symmetric inner format
-// 3): the double-float product of the corrected symmetric arena.
-int cg_step_inner64(afm_operator* op, const CgVectors<double>& V, cudaStream_t st) {
-    if (int s = enqueue_matmult(op, V.q, V.p, st, true)) return s;
-    double* sc = op->d_scalars;
-    double* part = sc + kScalarSlots;
-    AFM_CUDA(launch_cg_alpha(V.p, V.q, op->n_dofs, sc, part, st));
-    AFM_CUDA(launch_cg_update(V.x, V.r, V.z, V.p, V.q, V.dinv, op->n_dofs, sc, part, st));
+int cg_step(afm_operator* op, const CgVectors<T>& V, int k, bool inner64, cudaStream_t st) {
+    double* in = op->d_scalars + (k % 2) * kScalarSlots;
+    double* out = op->d_scalars + ((k + 1) % 2) * kScalarSlots;
+    double* part = op->d_scalars + kScalarSets * kScalarSlots;
+    uint32_t nb = 0;
+    if (int s = enqueue_matmult(op, V.q, V.p, st, inner64, part, &nb)) return s;
+    if (!nb) AFM_CUDA(launch_dot(V.p, V.q, op->n_dofs, part, &nb, false, st));
+    AFM_CUDA(launch_cg_iteration(V.x, V.r, V.p, V.q, V.dinv, op->n_dofs, in, out, part, nb, st));
     return AFM_SUCCESS;
 }
 
@@ -1480,12 +1481,7 @@ int ensure_cg_graph(afm_operator* op, afm_operator::CgGraph& gc, const CgVectors
     AFM_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int s = AFM_SUCCESS;
     op->own_capture = true;
-    for (int i = 0; i < batch && s == AFM_SUCCESS; i++) {
-        if constexpr (std::is_same<T, double>::value)
-            s = inner64 ? cg_step_inner64(op, V, st) : cg_step<T>(op, V, st);
-        else
-            s = cg_step<T>(op, V, st);
-    }
+    for (int i = 0; i < batch && s == AFM_SUCCESS; i++) s = cg_step(op, V, i, inner64, st);  // (batch is even)
     op->own_capture = false;
     if (s == AFM_SUCCESS &&
         cudaMemcpyAsync(h, op->d_scalars, sizeof(double) * kScalarSlots, cudaMemcpyDeviceToHost, st) != cudaSuccess)
@@ -1622,7 +1618,7 @@ int mixed_residual(MixedSolve& m) {
     if (s) return s;
     AFM_CUDA(cudaMemcpyAsync(W.r64, m.d_b, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
     AFM_CUDA(launch_axpby(W.r64, W.q64, -1.0, 1.0, n, st));
-    AFM_CUDA(launch_norm2(W.r64, n, op->d_scalars, op->d_scalars + kScalarSlots, st));
+    AFM_CUDA(launch_norm2(W.r64, n, op->d_scalars, op->d_scalars + kScalarSets * kScalarSlots, st));
     m.phase = MS_RESID;
     return mixed_record(m);
 }
@@ -1681,7 +1677,7 @@ int mixed_begin(MixedSolve& m) {
         AFM_CUDA(launch_invert(W.V.dinv, op->d_diag, n, st));
         AFM_CUDA(cudaMemsetAsync(W.V.x, 0, n * sizeof(float), st));
     }
-    AFM_CUDA(launch_norm2(m.d_b, n, op->d_scalars, op->d_scalars + kScalarSlots, st));
+    AFM_CUDA(launch_norm2(m.d_b, n, op->d_scalars, op->d_scalars + kScalarSets * kScalarSlots, st));
     m.phase = MS_NORMB;
     return mixed_record(m);
 }
@@ -1719,7 +1715,7 @@ int mixed_advance(MixedSolve& m) {
     cudaStream_t st = op->stream;
     const MixedVectors W = mixed_vectors(op);
     double* sc = op->d_scalars;
-    double* part = sc + kScalarSlots;
+    double* part = sc + kScalarSets * kScalarSlots;
     switch (m.phase) {
         case MS_NORMB:
             m.bn = std::sqrt(h[S_PQ]);
@@ -1919,7 +1915,7 @@ int afm_create(afm_operator** out, int bc_method, int device) {
     if (cudaStreamCreateWithFlags(&op->stream, cudaStreamNonBlocking) != cudaSuccess ||
         dalloc(op, &op->d_err, sizeof(int) * kErrWords) != cudaSuccess ||
         dalloc(op, &op->d_usc, sizeof(unsigned long long) * kUscWords) != cudaSuccess ||
-        dalloc(op, &op->d_scalars, sizeof(double) * (kScalarSlots + kPartialSlots)) != cudaSuccess ||
+        dalloc(op, &op->d_scalars, sizeof(double) * (kScalarSets * kScalarSlots + kPartialSlots)) != cudaSuccess ||
         cudaMallocHost((void**)&op->h_scalars, sizeof(double) * kScalarSlots) != cudaSuccess) {
         afm_destroy(op);
         return fail(AFM_ERR_CUDA, "afm_create: stream or buffer allocation failed");
@@ -2461,7 +2457,7 @@ int afm_finalize(afm_operator* op) {
         const bool small = op->n_patches / ncol < 16ull * (uint64_t)std::max(op->sm_count, 1);
         op->patch_one_launch = op->patch_mode == 3 || (op->patch_mode == 1 && small);
     }
-    std::vector<uint32_t> sdof(op->shared_dof);  // constrained ones flagged
+    std::vector<uint32_t> sdof(op->shared_dof), spos;  // sdof: constrained ones flagged
     for (uint32_t& d : sdof)
         if (is_bc[d]) d |= kBcFlag;
     {
@@ -2472,6 +2468,11 @@ int afm_finalize(afm_operator* op) {
     if (op->patch_one_launch) {
         AFM_CUDA(dalloc(op, &op->d_pv, sizeof(double) * std::max<size_t>(op->pv_count, 1)));
         AFM_CUDA(dalloc(op, &op->d_shared_dof, sizeof(uint32_t) * std::max<size_t>(op->shared_dof.size(), 1)));
+        spos.assign(op->n_dofs, kNoElement);
+        for (size_t i = 0; i < op->shared_dof.size(); i++) spos[op->shared_dof[i]] = (uint32_t)i;
+        AFM_CUDA(dalloc(op, &op->d_shared_pos, sizeof(uint32_t) * std::max<size_t>(spos.size(), 1)));
+        AFM_CUDA(cudaMemcpyAsync(op->d_shared_pos, spos.data(), sizeof(uint32_t) * spos.size(), cudaMemcpyHostToDevice,
+                                 op->stream));
         AFM_CUDA(dalloc(op, &op->d_shared_off, sizeof(uint32_t) * op->shared_off.size()));
         AFM_CUDA(dalloc(op, &op->d_shared_idx, sizeof(uint32_t) * std::max<size_t>(op->shared_idx.size(), 1)));
         AFM_CUDA(cudaMemcpyAsync(op->d_shared_dof, sdof.data(), sizeof(uint32_t) * sdof.size(),
@@ -2684,7 +2685,7 @@ int afm_solve_cg_device(afm_operator* op, const double* d_b, double* d_x, double
     CgVectors<double> V{op->d_work + 2 * n, op->d_work + 3 * n, op->d_work + 4 * n, op->d_work + 5 * n,
                         op->d_work + 6 * n, d_x};
     double* sc = op->d_scalars;
-    double* part = op->d_scalars + kScalarSlots;
+    double* part = op->d_scalars + kScalarSets * kScalarSlots;
     cudaStream_t st = op->stream;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);

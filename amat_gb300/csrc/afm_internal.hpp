@@ -147,6 +147,7 @@ struct PatchArgs {
     int* err;
     void* pv;                 // one launch for every colour: sums of shared DoFs go here (VO), others to v;
                               // null: one launch per colour, every sum added to v
+    int u_dep;                // u comes from the launch before: wait for it before reading
     int set_rows;             // one launch: v_c = u_c on constrained DoFs of one patch (u_rows has v's entry type)
     const void* u_rows;
     unsigned long long wait_ns;  // limit of each pipeline wait
@@ -174,10 +175,17 @@ cudaError_t launch_patch_combine(int vo_bytes, void* v, const void* pv, const ui
 // 3: the map lists whole nodes of three consecutive DoFs; b = 1: one list per
 // DoF); where mask is not null and mask[d] != 0, v[d] = u[d] instead. ve holds
 // ve_bytes-wide entries, v and u vt_bytes-wide ones (8 and 8, 8 and 4, 4 and
-// 4). Launched with programmatic dependence on the element launch.
+// 4). part not null: also the partials of v.u, *nb of them. Launched with
+// programmatic dependence on the element launch.
 cudaError_t launch_gather_sum(int ve_bytes, int vt_bytes, uint32_t b, void* v, const void* ve, const uint32_t* off,
-                              const uint32_t* idx, uint32_t n_dofs, const void* u, const uint8_t* mask,
-                              cudaStream_t st);
+                              const uint32_t* idx, uint32_t n_dofs, const void* u, const uint8_t* mask, double* part,
+                              uint32_t* nb, cudaStream_t st);
+// The combine pass over every DoF (constrained rows as with u_rows = u), with
+// the partials of v.u, *nb of them; pos[d]: the DoF's place in the combine
+// lists, or kNoElement.
+cudaError_t launch_patch_combine_dot(int vo_bytes, void* v, const void* pv, const uint32_t* pos, const uint32_t* dof,
+                                     const uint32_t* off, const uint32_t* idx, uint32_t n, const void* u, double* part,
+                                     uint32_t* nb, cudaStream_t st);
 // Shared memory of a patch launch (0 if it does not fit).
 size_t patch_smem_bytes(int prec, const PatchPlanGeom& pg, uint32_t copy_bytes);
 
@@ -394,6 +402,7 @@ struct afm_operator {
     uint32_t* d_shared_dof = nullptr;
     uint32_t* d_shared_off = nullptr;
     uint32_t* d_shared_idx = nullptr;
+    uint32_t* d_shared_pos = nullptr;  // per DoF: its place in the shared lists, or kNoElement
 
     // one launch for every element (plans of one element size): the element products go to d_ve and a gather
     // pass sums each DoF's entries in arena (colour) order

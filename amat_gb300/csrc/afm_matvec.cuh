@@ -519,6 +519,18 @@ __device__ __forceinline__ double ld_hint(const double* p, uint64_t pol) {
     asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(x) : "l"(p), "l"(pol) : "memory");
     return x;
 }
+// u of the patch kernel, which the launch before may have written while this one was already on the SMs
+// (PatchArgs::u_dep): not ld.global.nc
+__device__ __forceinline__ double ld_u_hint(const double* p, uint64_t pol) {
+    double x;
+    asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(x) : "l"(p), "l"(pol));
+    return x;
+}
+__device__ __forceinline__ float ld_u_hint(const float* p, uint64_t pol) {
+    float x;
+    asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(x) : "l"(p), "l"(pol));
+    return x;
+}
 __device__ __forceinline__ float ld_hint(const float* p, uint64_t pol) {
     float x;
     asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(x) : "l"(p), "l"(pol) : "memory");

@@ -26,7 +26,7 @@
 namespace {
 
 constexpr size_t kVecs = 5;  // r, z, p, q, 1/diag
-constexpr size_t kScratchDoubles = kVecs * (size_t)AFM_NOALLOC_MAX_DOFS + afm::kScalarSlots + afm::kPartialSlots;
+constexpr size_t kScratchDoubles = kVecs * (size_t)AFM_NOALLOC_MAX_DOFS + afm::kScalarSets * afm::kScalarSlots + afm::kPartialSlots;
 
 static __device__ __align__(256) double g_cg_scratch[kScratchDoubles];
 
@@ -85,7 +85,7 @@ extern "C" int afm_solve_cg_device_noalloc(afm_operator* op, const double* d_b, 
     double* q = base + 3 * N;
     double* dinv = base + 4 * N;
     double* sc = base + kVecs * N;
-    double* part = sc + kScalarSlots;
+    double* part = sc + kScalarSets * kScalarSlots;
     cudaStream_t st = op->stream;
     double* h = op->h_scalars;  // pinned, allocated by afm_create
     // stats->seconds: host wall time of the iterations (the allocating solve reports device time from
@@ -93,7 +93,7 @@ extern "C" int afm_solve_cg_device_noalloc(afm_operator* op, const double* d_b, 
     const auto t0 = std::chrono::steady_clock::now();
 
     // the array keeps the previous call's contents: start the solver state from zero
-    NA_CUDA(cudaMemsetAsync(sc, 0, sizeof(double) * (kScalarSlots + kPartialSlots), st));
+    NA_CUDA(cudaMemsetAsync(sc, 0, sizeof(double) * (kScalarSets * kScalarSlots + kPartialSlots), st));
     NA_CUDA(launch_invert(dinv, op->d_diag, n, st));
     s = afm_matmult_bc_device(op, q, d_x, st);
     if (s) return s;
@@ -118,9 +118,12 @@ extern "C" int afm_solve_cg_device_noalloc(afm_operator* op, const double* d_b, 
         if (it >= maxit) break;
         s = afm_matmult_bc_device(op, q, p, st);
         if (s) return s;
-        NA_CUDA(launch_cg_alpha(p, q, n, sc, part, st));
-        NA_CUDA(launch_cg_update(d_x, r, z, p, q, dinv, n, sc, part, st));
-        NA_CUDA(cudaMemcpyAsync(h, sc, sizeof(double) * kScalarSlots, cudaMemcpyDeviceToHost, st));
+        double* in = sc + (it % 2) * kScalarSlots;
+        double* out = sc + ((it + 1) % 2) * kScalarSlots;
+        uint32_t nb = 0;
+        NA_CUDA(launch_dot(p, q, n, part, &nb, false, st));
+        NA_CUDA(launch_cg_iteration(d_x, r, p, q, dinv, n, in, out, part, nb, st));
+        NA_CUDA(cudaMemcpyAsync(h, out, sizeof(double) * kScalarSlots, cudaMemcpyDeviceToHost, st));
         NA_CUDA(cudaStreamSynchronize(st));
         it++;
     }

@@ -178,7 +178,8 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
     // ring index of this group's first unit: units of the patches before it
     uint32_t base = 0;
     for (uint32_t k = 0; k < g && k < cnt; k++) base += desc[k].units;
-    bool waited_prior = false;
+    bool waited_prior = a.u_dep != 0;
+    if (waited_prior) wait_prior_grid();
     for (uint32_t k = g; k < cnt; k += kPatchGroups) {
         const PatchDesc d = desc[k];
         const uint32_t j = k / kPatchGroups;
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
                 for (int q = 0; q < kBatch; q++) {
                     const uint32_t i = i0 + q * kPatchGroupThreads;
                     m[q] = i < d.ndof ? glob[i] : 0u;
-                    x[q] = i < d.ndof ? ld_nc_hint(u + (m[q] & kPatchDofMask), keep) : VT(0);
+                    x[q] = i < d.ndof ? ld_u_hint(u + (m[q] & kPatchDofMask), keep) : VT(0);
                 }
 #pragma unroll
                 for (int q = 0; q < kBatch; q++) {

@@ -45,6 +45,45 @@ __device__ __forceinline__ double final_sum(const double* part, double* sh, uint
     return block_sum(s, sh);
 }
 
+// The FP64 pipe takes 16 cycles per warp instruction, so in the small launches
+// of a CG iteration the count of FP64 instructions per block is the time: a
+// sum over the block goes through shared memory to one warp (12 FP64 adds
+// instead of 43 with a shuffle tree in each warp), and one warp does what the
+// whole block needs once (a division, a square root).
+
+// Sum over the warp's lanes, in every lane.
+__device__ __forceinline__ double warp_sum(double x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// part[k * kRedBlocks + block] = the sums over the block of x[k], k < K. sh: K x kRedThreads.
+template <int K>
+__device__ __forceinline__ void block_partials(const double (&x)[K], double* sh, double* part) {
+#pragma unroll
+    for (int k = 0; k < K; k++) sh[k * kRedThreads + threadIdx.x] = x[k];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    if (k >= K) return;
+    double a[kRedThreads / 32];
+#pragma unroll
+    for (int i = 0; i < kRedThreads / 32; i++) a[i] = sh[k * kRedThreads + 32 * i + lane];
+#pragma unroll
+    for (int o = kRedThreads / 64; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; i++) a[i] += a[i + o];
+    const double s = warp_sum(a[0]);
+    if (lane == 0) part[k * kRedBlocks + blockIdx.x] = s;
+}
+
+// A warp's sum of nb partials, in every lane.
+__device__ __forceinline__ double row_sum(const double* part, uint32_t nb) {
+    double s = 0.0;
+    for (uint32_t i = threadIdx.x & 31; i < nb; i += 32) s += part[i];
+    return warp_sum(s);
+}
+
 #define kStride ((size_t)gridDim.x * kRedThreads)
 
 // Dot-product accumulators of one thread. FP64 vectors: FP64 fused
@@ -91,9 +130,11 @@ __global__ void __launch_bounds__(kRedThreads) k_set_constrained(T* v, const T* 
 
 // part[block]: partial sums of a.b
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_dot(const T* __restrict__ a, const T* __restrict__ b, size_t n,
+__global__ void __launch_bounds__(kRedThreads) k_dot(const T* a, const T* b, size_t n,
                                                      double* part) {
     __shared__ double sh[kRedThreads];
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     DotAcc<T> ab;
     size_t i = (size_t)blockIdx.x * kRedThreads + threadIdx.x;
     for (; i + (kUnroll - 1) * kStride < n; i += kUnroll * kStride) {
@@ -225,26 +266,6 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_reliable_p(T* __restrict__ p
         p[i] = fma_rn(beta, p[i], c * z[i]);
 }
 
-// alpha = rz / (p.q); flag on p.q <= 0 or NaN
-__global__ void __launch_bounds__(kRedThreads) k_cg_alpha(double* sc, const double* part, uint32_t nb) {
-    __shared__ double sh[kRedThreads];
-    const double pq = final_sum(part, sh, nb);
-    if (threadIdx.x == 0) {
-        if (sc[S_DONE] != 0.0) {  // finished earlier: this iteration changes nothing
-            sc[S_ALPHA] = 0.0;
-            return;
-        }
-        sc[S_PQ] = pq;
-        if (!(pq > 0.0)) {
-            sc[S_FLAG] = 1.0;
-            sc[S_DONE] = 1.0;
-            sc[S_ALPHA] = 0.0;
-        } else {
-            sc[S_ALPHA] = sc[S_RZ] / pq;
-        }
-    }
-}
-
 // sc[S_PQ] = sum of the partials (a plain reduction, no CG bookkeeping)
 __global__ void __launch_bounds__(kRedThreads) k_sum(double* sc, const double* part, uint32_t nb) {
     __shared__ double sh[kRedThreads];
@@ -252,82 +273,151 @@ __global__ void __launch_bounds__(kRedThreads) k_sum(double* sc, const double* p
     if (threadIdx.x == 0) sc[S_PQ] = s;
 }
 
-// x += alpha p, r -= alpha q, z = dinv r; partials of r.z, r.r, z.z
+// Launches of one CG iteration follow one another with programmatic
+// dependence: each waits for the one before it in full, but is on the SMs by
+// then. What a launch before may write is read with plain loads (no
+// __restrict__ const pointers, no ld.global.nc, whose lines may have been in
+// L1 since before the write).
+__device__ __forceinline__ void wait_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+
+// First half of an iteration: alpha = r.z / p.q (every block adds up the
+// partials of p.q itself), x += alpha p, r -= alpha q; partials of r.z, r.r,
+// z.z, z = dinv r. A solve that is done, or breaks down here (p.q <= 0 or NaN:
+// out[S_BREAK]), changes nothing. A one-block launch for alpha (and one for
+// beta) cost as much as the vector work up to 10^5 DoFs: the FP64 CG of hex8
+// Poisson 32^3 took 4.10 ms with them, 2.49 ms without.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_cg_update(T* __restrict__ x, T* __restrict__ r, T* __restrict__ z,
-                                                           const T* __restrict__ p, const T* __restrict__ q,
-                                                           const T* __restrict__ dinv, size_t n, const double* sc,
-                                                           double* part) {
-    __shared__ double sh[kRedThreads];
-    const T alpha = (T)sc[S_ALPHA];
-    DotAcc<T> rz, rr, zz;
-    auto step = [&](size_t i, T xi, T pi, T qi, T ri0, T di) {
-        x[i] = alpha * pi + xi;
-        const T ri = -alpha * qi + ri0;
-        const T zi = di * ri;
-        r[i] = ri;
-        z[i] = zi;
-        rz.add(ri, zi);
-        rr.add(ri, ri);
-        zz.add(zi, zi);
+__global__ void __launch_bounds__(kRedThreads) k_cg_xr(T* x, T* r, const T* p, const T* q, const T* dinv, size_t n,
+                                                       const double* in, double* out, const double* part_pq,
+                                                       uint32_t nb_pq, double* part) {
+    __shared__ double sh[3 * kRedThreads];
+    __shared__ double shared_alpha;
+    __shared__ bool shared_bad;
+    release_next();
+    wait_launch();
+    if (in[S_DONE] != 0.0) return;
+    if (threadIdx.x < 32) {
+        const double pq = row_sum(part_pq, nb_pq);
+        const bool bad = !(pq > 0.0);
+        const double a = in[S_RZ] / pq;
+        if (threadIdx.x == 0) {
+            shared_alpha = a;
+            shared_bad = bad;
+            if (blockIdx.x == 0) {
+                out[S_PQ] = pq;
+                out[S_ALPHA] = bad ? 0.0 : a;
+                out[S_BREAK] = bad ? 1.0 : 0.0;
+            }
+        }
+    }
+    // the first entries load while the first warp finds alpha
+    T xv[kUnroll], pv[kUnroll], qv[kUnroll], rv[kUnroll], dv[kUnroll];
+    auto load = [&](size_t i0) {
+#pragma unroll
+        for (int k = 0; k < kUnroll; k++) {
+            const size_t j = i0 + k * kStride;
+            if (j < n) xv[k] = x[j], pv[k] = p[j], qv[k] = q[j], rv[k] = r[j], dv[k] = dinv[j];
+        }
     };
     size_t i = (size_t)blockIdx.x * kRedThreads + threadIdx.x;
-    for (; i + (kUnroll - 1) * kStride < n; i += kUnroll * kStride) {
-        T xv[kUnroll], pv[kUnroll], qv[kUnroll], rv[kUnroll], dv[kUnroll];
+    load(i);
+    __syncthreads();
+    if (shared_bad) return;
+    const T alpha = (T)shared_alpha;
+    DotAcc<T> rz, rr, zz;
+    for (; i < n; i += kUnroll * kStride, load(i)) {
 #pragma unroll
         for (int k = 0; k < kUnroll; k++) {
             const size_t j = i + k * kStride;
-            xv[k] = x[j], pv[k] = p[j], qv[k] = q[j], rv[k] = r[j], dv[k] = dinv[j];
+            if (j < n) {
+                x[j] = alpha * pv[k] + xv[k];
+                const T ri = -alpha * qv[k] + rv[k];
+                const T zi = dv[k] * ri;
+                r[j] = ri;
+                rz.add(ri, zi);
+                rr.add(ri, ri);
+                zz.add(zi, zi);
+            }
         }
-#pragma unroll
-        for (int k = 0; k < kUnroll; k++) step(i + k * kStride, xv[k], pv[k], qv[k], rv[k], dv[k]);
     }
-    for (; i < n; i += kStride) step(i, x[i], p[i], q[i], r[i], dinv[i]);
     const double v[3] = {rz.value(), rr.value(), zz.value()};
-    for (int j = 0; j < 3; j++) {
-        const double t = block_sum(v[j], sh);
-        if (threadIdx.x == 0) part[j * kRedBlocks + blockIdx.x] = t;
-    }
+    block_partials(v, sh, part);
 }
 
-// beta = rz_new / rz
-__global__ void __launch_bounds__(kRedThreads) k_cg_beta(double* sc, const double* part, uint32_t nb) {
-    __shared__ double sh[kRedThreads];
-    const double rz = final_sum(part, sh, nb);
-    const double rr = final_sum(part + kRedBlocks, sh, nb);
-    const double zz = final_sum(part + 2 * kRedBlocks, sh, nb);
-    if (threadIdx.x == 0) {
-        if (sc[S_DONE] != 0.0) {
-            sc[S_BETA] = 0.0;
-            return;
-        }
-        const double old = sc[S_RZ];
-        sc[S_BETA] = (old != 0.0) ? rz / old : 0.0;
-        sc[S_RZOLD] = old;
-        sc[S_RZ] = rz;
-        sc[S_RR] = rr;
-        sc[S_ZZ] = zz;
-        const double it = sc[S_ITER] + 1.0;
-        sc[S_ITER] = it;
-        const double nrm = sqrt(sc[S_NORM] != 0.0 ? zz : rr);
-        if (rz < 0.0 || rz != rz || nrm != nrm) {
-            sc[S_FLAG] = 1.0;
-            sc[S_DONE] = 1.0;
-        } else if (nrm <= sc[S_TOL] || (sc[S_MAXIT] > 0.0 && it >= sc[S_MAXIT])) {
-            sc[S_DONE] = 1.0;
-        }
-    }
-}
-
+// Second half: beta = r.z / (the previous r.z), the stopping test, p = dinv r +
+// beta p. Block 0 writes the new scalars. A finished solve keeps its last
+// direction (the mixed-precision solve continues from it after a reliable
+// update).
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_cg_p(T* __restrict__ p, const T* __restrict__ z, size_t n,
-                                                      const double* sc) {
-    // a finished solve keeps its last direction (the mixed-precision solve
-    // continues from it after a reliable update)
-    if (sc[S_DONE] != 0.0) return;
-    const T beta = (T)sc[S_BETA];
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = beta * p[i] + z[i];
+__global__ void __launch_bounds__(kRedThreads) k_cg_p(T* p, const T* r, const T* dinv, size_t n, const double* in,
+                                                      double* out, const double* part, uint32_t nb) {
+    __shared__ double sums[3];
+    __shared__ double shared_beta;
+    __shared__ int shared_done;  // 1: done, 2: broke down
+    release_next();
+    wait_launch();
+    const uint32_t t = threadIdx.x;
+    const bool lead = blockIdx.x == 0;
+    if (in[S_DONE] != 0.0) {
+        if (lead && t < kScalarSlots) out[t] = in[t];
+        return;
+    }
+    if (out[S_BREAK] != 0.0) {  // (written by the first half)
+        if (lead && t < kScalarSlots && t != S_PQ && t != S_BREAK)
+            out[t] = t == S_FLAG || t == S_DONE ? 1.0 : t == S_ALPHA || t == S_BETA ? 0.0 : in[t];
+        return;
+    }
+    const double it = in[S_ITER] + 1.0;
+    if (t < 96) {
+        const double s = row_sum(part + (t >> 5) * kRedBlocks, nb);
+        if ((t & 31) == 0) sums[t >> 5] = s;
+    }
+    // the first entries load while the first warps find beta
+    T pv[kUnroll], rv[kUnroll], dv[kUnroll];
+    auto load = [&](size_t i0) {
+#pragma unroll
+        for (int k = 0; k < kUnroll; k++) {
+            const size_t j = i0 + k * kStride;
+            if (j < n) pv[k] = p[j], rv[k] = r[j], dv[k] = dinv[j];
+        }
+    };
+    size_t i = (size_t)blockIdx.x * kRedThreads + t;
+    load(i);
+    __syncthreads();
+    if (t < 32) {
+        const double rz = sums[0], old = in[S_RZ];
+        if (t == 0) shared_beta = old != 0.0 ? rz / old : 0.0;
+    } else if (t < 64) {
+        const double rz = sums[0], nrm = sqrt(in[S_NORM] != 0.0 ? sums[2] : sums[1]);
+        const bool bad = rz < 0.0 || rz != rz || nrm != nrm;
+        const bool done = nrm <= in[S_TOL] || (in[S_MAXIT] > 0.0 && it >= in[S_MAXIT]);
+        if (t == 32) shared_done = bad ? 2 : done ? 1 : 0;
+    }
+    __syncthreads();
+    const int done = shared_done;
+    if (lead && t < kScalarSlots && t != S_PQ && t != S_ALPHA && t != S_BREAK) {
+        double y = in[t];
+        if (t == S_RZ) y = sums[0];
+        if (t == S_RZOLD) y = in[S_RZ];
+        if (t == S_RR) y = sums[1];
+        if (t == S_ZZ) y = sums[2];
+        if (t == S_BETA) y = shared_beta;
+        if (t == S_ITER) y = it;
+        if (t == S_FLAG && done == 2) y = 1.0;
+        if (t == S_DONE && done) y = 1.0;
+        out[t] = y;
+    }
+    if (done) return;
+    const T beta = (T)shared_beta;
+    for (; i < n; i += kUnroll * kStride, load(i)) {
+#pragma unroll
+        for (int k = 0; k < kUnroll; k++) {
+            const size_t j = i + k * kStride;
+            const T zi = dv[k] * rv[k];
+            if (j < n) p[j] = beta * pv[k] + zi;
+        }
+    }
 }
 
 template <typename T>
@@ -384,11 +474,13 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long m) {
 // finish (counted in the low word of w[1]) reduces them, writes w[0] and
 // resets the counter, so one launch does it all and repeats cleanly inside a
 // captured graph. The maximum is exact, hence independent of the order.
-__global__ void __launch_bounds__(kRedThreads) k_umax(const double* __restrict__ u, const uint8_t* __restrict__ mask,
-                                                      size_t n, double* __restrict__ vz, size_t nv,
-                                                      unsigned long long* __restrict__ w) {
+__global__ void __launch_bounds__(kRedThreads) k_umax(const double* u, const uint8_t* mask,
+                                                      size_t n, double* vz, size_t nv,
+                                                      unsigned long long* w) {
     __shared__ unsigned long long sh[kRedThreads / 32];
     __shared__ bool last;
+    release_next();
+    wait_launch();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long m = 0;
@@ -456,12 +548,12 @@ __global__ void __launch_bounds__(kRedThreads) k_umax_cols(const double* __restr
 // next one added), one thread per shared DoF. Waits for the patch launch
 // (programmatic dependence) before reading.
 template <typename VO>
-__global__ void __launch_bounds__(kRedThreads) k_patch_combine(VO* __restrict__ v, const VO* __restrict__ pv,
-                                                               const uint32_t* __restrict__ dof,
-                                                               const uint32_t* __restrict__ off,
-                                                               const uint32_t* __restrict__ idx, uint32_t nb,
-                                                               const VO* __restrict__ u_rows) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+__global__ void __launch_bounds__(kRedThreads) k_patch_combine(VO* v, const VO* pv,
+                                                               const uint32_t* dof,
+                                                               const uint32_t* off,
+                                                               const uint32_t* idx, uint32_t nb,
+                                                               const VO* u_rows) {
+    wait_launch();
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += stride) {
         const uint32_t d = dof[i] & kDofMask;
@@ -476,46 +568,101 @@ __global__ void __launch_bounds__(kRedThreads) k_patch_combine(VO* __restrict__ 
     }
 }
 
+// The same over every DoF, with the partials of v.u: pos[d] = the DoF's place
+// in the combine lists, or kNoElement (v[d] is there already).
+template <typename VO>
+__global__ void __launch_bounds__(kRedThreads) k_patch_combine_dot(VO* v, const VO* pv,
+                                                                   const uint32_t* pos,
+                                                                   const uint32_t* dof,
+                                                                   const uint32_t* off,
+                                                                   const uint32_t* idx, uint32_t n,
+                                                                   const VO* u, double* part) {
+    __shared__ double sh[kRedThreads];
+    release_next();
+    DotAcc<VO> acc;
+    const uint32_t stride = gridDim.x * kRedThreads;
+    bool waited = false;
+    for (uint32_t d = blockIdx.x * kRedThreads + threadIdx.x; d < n; d += stride) {
+        const uint32_t i = __ldg(pos + d);
+        const bool sum = i != kNoElement;
+        const bool fixed = sum && (__ldg(dof + i) & kBcFlag) != 0;
+        const uint32_t k0 = sum ? __ldg(off + i) : 0u, k1 = sum ? __ldg(off + i + 1) : 0u;
+        if (!waited) {
+            wait_launch();
+            waited = true;
+        }
+        const VO ud = u[d];
+        VO s;
+        if (!sum) {
+            s = v[d];
+        } else {
+            s = fixed ? ud : pv[idx[k0]];
+            if (!fixed)
+                for (uint32_t k = k0 + 1; k < k1; k++) s += pv[idx[k]];
+            v[d] = s;
+        }
+        acc.add(s, ud);
+    }
+    if (!waited) wait_launch();
+    const double t[1] = {acc.value()};
+    block_partials(t, sh, part);
+}
+
 // Gather pass of a plan whose elements run in one launch (launch_gather_sum):
 // one thread per DoF; lists and mask are constant, so they load before the
-// wait for the element launch.
-template <typename VO, typename VT, uint32_t B>
-__global__ void __launch_bounds__(kRedThreads) k_gather_sum(VT* __restrict__ v, const VO* __restrict__ ve,
-                                                            const uint32_t* __restrict__ off,
-                                                            const uint32_t* __restrict__ idx, uint32_t n,
-                                                            const VT* __restrict__ u, const uint8_t* __restrict__ mask) {
+// wait for the element launch. DOT: the partials of v.u too, kRedBlocks blocks
+// at most.
+template <typename VO, typename VT, uint32_t B, bool DOT>
+__global__ void __launch_bounds__(kRedThreads) k_gather_sum(VT* v, const VO* ve,
+                                                            const uint32_t* off,
+                                                            const uint32_t* idx, uint32_t n,
+                                                            const VT* u, const uint8_t* mask,
+                                                            double* part) {
     constexpr int kAhead = 8;  // entries in flight per thread
-    const uint32_t d = blockIdx.x * kRedThreads + threadIdx.x;
-    const uint32_t m = d / B, c = d - m * B;
-    const bool live = d < n;
-    const uint32_t k0 = live ? __ldg(off + m) : 0u, k1 = live ? __ldg(off + m + 1) : 0u;
-    const bool fixed = live && mask && mask[d];
-    uint32_t at[kAhead];
+    __shared__ double sh[DOT ? kRedThreads : 1];
+    if constexpr (DOT) release_next();
+    DotAcc<VT> acc;
+    bool waited = false;
+    for (uint32_t d = blockIdx.x * kRedThreads + threadIdx.x; d < n; d += gridDim.x * kRedThreads) {
+        const uint32_t m = d / B, c = d - m * B;
+        const uint32_t k0 = __ldg(off + m), k1 = __ldg(off + m + 1);
+        const bool fixed = mask && mask[d];
+        uint32_t at[kAhead];
 #pragma unroll
-    for (int q = 0; q < kAhead; q++) at[q] = k0 + q < k1 ? __ldg(idx + k0 + q) : 0u;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!live) return;
-    if (fixed) {
-        v[d] = u[d];
-        return;
+        for (int q = 0; q < kAhead; q++) at[q] = k0 + q < k1 ? __ldg(idx + k0 + q) : 0u;
+        if (!waited) {
+            wait_launch();
+            waited = true;
+        }
+        VT ud = VT(0);
+        if (DOT || fixed) ud = u[d];
+        VO s = VO(0);
+        if (!fixed) {
+            VO x[kAhead];
+#pragma unroll
+            for (int q = 0; q < kAhead; q++) x[q] = k0 + q < k1 ? __ldcg(ve + at[q] + c) : VO(0);
+#pragma unroll
+            for (int q = 0; q < kAhead; q++)
+                if (k0 + q < k1) s += x[q];
+            for (uint32_t k = k0 + kAhead; k < k1; k += kAhead) {
+#pragma unroll
+                for (int q = 0; q < kAhead; q++) at[q] = k + q < k1 ? __ldg(idx + k + q) : 0u;
+#pragma unroll
+                for (int q = 0; q < kAhead; q++) x[q] = k + q < k1 ? __ldcg(ve + at[q] + c) : VO(0);
+#pragma unroll
+                for (int q = 0; q < kAhead; q++)
+                    if (k + q < k1) s += x[q];
+            }
+        }
+        const VT out = fixed ? ud : (VT)s;
+        v[d] = out;
+        if constexpr (DOT) acc.add(out, ud);
     }
-    VO s = VO(0);
-    VO x[kAhead];
-#pragma unroll
-    for (int q = 0; q < kAhead; q++) x[q] = k0 + q < k1 ? __ldcg(ve + at[q] + c) : VO(0);
-#pragma unroll
-    for (int q = 0; q < kAhead; q++)
-        if (k0 + q < k1) s += x[q];
-    for (uint32_t k = k0 + kAhead; k < k1; k += kAhead) {
-#pragma unroll
-        for (int q = 0; q < kAhead; q++) at[q] = k + q < k1 ? __ldg(idx + k + q) : 0u;
-#pragma unroll
-        for (int q = 0; q < kAhead; q++) x[q] = k + q < k1 ? __ldcg(ve + at[q] + c) : VO(0);
-#pragma unroll
-        for (int q = 0; q < kAhead; q++)
-            if (k + q < k1) s += x[q];
+    if (!waited) wait_launch();
+    if constexpr (DOT) {
+        const double t[1] = {acc.value()};
+        block_partials(t, sh, part);
     }
-    v[d] = (VT)s;
 }
 
 inline unsigned grid_for(size_t n) {
@@ -543,22 +690,44 @@ cudaError_t launch_cg_init(const T* b, const T* q, const T* dinv, T* r, T* z, T*
     return cudaGetLastError();
 }
 
+namespace {
+// A launch of kRedThreads-thread blocks, with programmatic dependence on the
+// launch before it if pdl.
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), uint32_t blocks, bool pdl, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kRedThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// Blocks of a CG iteration's launches: a DoF per thread while that fits
+// kRedBlocks (a function of n only).
+uint32_t cg_blocks(size_t n) {
+    const size_t b = (n + kRedThreads - 1) / kRedThreads;
+    return (uint32_t)(b < 1 ? 1 : b > (size_t)kRedBlocks ? (size_t)kRedBlocks : b);
+}
+}  // namespace
+
 template <typename T>
-cudaError_t launch_cg_alpha(const T* p, const T* q, size_t n, double* sc, double* part, cudaStream_t st) {
-    const uint32_t nb = red_blocks(n);
-    k_dot<T><<<nb, kRedThreads, 0, st>>>(p, q, n, part);
-    k_cg_alpha<<<1, kRedThreads, 0, st>>>(sc, part, nb);
-    return cudaGetLastError();
+cudaError_t launch_dot(const T* a, const T* b, size_t n, double* part, uint32_t* nb, bool pdl, cudaStream_t st) {
+    *nb = red_blocks(n);
+    return launch(k_dot<T>, *nb, pdl, st, a, b, n, part);
 }
 
 template <typename T>
-cudaError_t launch_cg_update(T* x, T* r, T* z, T* p, const T* q, const T* dinv, size_t n, double* sc, double* part,
-                             cudaStream_t st) {
-    const uint32_t nb = red_blocks(n);
-    k_cg_update<T><<<nb, kRedThreads, 0, st>>>(x, r, z, p, q, dinv, n, sc, part);
-    k_cg_beta<<<1, kRedThreads, 0, st>>>(sc, part, nb);
-    k_cg_p<T><<<grid_for(n), kRedThreads, 0, st>>>(p, z, n, sc);
-    return cudaGetLastError();
+cudaError_t launch_cg_iteration(T* x, T* r, T* p, const T* q, const T* dinv, size_t n, const double* in, double* out,
+                                double* part, uint32_t nb_pq, cudaStream_t st) {
+    const uint32_t nb = cg_blocks(n);
+    const cudaError_t e = launch(k_cg_xr<T>, nb, true, st, x, r, p, q, dinv, n, in, out, part, nb_pq, part + kRedBlocks);
+    if (e != cudaSuccess) return e;
+    return launch(k_cg_p<T>, nb, true, st, p, r, dinv, n, in, out, part + kRedBlocks, nb);
 }
 
 template <typename T>
@@ -617,54 +786,57 @@ cudaError_t launch_add_f32(double* x, double* d, size_t n, cudaStream_t st, doub
 cudaError_t launch_patch_combine(int vo_bytes, void* v, const void* pv, const uint32_t* dof, const uint32_t* off,
                                  const uint32_t* idx, uint32_t nb, const void* u_rows, cudaStream_t st) {
     if (nb == 0) return cudaSuccess;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid_for(nb));
-    cfg.blockDim = dim3(kRedThreads);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     if (vo_bytes == 8)
-        return cudaLaunchKernelEx(&cfg, k_patch_combine<double>, static_cast<double*>(v),
-                                  static_cast<const double*>(pv), dof, off, idx, nb,
-                                  static_cast<const double*>(u_rows));
-    return cudaLaunchKernelEx(&cfg, k_patch_combine<float>, static_cast<float*>(v), static_cast<const float*>(pv),
-                              dof, off, idx, nb, static_cast<const float*>(u_rows));
+        return launch(k_patch_combine<double>, grid_for(nb), true, st, static_cast<double*>(v),
+                      static_cast<const double*>(pv), dof, off, idx, nb, static_cast<const double*>(u_rows));
+    return launch(k_patch_combine<float>, grid_for(nb), true, st, static_cast<float*>(v),
+                  static_cast<const float*>(pv), dof, off, idx, nb, static_cast<const float*>(u_rows));
+}
+
+cudaError_t launch_patch_combine_dot(int vo_bytes, void* v, const void* pv, const uint32_t* pos, const uint32_t* dof,
+                                     const uint32_t* off, const uint32_t* idx, uint32_t n, const void* u, double* part,
+                                     uint32_t* nb, cudaStream_t st) {
+    *nb = cg_blocks(n);
+    if (vo_bytes == 8)
+        return launch(k_patch_combine_dot<double>, *nb, true, st, static_cast<double*>(v),
+                      static_cast<const double*>(pv), pos, dof, off, idx, n, static_cast<const double*>(u), part);
+    return launch(k_patch_combine_dot<float>, *nb, true, st, static_cast<float*>(v), static_cast<const float*>(pv),
+                  pos, dof, off, idx, n, static_cast<const float*>(u), part);
 }
 
 namespace {
+template <typename VO, typename VT, uint32_t B>
+cudaError_t gather_sum(void* v, const void* ve, const uint32_t* off, const uint32_t* idx, uint32_t n, const void* u,
+                       const uint8_t* mask, double* part, uint32_t* nb, cudaStream_t st) {
+    const uint32_t all = (n + kRedThreads - 1) / kRedThreads;
+    VT* const vt = static_cast<VT*>(v);
+    const VO* const vo = static_cast<const VO*>(ve);
+    const VT* const ut = static_cast<const VT*>(u);
+    if (!part) return launch(k_gather_sum<VO, VT, B, false>, all, true, st, vt, vo, off, idx, n, ut, mask, part);
+    *nb = cg_blocks(n);
+    return launch(k_gather_sum<VO, VT, B, true>, *nb, true, st, vt, vo, off, idx, n, ut, mask, part);
+}
 template <typename VO, typename VT>
-cudaError_t gather_sum(uint32_t b, void* v, const void* ve, const uint32_t* off, const uint32_t* idx, uint32_t n,
-                       const void* u, const uint8_t* mask, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n + kRedThreads - 1) / kRedThreads);
-    cfg.blockDim = dim3(kRedThreads);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, b == 3 ? k_gather_sum<VO, VT, 3> : k_gather_sum<VO, VT, 1>, static_cast<VT*>(v),
-                              static_cast<const VO*>(ve), off, idx, n, static_cast<const VT*>(u), mask);
+cudaError_t gather_sum_b(uint32_t b, void* v, const void* ve, const uint32_t* off, const uint32_t* idx, uint32_t n,
+                         const void* u, const uint8_t* mask, double* part, uint32_t* nb, cudaStream_t st) {
+    return b == 3 ? gather_sum<VO, VT, 3>(v, ve, off, idx, n, u, mask, part, nb, st)
+                  : gather_sum<VO, VT, 1>(v, ve, off, idx, n, u, mask, part, nb, st);
 }
 }  // namespace
 
 cudaError_t launch_gather_sum(int ve_bytes, int vt_bytes, uint32_t b, void* v, const void* ve, const uint32_t* off,
-                              const uint32_t* idx, uint32_t n_dofs, const void* u, const uint8_t* mask,
-                              cudaStream_t st) {
-    if (n_dofs == 0) return cudaSuccess;
-    if (ve_bytes == 8 && vt_bytes == 8) return gather_sum<double, double>(b, v, ve, off, idx, n_dofs, u, mask, st);
-    if (ve_bytes == 8) return gather_sum<double, float>(b, v, ve, off, idx, n_dofs, u, mask, st);
-    return gather_sum<float, float>(b, v, ve, off, idx, n_dofs, u, mask, st);
+                              const uint32_t* idx, uint32_t n, const void* u, const uint8_t* mask, double* part,
+                              uint32_t* nb, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    if (ve_bytes == 8 && vt_bytes == 8)
+        return gather_sum_b<double, double>(b, v, ve, off, idx, n, u, mask, part, nb, st);
+    if (ve_bytes == 8) return gather_sum_b<double, float>(b, v, ve, off, idx, n, u, mask, part, nb, st);
+    return gather_sum_b<float, float>(b, v, ve, off, idx, n, u, mask, part, nb, st);
 }
 
 cudaError_t launch_umax(const double* u, const uint8_t* mask, size_t n, double* vz, size_t nv,
-                        unsigned long long* w, cudaStream_t st) {
-    k_umax<<<red_blocks(n > nv ? n : nv), kRedThreads, 0, st>>>(u, mask, n, vz, nv, w);
-    return cudaGetLastError();
+                        unsigned long long* w, bool pdl, cudaStream_t st) {
+    return launch(k_umax, red_blocks(n > nv ? n : nv), pdl, st, u, mask, n, vz, nv, w);
 }
 
 cudaError_t launch_umax_cols(const double* U, const uint8_t* mask, size_t rows, uint32_t R, uint32_t ld,
@@ -680,9 +852,9 @@ cudaError_t launch_umax_cols(const double* U, const uint8_t* mask, size_t rows, 
     template cudaError_t launch_set_constrained<T>(T*, const T*, const uint32_t*, uint32_t, cudaStream_t);            \
     template cudaError_t launch_cg_init<T>(const T*, const T*, const T*, T*, T*, T*, size_t, double*, double*,        \
                                            cudaStream_t);                                                             \
-    template cudaError_t launch_cg_alpha<T>(const T*, const T*, size_t, double*, double*, cudaStream_t);              \
-    template cudaError_t launch_cg_update<T>(T*, T*, T*, T*, const T*, const T*, size_t, double*, double*,            \
-                                             cudaStream_t);                                                           \
+    template cudaError_t launch_dot<T>(const T*, const T*, size_t, double*, uint32_t*, bool, cudaStream_t);           \
+    template cudaError_t launch_cg_iteration<T>(T*, T*, T*, const T*, const T*, size_t, const double*, double*,       \
+                                                double*, uint32_t, cudaStream_t);                                     \
     template cudaError_t launch_invert<T>(T*, const double*, size_t, cudaStream_t);                                   \
     template cudaError_t launch_norm2<T>(const T*, size_t, double*, double*, cudaStream_t);
 

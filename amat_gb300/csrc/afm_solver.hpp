@@ -9,6 +9,10 @@ namespace afm {
 
 constexpr int kRedBlocks = 512;
 constexpr int kRedThreads = 256;
+// Products of at most this many DoFs leave the partials of p.q in the pass
+// that writes q (two DoFs per thread of kRedBlocks blocks); a larger one's
+// separate pass over p and q costs less than that pass loses in parallelism.
+constexpr uint32_t kFusedDotDofs = 2u * kRedBlocks * kRedThreads;
 
 // Blocks of a reduction over n entries: about 2048 entries per block, at
 // least 1 and at most kRedBlocks (a function of n only: deterministic sums).
@@ -29,9 +33,13 @@ inline uint32_t red_blocks(size_t n) {
 // orthogonalisation coefficient.
 enum : int {
     S_RZ = 0, S_PQ, S_ALPHA, S_BETA, S_RR, S_ZZ, S_BB, S_DB, S_FLAG,
-    S_DONE, S_TOL, S_ITER, S_MAXIT, S_NORM, S_RZOLD, S_GAMMA,
-    kScalarSlots = 16
+    S_DONE, S_TOL, S_ITER, S_MAXIT, S_NORM, S_RZOLD, S_GAMMA, S_BREAK,
+    kScalarSlots = 18
 };
+// An iteration reads one set of scalars and writes the other (see
+// launch_cg_iteration), so the state is two sets; every other kernel and the
+// host use the first, which an even number of iterations ends on.
+constexpr int kScalarSets = 2;
 constexpr int kPartialSlots = 5 * kRedBlocks;
 
 // T = double (FP64 CG) or float (inner CG of the mixed-precision solve);
@@ -42,11 +50,18 @@ cudaError_t launch_set_constrained(T* v, const T* u, const uint32_t* idx, uint32
 template <typename T>
 cudaError_t launch_cg_init(const T* b, const T* q, const T* dinv, T* r, T* z, T* p, size_t n, double* sc,
                            double* part, cudaStream_t st);
+// Partial sums of a.b, one per block (returned in *nb), for launch_cg_iteration.
 template <typename T>
-cudaError_t launch_cg_alpha(const T* p, const T* q, size_t n, double* sc, double* part, cudaStream_t st);
+cudaError_t launch_dot(const T* a, const T* b, size_t n, double* part, uint32_t* nb, bool pdl, cudaStream_t st);
+// The rest of a CG iteration after the product q = A p and the nb_pq partials
+// of p.q in part: x += alpha p, r -= alpha q, p = dinv r + beta p, in two
+// launches whose blocks each add up the partials of the launch before (so that
+// no one-block launch stands between them): reads the scalars of set `in`,
+// writes set `out` (kScalarSlots each). part: nb_pq partials of p.q, then
+// kRedBlocks x 3 partials of the second launch's sums.
 template <typename T>
-cudaError_t launch_cg_update(T* x, T* r, T* z, T* p, const T* q, const T* dinv, size_t n, double* sc, double* part,
-                             cudaStream_t st);
+cudaError_t launch_cg_iteration(T* x, T* r, T* p, const T* q, const T* dinv, size_t n, const double* in, double* out,
+                                double* part, uint32_t nb_pq, cudaStream_t st);
 template <typename T>
 cudaError_t launch_invert(T* dinv, const double* d, size_t n, cudaStream_t st);
 // sc[S_PQ] = ||a||^2 (no CG bookkeeping)
@@ -82,8 +97,9 @@ constexpr int kUscColsOffset = 2 + kRedBlocks;
 // w[0] = max over the unmasked i < n of |u[i]| (double bits) and vz[0 .. nv) =
 // 0, in one launch (mask may be null; w[1] must be 0 before the first launch
 // and is left 0).
+// pdl: programmatic dependence on the launch before it.
 cudaError_t launch_umax(const double* u, const uint8_t* mask, size_t n, double* vz, size_t nv,
-                        unsigned long long* w, cudaStream_t st);
+                        unsigned long long* w, bool pdl, cudaStream_t st);
 // cm[j] = max over the unmasked rows of |U(:, j)|, j < R <= kMaxUmaxCols.
 cudaError_t launch_umax_cols(const double* U, const uint8_t* mask, size_t rows, uint32_t R, uint32_t ld,
                              unsigned long long* cm, cudaStream_t st);
