@@ -28,6 +28,7 @@
 #include "afm_internal.hpp"
 #include "afm_mixed.hpp"
 #include "afm_shape.hpp"
+#include "afm_batched_patch.hpp"
 #include "afm_solver.hpp"
 
 namespace afm {
@@ -234,6 +235,13 @@ void free_device(afm_operator* op) {
     drop_graph(op->bcg64);
     drop_graph(op->bcg32);
     op->batch_tune.clear();
+    dfree(op, op->d_bp_hdr);
+    dfree(op, op->d_bp_dof);
+    dfree(op, op->d_bp_off);
+    dfree(op, op->d_bp_idx);
+    dfree(op, op->d_bp_pv);
+    op->bp_state = 0;
+    op->bp_pv_bytes = 0;
     dfree(op, op->d_bwork);
     dfree(op, op->d_bsc);
     op->bwork_elems = 0;
@@ -246,9 +254,7 @@ void free_device(afm_operator* op) {
     dfree(op, op->d_bc_val);
     dfree(op, op->d_bcmask);
     dfree(op, op->d_gbar);
-    dfree(op, op->d_gather_off);
-    dfree(op, op->d_gather_idx);
-    dfree(op, op->d_ve);
+    dfree(op, op->d_ve);  // (and the gather lists)
     op->gather_b = 0;
     op->ve_stream = nullptr;
     op->fused_ok = false;
@@ -689,37 +695,44 @@ int build_gather(afm_operator* op, uint32_t n, const std::vector<uint32_t>& colo
     }
     const uint32_t b = nodes3 ? 3 : 1, lists = op->n_dofs / b, per = n / b;
     std::vector<uint32_t> off((size_t)lists + 1, 0), idx(entries / b);
-    for (uint64_t k = 0; k < entries; k += b) off[op->map[k] / b + 1]++;
-    for (uint32_t m = 0; m < lists; m++) off[m + 1] += off[m];
-    std::vector<uint32_t> fill(off.begin(), off.end() - 1);
-    for (size_t c = 0; c + 1 < color_first.size(); c++) {
-        // elements of one colour share no DoF: their lists are filled side by side
-#pragma omp parallel for schedule(static)
-        for (int64_t p = color_first[c]; p < (int64_t)color_first[c + 1]; p++) {
-            const uint32_t* m = op->map.data() + op->offsets[op->perm[p]];
-            for (uint32_t j = 0; j < per; j++) idx[fill[m[j * b] / b]++] = (uint32_t)p * n + j * b;
+    for (int pass = 0; pass < 2; pass++) {
+        std::vector<uint32_t> fill(off.begin(), off.end() - 1);
+        for (size_t c = 0; c + 1 < color_first.size(); c++) {
+            // elements of one colour share no DoF: their lists are filled side by side
+#pragma omp parallel for schedule(static) if (color_first[c + 1] - color_first[c] > 1024)
+            for (int64_t p = color_first[c]; p < (int64_t)color_first[c + 1]; p++) {
+                const uint32_t* m = op->map.data() + op->offsets[op->perm[p]];
+                for (uint32_t j = 0; j < per; j++) {
+                    if (pass == 0)
+                        off[m[j * b] / b + 1]++;
+                    else
+                        idx[fill[m[j * b] / b]++] = (uint32_t)p * n + j * b;
+                }
+            }
         }
+        if (pass == 0)
+            for (uint32_t m = 0; m < lists; m++) off[m + 1] += off[m];
     }
-    AFM_CUDA(dalloc(op, &op->d_gather_off, sizeof(uint32_t) * off.size()));
-    AFM_CUDA(dalloc(op, &op->d_gather_idx, sizeof(uint32_t) * idx.size()));
-    AFM_CUDA(dalloc(op, &op->d_ve, (gather_pays(op, false, 8) ? 8 : 4) * entries));
+    // one allocation: the products, then the lists and their offsets
+    const size_t ve_bytes = ((gather_pays(op, false, 8) ? 8 : 4) * entries + 15) / 16 * 16;
+    AFM_CUDA(dalloc(op, &op->d_ve, ve_bytes + sizeof(uint32_t) * (idx.size() + off.size())));
+    op->d_gather_idx = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(op->d_ve) + ve_bytes);
+    op->d_gather_off = op->d_gather_idx + idx.size();
     AFM_CUDA(cudaMemcpyAsync(op->d_gather_off, off.data(), sizeof(uint32_t) * off.size(), cudaMemcpyHostToDevice,
                              op->stream));
     AFM_CUDA(cudaMemcpyAsync(op->d_gather_idx, idx.data(), sizeof(uint32_t) * idx.size(), cudaMemcpyHostToDevice,
-                             op->stream));
-    AFM_CUDA(cudaStreamSynchronize(op->stream));
+                             op->stream));  // (pageable memory: staged before the call returns)
     op->gather_b = b;
     return AFM_SUCCESS;
 }
 
-// Whether a product (wide: 8-byte staged u) enqueued on st may use the element-product buffer, which
+// Whether a product enqueued on st may use the element-product (or batched combine) buffer, which
 // the operator's products share. A product on another stream than the one
 // before waits for that one's end; inside a caller's own capture, whose graph
 // may be replayed beside other products, the colour launches (no shared
 // buffer) run instead.
-int gather_ready(afm_operator* op, bool wide, uint32_t ve_bytes, cudaStream_t st, bool* use) {
+int buffer_ready(afm_operator* op, cudaStream_t st, bool* use) {
     *use = false;
-    if (!op->gather_b || !gather_pays(op, wide, ve_bytes)) return AFM_SUCCESS;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     AFM_CUDA(cudaStreamIsCapturing(st, &cap));
     const bool own = op->own_capture && st == op->stream;  // after a product of the same solve on this stream
@@ -739,7 +752,13 @@ int gather_ready(afm_operator* op, bool wide, uint32_t ve_bytes, cudaStream_t st
     return AFM_SUCCESS;
 }
 
-int gather_done(afm_operator* op, cudaStream_t st) {
+int gather_ready(afm_operator* op, bool wide, uint32_t ve_bytes, cudaStream_t st, bool* use) {
+    *use = false;
+    if (!op->gather_b || !gather_pays(op, wide, ve_bytes)) return AFM_SUCCESS;
+    return buffer_ready(op, st, use);
+}
+
+int buffer_done(afm_operator* op, cudaStream_t st) {
     if (st == op->stream) return AFM_SUCCESS;
     if (!op->ve_event) AFM_CUDA(cudaEventCreateWithFlags(&op->ve_event, cudaEventDisableTiming));
     AFM_CUDA(cudaEventRecord(op->ve_event, st));
@@ -960,7 +979,7 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
         AFM_CUDA(launch_gather_sum(vb, vb, op->gather_b, d_v, op->d_ve, op->d_gather_off, op->d_gather_idx, op->n_dofs,
                                    d_u, tail ? op->d_bcmask : nullptr, part, tail ? &tail->nb : nullptr, st));
         if (tail) tail->bc_done = true;
-        return gather_done(op, st);
+        return buffer_done(op, st);
     }
     AFM_CUDA(cudaMemsetAsync(d_v, 0, (size_t)op->n_dofs * vb, st));
     for (size_t c = 0; c + 1 < op->free_color_first.size(); c++) {
@@ -1037,7 +1056,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
                                    op->d_gather_off, op->d_gather_idx, op->n_dofs, d_u_in,
                                    tail ? op->d_bcmask : nullptr, part, tail ? &tail->nb : nullptr, st));
         if (tail) tail->bc_done = true;
-        return gather_done(op, st);
+        return buffer_done(op, st);
     }
     // one launch over every patch and its combine pass write every DoF that an element lists; else v = 0, and
     // for a segment plan max|u| for the launches' power-of-two u scale, in one launch before the first element
@@ -1163,10 +1182,107 @@ cudaStream_t pick_stream(afm_operator* op, void* stream) {
 
 // ---- batched (multi right-hand side) products ------------------------------
 
+constexpr int kPatchTile = -1;  // "columns of the lane tile" of the patch plan
+
+// The patch plan of the batched product, where the elements have one size that
+// its kernel takes in this arithmetic and list no DoF twice; and its combine
+// buffer for nrhs columns. Call outside stream capture.
+int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, cudaStream_t st, bool* usable) {
+    *usable = false;
+    if (op->bp_state < 0 || (!f32 && op->precision != AFM_PREC_FP64_SPLIT)) return AFM_SUCCESS;
+    if (op->bp_state == 0) {
+        op->bp_state = -1;
+        if (op->dup_in_element || op->segs.empty()) return AFM_SUCCESS;
+        const uint32_t n = op->segs[0].n;
+        for (const Segment& s : op->segs)
+            if (s.n != n || s.regime != REG_WPE) return AFM_SUCCESS;
+        if (!bpatch_supported(n, true) && !bpatch_supported(n, false)) return AFM_SUCCESS;
+        std::vector<uint32_t> first;
+        for (const Segment& s : op->segs) first.push_back((uint32_t)s.first_pos);
+        first.push_back(op->n_elem);
+        std::vector<uint8_t> is_bc(op->n_dofs, 0);
+        for (uint32_t d : op->bc_unique) is_bc[d] = 1;
+        BPatchPlanHost plan;
+        build_bpatch_plan(op->n_elem, op->n_dofs, n, op->map.data(), op->perm.data(), first, is_bc.data(), plan);
+        AFM_CUDA(dalloc(op, &op->d_bp_hdr, std::max<size_t>(plan.hdr.size(), 16)));
+        AFM_CUDA(dalloc(op, &op->d_bp_dof, sizeof(uint32_t) * std::max<size_t>(plan.shared_dof.size(), 1)));
+        AFM_CUDA(dalloc(op, &op->d_bp_off, sizeof(uint32_t) * plan.shared_off.size()));
+        AFM_CUDA(dalloc(op, &op->d_bp_idx, sizeof(uint32_t) * std::max<size_t>(plan.shared_idx.size(), 1)));
+        auto up = [&](void* d, const void* h, size_t bytes) {
+            return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, op->stream);
+        };
+        AFM_CUDA(up(op->d_bp_hdr, plan.hdr.data(), plan.hdr.size()));
+        AFM_CUDA(up(op->d_bp_dof, plan.shared_dof.data(), sizeof(uint32_t) * plan.shared_dof.size()));
+        AFM_CUDA(up(op->d_bp_off, plan.shared_off.data(), sizeof(uint32_t) * plan.shared_off.size()));
+        AFM_CUDA(up(op->d_bp_idx, plan.shared_idx.data(), sizeof(uint32_t) * plan.shared_idx.size()));
+        AFM_CUDA(cudaStreamSynchronize(op->stream));
+        op->bp_n = n;
+        op->bp_patches = plan.geom.patches;
+        op->bp_max_rows = plan.geom.max_rows;
+        op->bp_pv_rows = plan.geom.pv_rows;
+        op->bp_shared = plan.geom.shared;
+        op->bp_state = 1;
+    }
+    if (!bpatch_supported(op->bp_n, f32)) return AFM_SUCCESS;
+    const size_t bytes = std::max<size_t>((size_t)op->bp_pv_rows * nrhs * (f32 ? 4 : 8), 16);
+    if (op->bp_pv_bytes < bytes) {
+        // products on other streams may still read the old buffer
+        if (op->ve_stream && op->ve_stream != op->stream && op->ve_event)
+            AFM_CUDA(cudaStreamWaitEvent(op->stream, op->ve_event, 0));
+        dfree(op, op->d_bp_pv);
+        op->bp_pv_bytes = 0;
+        if (cudaMallocAsync((void**)&op->d_bp_pv, bytes, op->stream) != cudaSuccess) {
+            cudaGetLastError();  // no room: the launches per colour need none
+            op->d_bp_pv = nullptr;
+            return AFM_SUCCESS;
+        }
+        op->bp_pv_bytes = bytes;
+        op->generation++;  // captured iterations hold the old buffer
+    }
+    if (st != op->stream) AFM_CUDA(cudaStreamSynchronize(op->stream));  // (the plan and the buffer are there)
+    *usable = true;
+    return AFM_SUCCESS;
+}
+
+// tr = kPatchTile: the patch plan (ensure_bpatch), in the arithmetic it was made usable for.
 int enqueue_matvec_batched(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, uint32_t ld, int bc_mode,
                            cudaStream_t st, bool f32, int tr, int ng) {
     const int kprec = f32 ? AFM_PREC_FP32 : op->precision;
     const size_t vb = (kprec == AFM_PREC_FP32 ? 4 : 8);
+    if (tr == kPatchTile) {
+        bool use = false;
+        if (int s = buffer_ready(op, st, &use)) return s;
+        if (use) {
+            if (op->n_unlisted) AFM_CUDA(cudaMemsetAsync(d_V, 0, (size_t)op->n_dofs * ld * vb, st));
+            if (!f32)
+                AFM_CUDA(launch_umax_cols(static_cast<const double*>(d_U), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
+                                          nrhs, ld, op->d_usc + kUscColsOffset, st));
+            BPatchGeom g;
+            g.n = op->bp_n;
+            g.patches = op->bp_patches;
+            g.max_rows = op->bp_max_rows;
+            g.hdr_bytes = bpatch_hdr_bytes(g.n, g.max_rows);
+            g.pv_rows = op->bp_pv_rows;
+            g.shared = op->bp_shared;
+            BPatchArgs a;
+            a.hdr = op->d_bp_hdr;
+            a.ke = op->d_ke;
+            a.unit_bytes = op->segs[0].unit_bytes;
+            a.plane = op->segs[0].plane;
+            a.u = d_U;
+            a.v = d_V;
+            a.pv = op->d_bp_pv;
+            a.nrhs = nrhs;
+            a.ld = ld;
+            a.bc_mode = bc_mode;
+            a.umax = op->d_usc + kUscColsOffset;
+            AFM_CUDA(launch_bpatch(g, a, f32, op->d_bp_dof, op->d_bp_off, op->d_bp_idx, op->sm_count, st));
+            return buffer_done(op, st);
+        }
+        // a caller's capture: the launches per colour, with the tile tuned for them
+        tr = nrhs % 8 == 0 ? 8 : 4;
+        ng = 4;
+    }
     AFM_CUDA(cudaMemsetAsync(d_V, 0, (size_t)op->n_dofs * ld * vb, st));
     // split arithmetic: max|U(:, j)| of every column for the per-column u scale
     if (kprec == AFM_PREC_FP64_SPLIT)
@@ -1241,12 +1357,21 @@ int batch_tuning(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, ui
                  int* tr, int* ng, bool allow_tc = true) {
     const int kprec = f32 ? AFM_PREC_FP32 : op->precision;
     const uint64_t key = ((uint64_t)nrhs << 40) | ((uint64_t)ld << 8) | (uint64_t)kprec | (allow_tc ? 0u : 0x80u);
+    bool patch = false;
     for (const auto& t : op->batch_tune)
         if (t.key == key) {
-            *tr = t.tr;
+            *tr = t.patch ? kPatchTile : t.tr;
             *ng = t.ng;
+            if (t.patch) {  // (its combine buffer may have been made for fewer columns)
+                cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+                AFM_CUDA(cudaStreamIsCapturing(st, &cap));
+                if (cap == cudaStreamCaptureStatusNone)
+                    if (int s = ensure_bpatch(op, nrhs, f32, st, &patch)) return s;
+                if (!patch) *tr = t.tr;
+            }
             return AFM_SUCCESS;
         }
+    if (int s = ensure_bpatch(op, nrhs, f32, st, &patch)) return s;
     // (columns, rows) of the lane tile; (0, 0): the tensor-core kernel (FP32 products)
     std::vector<std::pair<int, int>> cand = {{8, 6}, {8, 4}, {8, 2}, {4, 4}};
     if (f32 && allow_tc && batched_tc_all(op, nrhs)) cand.insert(cand.begin(), {0, 0});
@@ -1255,31 +1380,43 @@ int batch_tuning(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, ui
     cudaEventCreate(&e1);
     float best = 1e30f;
     int btr = 4, bng = 2;
+    // products of a candidate after others of it (its status); *ms is lowered to the time of one
+    // (one after one where the patch plan will most likely beat them all)
+    const int warm = patch ? 1 : 2, runs = patch ? 1 : 3;
+    auto time = [&](int ct, int rt, float* ms) {
+        for (int r = 0; r < warm; r++)
+            if (int s = enqueue_matvec_batched(op, d_V, d_U, nrhs, ld, 0, st, f32, ct, rt)) return s;
+        cudaEventRecord(e0, st);
+        for (int r = 0; r < runs; r++) enqueue_matvec_batched(op, d_V, d_U, nrhs, ld, 0, st, f32, ct, rt);
+        cudaEventRecord(e1, st);
+        cudaEventSynchronize(e1);
+        float t = 0.f;
+        cudaEventElapsedTime(&t, e0, e1);
+        *ms = std::min(*ms, t / (float)runs);
+        return (int)AFM_SUCCESS;
+    };
     for (auto c : cand) {
         if (c.first != 0 && nrhs % (uint32_t)c.first) continue;  // a lane tile must divide the columns
-        int s = enqueue_matvec_batched(op, d_V, d_U, nrhs, ld, 0, st, f32, c.first, c.second);  // warm-up
-        if (s) {
+        const float before = best;
+        if (time(c.first, c.second, &best)) {
             g_last_error.clear();
             continue;
         }
-        enqueue_matvec_batched(op, d_V, d_U, nrhs, ld, 0, st, f32, c.first, c.second);  // a second warm-up
-        cudaEventRecord(e0, st);
-        for (int r = 0; r < 3; r++) enqueue_matvec_batched(op, d_V, d_U, nrhs, ld, 0, st, f32, c.first, c.second);
-        cudaEventRecord(e1, st);
-        cudaEventSynchronize(e1);
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best) {
-            best = ms;
+        if (best < before) {
             btr = c.first;
             bng = c.second;
         }
     }
+    if (patch) {
+        const float tile = best;
+        if (time(kPatchTile, 0, &best)) return AFM_ERR_CUDA;
+        patch = best < tile;
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (best >= 1e30f) return fail(AFM_ERR_CUDA, "no batched kernel configuration runs");
-    op->batch_tune.push_back({key, btr, bng, best / 3.0f});
-    *tr = btr;
+    op->batch_tune.push_back({key, btr, bng, best, patch});
+    *tr = patch ? kPatchTile : btr;
     *ng = bng;
     return AFM_SUCCESS;
 }
@@ -1362,7 +1499,9 @@ int run_bcg(afm_operator* op, const BVectors<T>& V, uint32_t R, double maxit, in
         AFM_CUDA(cudaStreamSynchronize(st));
         AFM_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         int s = AFM_SUCCESS;
+        op->own_capture = true;
         for (int i = 0; i < batch && s == AFM_SUCCESS; i++) s = step();
+        op->own_capture = false;
         if (s == AFM_SUCCESS && cudaMemcpyAsync(op->h_bremain, remaining, sizeof(unsigned int),
                                                 cudaMemcpyDeviceToHost, st) != cudaSuccess)
             s = fail(AFM_ERR_CUDA, "capture: counter copy");
@@ -1906,7 +2045,7 @@ int afm_create(afm_operator** out, int bc_method, int device) {
     if (configure_kernels_fp64() != cudaSuccess || configure_kernels_split() != cudaSuccess ||
         configure_kernels_fp32() != cudaSuccess || configure_kernels_f32sym() != cudaSuccess ||
         configure_kernels_f32symx() != cudaSuccess || configure_kernels_splitsymx() != cudaSuccess ||
-        configure_kernels_f32symc() != cudaSuccess)
+        configure_kernels_f32symc() != cudaSuccess || configure_bpatch() != cudaSuccess)
         return fail(AFM_ERR_CUDA, "kernel configuration failed on device %d", device);
     auto* op = new afm_operator();
     op->device = device;
@@ -2894,6 +3033,7 @@ int afm_set_batch_tuning(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, 
         if (t.key == key) {
             t.tr = cols_per_thread;
             t.ng = groups_per_cta;
+            t.patch = false;
             return ok();
         }
     op->batch_tune.push_back({key, cols_per_thread, groups_per_cta, 0.0f});

@@ -407,10 +407,10 @@ struct afm_operator {
     // one launch for every element (plans of one element size): the element products go to d_ve and a gather
     // pass sums each DoF's entries in arena (colour) order
     uint32_t gather_b = 0;          // DoFs per list of the gather pass (0: the plan has none)
-    uint32_t* d_gather_off = nullptr;
+    double* d_ve = nullptr;            // owns the lists too
     uint32_t* d_gather_idx = nullptr;
-    double* d_ve = nullptr;
-    cudaStream_t ve_stream = nullptr;  // stream of the last product that used d_ve
+    uint32_t* d_gather_off = nullptr;
+    cudaStream_t ve_stream = nullptr;  // stream of the last product that used d_ve or d_bp_pv
     cudaEvent_t ve_event = nullptr;    // its end, where that stream is not the operator's own
     bool own_capture = false;          // the operator's solver is capturing its iterations on `stream`
 
@@ -423,8 +423,18 @@ struct afm_operator {
     unsigned int* h_bremain = nullptr;
     struct BatchTune {
         uint64_t key;
-        int tr, ng;  // lane tile: columns, rows
+        int tr, ng;  // lane tile of the launches per colour: columns, rows
         float ms;
+        bool patch = false;  // the patch plan beats every tile (ms is its time then)
     };
+    // patch plan of the batched product (afm_batched_patch.hpp), built by the first batched call that can use it
+    int bp_state = 0;               // 0 not looked at, 1 built, -1 none
+    uint32_t bp_n = 0, bp_patches = 0, bp_max_rows = 0, bp_pv_rows = 0, bp_shared = 0;
+    unsigned char* d_bp_hdr = nullptr;
+    uint32_t* d_bp_dof = nullptr;
+    uint32_t* d_bp_off = nullptr;
+    uint32_t* d_bp_idx = nullptr;
+    unsigned char* d_bp_pv = nullptr;  // combine buffer
+    size_t bp_pv_bytes = 0;
     std::vector<BatchTune> batch_tune;  // autotuner choices
 };

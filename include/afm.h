@@ -348,11 +348,14 @@ int afm_matmult_bc_device_f32(afm_operator* op, float* d_v, const float* d_u, vo
  * are contiguous), 16-byte aligned; nrhs is a multiple of 4, at most 256, ld
  * >= nrhs a multiple of 4; every element must have more than 16 DoFs. Each
  * element matrix is streamed once per call and applied to all columns (for
- * example hex8 elasticity with 64 right-hand sides): a warp per element, a
+ * example hex8 elasticity with 64 right-hand sides): over patches of elements
+ * of one size (24, 30 or 60 DoFs; not in AFM_PREC_FP64), whose rows of V a
+ * warp sums in shared memory, or in a launch per colour, a warp per element, a
  * register tile of V_e per lane. The first call for a given (nrhs, ld,
- * arithmetic) runs the autotuner, which times the lane tile shapes on the
- * caller's data and keeps the fastest for the operator. No counterpart in
- * the reference, whose matvec takes one vector. */
+ * arithmetic) runs the autotuner, which times the patches and the lane tile
+ * shapes on the caller's data and keeps the fastest for the operator (inside a
+ * caller's stream capture always a launch per colour). No counterpart in the
+ * reference, whose matvec takes one vector. */
 int afm_matvec_batched_device(afm_operator* op, double* d_V, const double* d_U, uint32_t nrhs, uint32_t ld,
                               void* stream);
 int afm_matvec_batched_device_f32(afm_operator* op, float* d_V, const float* d_U, uint32_t nrhs, uint32_t ld,
@@ -363,7 +366,8 @@ int afm_matmult_bc_batched_device(afm_operator* op, double* d_V, const double* d
 int afm_matmult_bc_batched_device_f32(afm_operator* op, float* d_V, const float* d_U, uint32_t nrhs, uint32_t ld,
                                       void* stream);
 /* The autotuner's choice for (nrhs, ld, f32): columns and rows of the lane
- * tile, and the time of one product in ms. f32 = 0: FP64 (or split) products;
+ * tile (the best of the launches per colour, also where the patches are
+ * faster than all of them), and the time of one product in ms. f32 = 0: FP64 (or split) products;
  * 1: FP32 products; 2: the FP32 products of the batched mixed solve. */
 int afm_get_batch_tuning(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, int* cols_per_thread,
                          int* rows_per_thread, float* ms);
