@@ -76,6 +76,10 @@ cudaError_t launch_segment_f32symc(const Segment& s, const SegArgs& a, int sm_co
 cudaError_t launch_patches_f32symc(const PatchPlanGeom& pg, const PatchArgs& a, int sm_count, bool pdl,
                                    cudaStream_t st);
 cudaError_t configure_kernels_f32symc();
+cudaError_t launch_patches_splitsym(const PatchPlanGeom& pg, const PatchArgs& a, int sm_count, bool pdl,
+                                    cudaStream_t st);
+cudaError_t configure_kernels_splitsym();
+size_t patch_smem_splitsym(const PatchPlanGeom& pg, uint32_t copy_bytes);
 size_t patch_smem_f32symc(const PatchPlanGeom& pg, uint32_t copy_bytes);
 size_t segment_smem_f32symc(const Segment& s);
 size_t patch_smem_splitsymx(const PatchPlanGeom& pg, uint32_t copy_bytes);
@@ -103,6 +107,7 @@ cudaError_t launch_patches(int prec, const PatchPlanGeom& pg, const PatchArgs& a
         case kPrecF32SymX: return launch_patches_f32symx(pg, a, sm_count, pdl, stream);
         case kPrecSplitSymX: return launch_patches_splitsymx(pg, a, sm_count, pdl, stream);
         case kPrecF32SymC: return launch_patches_f32symc(pg, a, sm_count, pdl, stream);
+        case kPrecSplitSym: return launch_patches_splitsym(pg, a, sm_count, pdl, stream);
         default: return launch_patches_fp32(pg, a, sm_count, pdl, stream);
     }
 }
@@ -115,6 +120,7 @@ size_t patch_smem_bytes(int prec, const PatchPlanGeom& pg, uint32_t copy_bytes) 
         case kPrecF32SymX: return patch_smem_f32symx(pg, copy_bytes);
         case kPrecSplitSymX: return patch_smem_splitsymx(pg, copy_bytes);
         case kPrecF32SymC: return patch_smem_f32symc(pg, copy_bytes);
+        case kPrecSplitSym: return patch_smem_splitsym(pg, copy_bytes);
         default: return patch_smem_fp32(pg, copy_bytes);
     }
 }
@@ -269,6 +275,7 @@ void free_device(afm_operator* op) {
     dfree(op, op->d_shared_idx);
     dfree(op, op->d_shared_pos);
     dfree(op, op->d_sym);
+    dfree(op, op->d_packed);
     dfree(op, op->d_vx);
     dfree(op, op->d_csr_rp);
     dfree(op, op->d_csr_cols);
@@ -766,10 +773,11 @@ int buffer_done(afm_operator* op, cudaStream_t st) {
 }
 
 // True when every element matrix is symmetric to within 1e-6 of its largest
-// diagonal entry (exactly, for an element whose diagonal is zero).
-bool ke_is_symmetric(const afm_operator* op) {
-    int sym = 1;
-#pragma omp parallel for schedule(static) reduction(&& : sym)
+// diagonal entry (exactly, for an element whose diagonal is zero). *exact:
+// every one equal to its transpose.
+bool ke_is_symmetric(const afm_operator* op, bool* exact) {
+    int sym = 1, same = 1;
+#pragma omp parallel for schedule(static) reduction(&& : sym, same)
     for (int64_t e = 0; e < (int64_t)op->n_elem; e++) {
         if (!sym) continue;
         const uint32_t n = op->offsets[e + 1] - op->offsets[e];
@@ -778,12 +786,17 @@ bool ke_is_symmetric(const afm_operator* op) {
         for (uint32_t r = 0; r < n; r++) dmax = std::max(dmax, std::fabs(k[(size_t)r * n + r]));
         const double tol = 1e-6 * dmax;
         for (uint32_t r = 0; r < n && sym; r++)
-            for (uint32_t c = r + 1; c < n; c++)
-                if (!(std::fabs(k[(size_t)r * n + c] - k[(size_t)c * n + r]) <= tol)) {
+            for (uint32_t c = r + 1; c < n; c++) {
+                const double x = k[(size_t)r * n + c], y = k[(size_t)c * n + r];
+                if (x == y) continue;
+                same = 0;
+                if (!(std::fabs(x - y) <= tol)) {
                     sym = 0;
                     break;
                 }
+            }
     }
+    *exact = sym && same;
     return sym != 0;
 }
 
@@ -1092,11 +1105,18 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
             a.copy_bytes = (uint32_t)a.unit_bytes;
             a.plane = sym ? s.sym_plane : s.plane;
             if (f32 && !sym && op->precision == AFM_PREC_FP64_SPLIT) a.copy_bytes = s.plane * 4;
+            const bool packed = kprec == AFM_PREC_FP64_SPLIT && op->d_packed;
+            if (packed) {
+                a.ke = op->d_packed;
+                a.plane = s.n * (s.n + 1) / 2 * kTpeWidth;
+                a.unit_bytes = 8ull * a.plane;
+                a.copy_bytes = (uint32_t)a.unit_bytes;
+            }
             a.bc_mode = bc_mode;
             a.err = op->d_err;
             a.wait_ns = op->wait_ns;
             a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
-            AFM_CUDA(launch_patches(kprec, op->patch_geom, a, op->sm_count, !first || a.u_dep, st));
+            AFM_CUDA(launch_patches(packed ? kPrecSplitSym : kprec, op->patch_geom, a, op->sm_count, !first || a.u_dep, st));
             first = false;
         }
         const int vo_bytes = (f32 || kprec == AFM_PREC_FP32) && !symx ? 4 : 8;
@@ -2045,7 +2065,8 @@ int afm_create(afm_operator** out, int bc_method, int device) {
     if (configure_kernels_fp64() != cudaSuccess || configure_kernels_split() != cudaSuccess ||
         configure_kernels_fp32() != cudaSuccess || configure_kernels_f32sym() != cudaSuccess ||
         configure_kernels_f32symx() != cudaSuccess || configure_kernels_splitsymx() != cudaSuccess ||
-        configure_kernels_f32symc() != cudaSuccess || configure_bpatch() != cudaSuccess)
+        configure_kernels_f32symc() != cudaSuccess || configure_kernels_splitsym() != cudaSuccess ||
+        configure_bpatch() != cudaSuccess)
         return fail(AFM_ERR_CUDA, "kernel configuration failed on device %d", device);
     auto* op = new afm_operator();
     op->device = device;
@@ -2647,16 +2668,27 @@ int afm_finalize(afm_operator* op) {
     // symmetric inner arena (built on the first FP32 product): split arena,
     // symmetric Ke, and elements that run as patches or on the warp-group kernel
     op->ke_symmetric = false;
+    op->ke_sym_exact = false;
     op->sym_ok = false;
     op->sym_bytes = 0;
     op->sym_built = 0;
     if (prec == AFM_PREC_FP64_SPLIT && !op->dup_in_element && op->n_elem > 0) {
-        op->ke_symmetric = ke_is_symmetric(op);
+        op->ke_symmetric = ke_is_symmetric(op, &op->ke_sym_exact);
         bool covered = true;
         if (!op->use_patches)
             for (const Segment& s : op->segs)
                 if (s.units && s.regime != REG_WPE) covered = false;
         op->sym_ok = op->ke_symmetric && covered;
+        if (op->use_patches && op->ke_sym_exact) {
+            const Segment& s = op->segs[0];
+            const size_t bytes = (size_t)s.units * s.n * (s.n + 1) * kTpeWidth * 4;
+            if (dalloc(op, &op->d_packed, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+                cudaGetLastError();  // no room: FP64 products read the whole matrices
+                op->d_packed = nullptr;
+            } else {
+                AFM_CUDA(pack_split_units(op->d_ke, s.n, s.units, op->d_packed, op->sm_count, op->stream));
+            }
+        }
     }
     op->ke_dirty = false;
     op->finalized = true;

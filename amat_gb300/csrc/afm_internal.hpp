@@ -214,6 +214,13 @@ constexpr int kPrecSplitSymX = 18;
 // The corrected arena on FP32 u with FP32 row sums and FP64 v (ArithF32SymC).
 constexpr int kPrecF32SymC = 19;
 
+// FP64 vectors, the split arithmetic on packed symmetric patch units (ArithSplitSym).
+constexpr int kPrecSplitSym = 20;
+
+// Packs a patch plan's split units (afm_mv_splitsym.cu).
+cudaError_t pack_split_units(const unsigned char* ke, uint32_t n, uint32_t units, unsigned char* packed, int sm_count,
+                             cudaStream_t st);
+
 // Fills segment s's part of the symmetric inner arena from its split-arena
 // units (afm_mv_f32sym.cu).
 cudaError_t build_sym_segment(const Segment& s, const unsigned char* ke, unsigned char* sym, int sm_count,
@@ -358,6 +365,9 @@ struct afm_operator {
     // symmetric inner arena: FP32 element matrices with each symmetric pair of
     // entries stored once, built from the split arena on the first FP32 product
     bool ke_symmetric = false;      // every Ke symmetric to 1e-6 of its largest diagonal entry
+    bool ke_sym_exact = false;      // every Ke equal to its transpose bit for bit
+    // the split units of a patch plan with such Ke, packed (FP64 products read them; null: they read d_ke)
+    unsigned char* d_packed = nullptr;
     bool sym_ok = false;            // symmetric, split arena, and a layout the symmetric kernels cover
     int sym_mode = 1;               // afm_set_symmetric_inner: 0 off, 1 FP32, 2 FP32 + BF16 correction
     int sym_built = 0;              // format of d_sym (1 or 2; 0: not built)

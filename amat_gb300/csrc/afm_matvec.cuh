@@ -354,6 +354,13 @@ struct ArithF32SymC {
     static __device__ __forceinline__ void combine(Acc& a, const Acc& b) { a.s += b.s; }
 };
 
+// The split arithmetic on patch units that hold the packed upper triangle in
+// both planes (every Ke equal to its transpose bit for bit, so nothing is
+// rounded): 55% of the bytes for n = 10, the same products and sums.
+struct ArithSplitSym : ArithSplit {
+    static constexpr bool kSym = true;
+};
+
 // FP64 products from the corrected symmetric arena (the arena of ArithF32SymX:
 // K to about 2^-32, each pair of entries once): u and v are FP64 vectors, u is
 // staged as a scaled float pair like the split arithmetic, and each product

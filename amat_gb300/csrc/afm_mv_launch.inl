@@ -1,7 +1,7 @@
 // Instantiation and dispatch of the matvec kernels for one arithmetic policy
-// (included by afm_mv_fp64.cu, afm_mv_split.cu, afm_mv_fp32.cu and
-// afm_mv_f32sym.cu, which define ARITH and LAUNCH_FN so that they compile in
-// parallel; BATCH_FN is left undefined where there is no batched product).
+// (included by the afm_mv_*.cu files, which define ARITH and LAUNCH_FN so that
+// they compile in parallel; BATCH_FN is left undefined where there is no
+// batched product, LAUNCH_FN where the arithmetic runs on patches only).
 #include <algorithm>
 
 #include "afm_batched.cuh"
@@ -9,6 +9,7 @@
 
 namespace afm {
 
+#ifdef LAUNCH_FN
 namespace {
 
 // Element sizes with a compile-time specialisation; any other n <= 16 (TPE)
@@ -64,6 +65,7 @@ void* pick_kernel(int regime, uint32_t n, bool dup, bool chunked = false, bool v
 }
 
 }  // namespace
+#endif  // LAUNCH_FN
 
 // Ring stages that fit beside `extra` bytes: per stage the slot, two
 // mbarriers and a tag; 32 bytes for the flag word and the tags' padding. Up to
@@ -71,6 +73,7 @@ void* pick_kernel(int regime, uint32_t n, bool dup, bool chunked = false, bool v
 // land, and each SM needs ~200 KB of copies in flight to keep HBM busy, which
 // small slots reach only with many stages.
 constexpr uint32_t kMaxStages = 32;
+#ifdef LAUNCH_FN
 static uint32_t stages_for(uint32_t slot_bytes, uint32_t extra) {
     if (extra + 32 >= kSmemBudget) return 0;
     uint32_t st = (kSmemBudget - extra - 32) / (slot_bytes + 20);
@@ -239,17 +242,21 @@ cudaError_t BATCH_FN(const Segment& s, const BatchArgs& a, int sm_count, int ct,
 
 #endif  // BATCH_FN
 
+#endif  // LAUNCH_FN
+
 // ---- patch path (small elements) -----------------------------------------
 
 namespace {
 // consumer groups (G) of GW warps of the patch kernel for this arithmetic
-// (see afm_patch.cuh): FP32 tries 8 groups of 2 warps, then 4; 8-byte entries
-// 4 groups of 2 warps, then 2 of 4 (their 25.6 KB units leave few ring slots).
+// (measured at kPatchMaxGroups in afm_patch.cuh): FP32 tries 8 groups of 2
+// warps, then 4; 8-byte entries 8 groups of 2 warps where a patch has at most 64
+// slots (small meshes), else 4 groups of 4, then 2 of 4 (their units leave few
+// ring slots).
 constexpr bool kF32Patch = sizeof(typename ARITH::VT) == 4;
 constexpr uint32_t kMinPatchStages = kF32Patch ? 6 : 5;  // ring slots below which fewer groups are used
 
 // warps per group for G groups
-constexpr int patch_gw(int G) { return kF32Patch ? 2 : (G == 4 ? 2 : 4); }
+constexpr int patch_gw(int G) { return kF32Patch || G == 8 ? 2 : 4; }
 
 template <int G>
 void* patch_kernel_g(uint32_t n) {
@@ -263,8 +270,10 @@ void* patch_kernel_g(uint32_t n) {
 }
 
 void* pick_patch_kernel(uint32_t n, uint32_t groups) {
-    if constexpr (kF32Patch) return groups == 8 ? patch_kernel_g<8>(n) : patch_kernel_g<4>(n);
-    else return groups == 4 ? patch_kernel_g<4>(n) : patch_kernel_g<2>(n);
+    if (groups == 8) return patch_kernel_g<8>(n);
+    if constexpr (!kF32Patch)
+        if (groups == 2) return patch_kernel_g<2>(n);
+    return patch_kernel_g<4>(n);
 }
 
 PatchLayout patch_layout_g(const PatchPlanGeom& pg, uint32_t copy_bytes, uint32_t groups) {
@@ -284,10 +293,12 @@ PatchLayout patch_layout_g(const PatchPlanGeom& pg, uint32_t copy_bytes, uint32_
 }
 
 PatchLayout patch_layout(const PatchPlanGeom& pg, uint32_t copy_bytes) {
-    const uint32_t more = kF32Patch ? 8 : 4, fewer = kF32Patch ? 4 : 2;
-    const PatchLayout L = patch_layout_g(pg, copy_bytes, more);
-    if (L.stages >= kMinPatchStages) return L;
-    return patch_layout_g(pg, copy_bytes, fewer);
+    for (uint32_t groups : {8u, 4u}) {
+        if (!kF32Patch && groups == 8 && pg.max_slots > 64) continue;
+        const PatchLayout L = patch_layout_g(pg, copy_bytes, groups);
+        if (L.stages >= kMinPatchStages) return L;
+    }
+    return patch_layout_g(pg, copy_bytes, kF32Patch ? 4 : 2);
 }
 }  // namespace
 
@@ -316,6 +327,7 @@ size_t PATCH_SMEM_FN(const PatchPlanGeom& pg, uint32_t copy_bytes) {
     return L.stages >= 2 ? L.total() : 0;
 }
 
+#ifdef LAUNCH_FN
 size_t SMEM_FN(const Segment& s) { return ring_layout(s, s.unit_bytes, s.unit_bytes, false, nullptr).total(); }
 
 #ifdef FUSED_FN
@@ -395,10 +407,12 @@ void AFM_CAT(SMEM_FN, _geom)(const Segment& s, uint64_t copy_bytes, uint64_t uni
     out[4] = G.gc;
     out[5] = L.total();
 }
+#endif  // LAUNCH_FN
 
 // Raises the dynamic shared-memory limit of every kernel instance on the
 // current device; called once per device before any launch or capture.
 cudaError_t CONFIG_FN() {
+#ifdef LAUNCH_FN
     for (int reg = 0; reg < 2; reg++)
         for (uint32_t nn : {4u, 8u, 10u, 20u, 24u, 30u, 60u, 0u})
             for (int d = 0; d < 2; d++)
@@ -409,6 +423,7 @@ cudaError_t CONFIG_FN() {
                                                          (int)(kSmemBudget + 1024));
                     if (e != cudaSuccess) return e;
                 }
+#endif
     for (uint32_t nn : {4u, 8u, 10u, 0u})
         for (uint32_t gg : {2u, 4u, 8u}) {
             cudaError_t e = cudaFuncSetAttribute(pick_patch_kernel(nn, gg),

@@ -38,11 +38,15 @@
 namespace afm {
 
 // G consumer groups of GW warps: 8 groups of 2 warps for FP32 (or 4 when the
-// shared memory of 8 would leave the ring too few slots), 4 groups of 2 warps
-// for 8-byte entries (or 2 groups of 4 when their 25.6 KB units would leave
-// the ring too few slots). A group's patch passes through phases bound by
-// memory latency (the index block, the gather of u), so the patches in flight
-// per SM, not the multiply, set the kernel's pace.
+// shared memory of 8 would leave the ring too few slots), for 8-byte entries 8
+// of 2 where a patch has one or two units, else 4 of 4 (or 2 of 4 when their
+// units would leave the ring too few slots). A group's patch passes through
+// phases bound by memory latency (the index block, the gather of u), so the
+// patches in flight per SM set the pace of the FP32 kernels; the double-float
+// products of a unit take long enough that a warp per unit pays (4 groups, 2 ->
+// 4 warps each: tet10 Poisson 52^3 x 6 124 -> 110 us, hex8 Poisson 80^3 58 ->
+// 50), but only where a patch has that many units (hex8 Poisson 32^3, one unit:
+// 10.7 -> 11.7; 8 groups of 2: 10.6). FP32: 3 warps 47 -> 51 us, 12 groups 56.
 constexpr uint32_t kPatchMaxGroups = 8;
 constexpr int kBatch = 8;  // global loads a thread keeps in flight in the gather
 
@@ -114,36 +118,43 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
     if (warp == kPatchGroups * kPatchGroupWarps) {  // producer
         if (lane == 0) {
             const uint64_t pol = l2_evict_first_policy();
-            uint32_t issued = 0;  // Ke units
+            // One thread issues every copy of the CTA, so its path per copy is short: the next descriptor is
+            // loaded a patch ahead, slot and round advance by increments (with a load and two divisions per copy
+            // the FP32 product of tet10 Poisson 50^3 x 6 was bound by it, 0.64 G copies/s: 47.2 -> 43.4 us;
+            // hex8 Poisson 80^3 34.7 -> 28.6).
+            uint32_t issued = 0, slot = 0, round = 0;  // Ke units; the next unit's ring slot and round
             uint32_t idx_issued[kPatchGroups] = {};
             bool stop = false;
+            uint32_t g = 0, j = 0;  // the patch's group and its place among the group's patches
+            // 8-byte entries: the group's next index block into L2 while its patch runs, so that its copy (issued
+            // once the patch is done) does not wait on HBM (measured: split tet10 product 1.115 -> 1.065 ms; the
+            // FP32 kernels, with twice the groups, ran slower with it)
+            constexpr bool kAhead = sizeof(VT) == 8;
+            auto at = [&](uint32_t k) { return k < cnt ? desc[k] : PatchDesc{}; };
+            PatchDesc d = at(0), d2 = kAhead ? at(kPatchGroups) : PatchDesc{};
             for (uint32_t k = 0; k < cnt && !stop; k++) {
-                const uint32_t g = k % kPatchGroups, j = k / kPatchGroups;
-                const PatchDesc d = desc[k];
+                const PatchDesc dn = at(k + 1), d2n = kAhead ? at(k + 1 + kPatchGroups) : PatchDesc{};
                 if (j >= 1 && !mbar_wait_abortable(&idx_empty[g], (j - 1) & 1, abort, a.wait_ns)) break;
                 mbar_arrive_expect_tx(&idx_full[g], d.idx_bytes);
                 bulk_load(smem + L.group_offset() + g * L.group_bytes(), a.idx + d.idx_off, d.idx_bytes,
                           &idx_full[g], pol);
                 idx_issued[g] = j + 1;
-                // 8-byte entries: the group's next index block into L2 now, so that its copy (issued once
-                // this patch is done) does not wait on HBM (measured: split tet10 product 1.115 -> 1.065 ms;
-                // the FP32 kernels, with twice the groups, ran slower with it)
-                if (sizeof(VT) == 8 && k + kPatchGroups < cnt) {
-                    const PatchDesc d2 = desc[k + kPatchGroups];
-                    bulk_prefetch_l2(a.idx + d2.idx_off, d2.idx_bytes);
-                }
-                for (uint32_t u = 0; u < d.units; u++) {
-                    const uint32_t s = issued % S;
-                    if (issued >= S && !mbar_wait_abortable(&empty[s], ((issued / S) - 1) & 1, abort, a.wait_ns)) {
+                if (kAhead && d2.idx_bytes) bulk_prefetch_l2(a.idx + d2.idx_off, d2.idx_bytes);
+                const unsigned char* src = a.ke + (uint64_t)d.unit0 * a.unit_bytes;
+                for (uint32_t u = 0; u < d.units; u++, src += a.unit_bytes) {
+                    if (round && !mbar_wait_abortable(&empty[slot], (round - 1) & 1, abort, a.wait_ns)) {
                         stop = true;
                         break;
                     }
-                    tag[s] = issued;
-                    mbar_arrive_expect_tx(&full[s], a.copy_bytes);
-                    bulk_load(smem + (size_t)s * L.slot_bytes, a.ke + (uint64_t)(d.unit0 + u) * a.unit_bytes,
-                              a.copy_bytes, &full[s], pol);
+                    tag[slot] = issued;
+                    mbar_arrive_expect_tx(&full[slot], a.copy_bytes);
+                    bulk_load(smem + (size_t)slot * L.slot_bytes, src, a.copy_bytes, &full[slot], pol);
                     issued++;
+                    if (++slot == S) slot = 0, round++;
                 }
+                d = dn;
+                d2 = d2n;
+                if (++g == kPatchGroups) g = 0, j++;
             }
             allow_dependent_launch();
             if (*abort) atomicOr(a.err, kErrTimeout);
@@ -244,15 +255,37 @@ __global__ void __launch_bounds__((G * GW + 1) * 32, 1) afm_patch_kernel(PatchAr
                 for (int c = 0; c < NM; c++)
                     if (c < (int)n) ul[c] = us[lmap[(un * n + c) * 32u + lane]];
                 const uint32_t e = un * 32u + lane;
+                if constexpr (A::kSym) {
+                    // each stored entry once: row i takes u_j and row j takes u_i, so that every row still sums its
+                    // columns in ascending order
+                    Acc acc[NM];
 #pragma unroll
-                for (int r = 0; r < NM; r++) {
-                    if (r < (int)n) {
-                        typename A::Acc acc = A::zero();
+                    for (int r = 0; r < NM; r++) acc[r] = A::zero();
 #pragma unroll
-                        for (int c = 0; c < NM; c++)
-                            if (c < (int)n) A::fma(acc, A::kload(ks, (size_t)tpe_entry<A>(r, c, n) * 32u + lane, a.plane),
-                                              ul[c]);
-                        ve[r * cap + e] = acc;
+                    for (int j = 0; j < NM; j++) {
+                        if (j < (int)n) {
+#pragma unroll
+                            for (int i = 0; i <= j; i++) {
+                                const KT k = A::kload(ks, (size_t)(j * (j + 1) / 2 + i) * 32u + lane, a.plane);
+                                A::fma(acc[j], k, ul[i]);
+                                if (i < j) A::fma(acc[i], k, ul[j]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < NM; r++)
+                        if (r < (int)n) ve[r * cap + e] = acc[r];
+                } else {
+#pragma unroll
+                    for (int r = 0; r < NM; r++) {
+                        if (r < (int)n) {
+                            Acc acc = A::zero();
+#pragma unroll
+                            for (int c = 0; c < NM; c++)
+                                if (c < (int)n)
+                                    A::fma(acc, A::kload(ks, (size_t)tpe_entry<A>(r, c, n) * 32u + lane, a.plane), ul[c]);
+                            ve[r * cap + e] = acc;
+                        }
                     }
                 }
             }
