@@ -666,21 +666,22 @@ void build_segments(afm_operator* op, int prec) {
 // Whether one launch for every element plus the gather pass beats a launch
 // per colour. The gather pass costs its traffic (element products written and
 // read, lists read), a colour launch its ramp and tail, so the line is a
-// number of entries (elements x DoFs) per colour; and the products
-// (ve_bytes each) must stay in the 126 MB L2. Measured, colours -> gather:
-// 8-byte staged u (FP64, split): hex20 elasticity 12^3 27 -> 20 us, 32^3 188 ->
-// 172 (0.25 M entries per colour), 42^3 389 -> 377 (0.56 M), 48^3 556 -> 561
-// (0.83 M), 56^3 885 -> 897 (1.3 M); hex8 elasticity 16^3 45 -> 14 us, 48^3
-// 146 -> 123 (0.33 M), 56^3 211 -> 192 (0.53 M); tet10 elasticity 16^3 x 6 136
-// -> 49 us, 32^3 x 6 392 -> 320. FP32 products and inner formats, whose
-// element launches are shorter: hex8 elasticity 72^3 164 -> 142 us (1.1 M),
-// hex20 42^3 (format 4) 231 -> 204 (0.56 M), 56^3 (FP32) 305 -> 309 (1.3 M);
-// tet10 elasticity 44^3 x 6: FP32 349 -> 287 (61 MB of products), format 4
-// 618 -> 635 (123 MB).
+// number of entries (elements x DoFs) per colour; elements of two row groups
+// and more (n > 32) stream more of Ke per entry and have few element groups per
+// SM, so their colour launches ramp faster. And the products (ve_bytes each)
+// must stay in the 126 MB L2. Measured, colours -> gather: 8-byte staged u
+// (FP64, split): hex20 elasticity 12^3 27 -> 16 us, 26^3 91 -> 82 (0.13 M entries
+// per colour), 32^3 146 -> 149 (0.25 M), 42^3 306 -> 329 (0.56 M); hex8
+// elasticity 16^3 45 -> 12 us, 48^3 116 -> 92 (0.33 M), 56^3 159 -> 144 (0.53 M),
+// 72^3 294 -> 302 (1.1 M); tet10 elasticity 16^3 x 6 102 -> 40 us, 32^3 x 6 336 ->
+// 248. FP32 products and inner formats, whose element launches are shorter:
+// hex20 42^3 FP32 122 -> 98 us, format 4 225 -> 195 (0.56 M), 56^3 232 -> 236 and
+// 462 -> 458 (1.3 M); hex8 elasticity 72^3 159 -> 126 us (1.1 M), 90^3 258 -> 242
+// (2.2 M); tet10 elasticity 44^3 x 6 FP32 339 -> 242.
 bool gather_pays(const afm_operator* op, bool wide, uint32_t ve_bytes) {
     const uint64_t entries = (uint64_t)op->n_elem * op->nmax;
-    return entries / std::max<uint32_t>(op->n_colors, 1) <= (wide ? 700000u : 1200000u) &&
-           entries * ve_bytes <= 100000000u;
+    const uint64_t most = op->nmax > 32 ? (wide ? 200000u : 1200000u) : (wide ? 900000u : 2200000u);
+    return entries / std::max<uint32_t>(op->n_colors, 1) <= most && entries * ve_bytes <= 100000000u;
 }
 
 // Lists of the gather pass (launch_gather_sum) for a plan whose elements all

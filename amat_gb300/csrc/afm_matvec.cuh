@@ -31,7 +31,7 @@ namespace afm {
 
 constexpr unsigned long long kDefaultWaitNs = 4000000000ull;  // 4 s per wait unless the operator sets another
 constexpr unsigned long long kDrainLimitNs = 4000000000ull;   // copies in flight at exit: always 4 s
-constexpr uint32_t kSmemBudget = 220 * 1024;
+constexpr uint32_t kSmemBudget = 226 * 1024;
 constexpr uint32_t kSlotAlign = 128;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -183,11 +183,40 @@ __device__ __forceinline__ void report_bad(int* err, int kind, uint32_t a0, uint
     atomicOr(err, kErrBounds);
 }
 
+// ---- packed pairs of floats (two IEEE FP32 operations per instruction) --------
+using f2 = unsigned long long;  // two packed floats
+__device__ __forceinline__ f2 pack2(float x, float y) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // ---- arithmetic policies ----------------------------------------------------
 // KT: stored Ke entry, UT: staged u entry, VT: vector entry, Acc: accumulator.
 
 struct ArithF64 {
     static constexpr bool kSym = false;
+    static constexpr bool kPair = false;  // rows in pairs in the warp-group kernel (wpg_pair_groups)
     static constexpr bool kScaled = false;  // u scaled by a power of two per launch (stage_s, finish_s)
     static constexpr uint32_t kWpgWarps = 16;  // consumer warps of the warp-group kernel
     using KT = double;
@@ -213,6 +242,7 @@ struct ArithF64 {
 // The _rn intrinsics keep the compiler from fusing the steps.
 struct ArithSplit {
     static constexpr bool kSym = false;
+    static constexpr bool kPair = true;
     static constexpr bool kScaled = true;
     static constexpr uint32_t kWpgWarps = 16;
     using KT = float2;
@@ -254,6 +284,7 @@ struct ArithSplit {
 
 struct ArithF32 {
     static constexpr bool kSym = false;
+    static constexpr bool kPair = false;
     static constexpr bool kScaled = false;
     static constexpr uint32_t kWpgWarps = 24;  // more elements in flight: see wpg_gc
     using KT = float;
@@ -295,6 +326,7 @@ struct ArithF32Sym : ArithF32 {
 // markedly; this arithmetic removes both.
 struct ArithF32SymX {
     static constexpr bool kSym = true;
+    static constexpr bool kPair = false;
     static constexpr bool kScaled = false;
     static constexpr uint32_t kWpgWarps = 24;
     using KT = float2;  // (hi, lo)
@@ -337,6 +369,7 @@ struct ArithF32SymX {
 // FP32 Ke alone +50% CG iterations, FP32 sums on top of it +10%).
 struct ArithF32SymC {
     static constexpr bool kSym = true;
+    static constexpr bool kPair = false;
     static constexpr bool kScaled = false;
     static constexpr uint32_t kWpgWarps = 24;
     using KT = float2;  // (hi, lo)
@@ -371,6 +404,7 @@ struct ArithSplitSym : ArithSplit {
 // large ill-conditioned systems.
 struct ArithSplitSymX {
     static constexpr bool kSym = true;
+    static constexpr bool kPair = false;
     static constexpr bool kScaled = true;
     static constexpr uint32_t kWpgWarps = 16;
     using KT = float2;  // (hi, lo)
@@ -820,6 +854,42 @@ __device__ __forceinline__ void sym_terms(typename A::Acc& acc, const unsigned c
     }
 }
 
+// Rows in pairs (split arithmetic, elements of 24, 30 and 60 DoFs): a lane owns
+// rows 2 l and 2 l + 1 and runs both on packed instructions, so a warp covers
+// every row of an element and its g warps (times wpg_pair_groups column groups
+// in each, where two rows per lane leave lanes over) split the columns. Half
+// the instructions per entry, and shorter columns than with a row per lane (15
+// instead of 30 for hex20): an element holds its ring slot for less time, which
+// leaves more copies in flight, and that was the bound (5.4 TB/s with 7 slots of
+// 28.8 KB, 4 of them held). hex20 elasticity 42^3 389 -> 302 us (7.1 TB/s), 56^3 885
+// -> 714; hex8 elasticity 72^3 405 -> 348. 0: a row per lane.
+__host__ __device__ constexpr uint32_t wpg_pair_groups(uint32_t n) {
+    return n == 60 ? 1u : n == 24 || n == 30 ? 2u : 0u;
+}
+
+// Columns [0, NC) of two rows of an element (kh, kl: the pair's entries of the
+// first column in the hi and lo planes, u: the staged pairs of the columns):
+// the products of ArithSplit::fma, each difference written as a multiply-add by
+// -1 (exact products: the same roundings).
+template <int NT, int NC>
+__device__ __forceinline__ void split_pair_terms(f2& hi, f2& lo, const float* kh, const float* kl, const float2* u) {
+    const f2 m1 = pack2(-1.0f, -1.0f);
+    hi = lo = 0ull;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+        const f2 kx = *reinterpret_cast<const f2*>(kh + c * NT), ky = *reinterpret_cast<const f2*>(kl + c * NT);
+        const float2 x = u[c];
+        const f2 uh = pack2(x.x, x.x), nh = pack2(-x.x, -x.x), nl = pack2(-x.y, -x.y);
+        const f2 p = mul2(kx, uh);
+        const f2 nt = fma2(kx, nl, fma2(ky, nh, fma2(kx, nh, p)));  // -(k u - p + the cross terms)
+        const f2 s = add2(hi, p);
+        const f2 bp = fma2(hi, m1, s);
+        const f2 err = add2(fma2(fma2(bp, m1, s), m1, hi), fma2(bp, m1, p));
+        hi = s;
+        lo = add2(lo, fma2(nt, m1, err));
+    }
+}
+
 // Synchronises an element group: a one-warp group with __syncwarp, a larger
 // one with its named barrier (ids 1..15).
 __device__ __forceinline__ void group_sync(uint32_t id, uint32_t threads) {
@@ -936,30 +1006,30 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
     if (warp == G.ng * G.g) {  // producer
         if (lane == 0) {
             const uint64_t pol = l2_evict_first_policy();
-            // ring index g runs on across colours: the copies of a colour start while the previous one drains
-            uint32_t issued = 0, gbase = 0;
+            // ring index g runs on across colours: the copies of a colour start while the previous one drains. One
+            // thread issues every copy of the CTA: slot and round advance by increments (two divisions per copy
+            // held every kernel on units of a few KB to 0.6-0.65 G copies/s: split tet10 elasticity 32^3 x 6 322 ->
+            // 248 us, hex8 elasticity 72^3 348 -> 294)
+            uint32_t g = 0, s = 0, round = 0;
             bool stop = false;
             for (uint32_t col = 0; col < ncol && !stop; col++) {
                 uint32_t begin, cnt;
                 share(col, begin, cnt);
-                const unsigned char* ke = FU ? a.ke + T->ke_off[col] : a.ke;
-                const uint32_t nch = (cnt + E - 1) / E;
-                for (uint32_t c = 0; c < nch; c++) {
-                    const uint32_t g = gbase + c, s = g % S;
-                    if (g >= S && !mbar_wait_abortable(&empty[s], ((g / S) - 1) & 1, abort, a.wait_ns)) {
+                const unsigned char* src = (FU ? a.ke + T->ke_off[col] : a.ke) + (size_t)begin * a.unit_bytes;
+                // E > 1 only for whole units (copy_bytes == unit_bytes), so the chunk is contiguous
+                for (uint32_t e0 = 0; e0 < cnt; e0 += E, src += (size_t)E * a.unit_bytes) {
+                    if (round && !mbar_wait_abortable(&empty[s], (round - 1) & 1, abort, a.wait_ns)) {
                         stop = true;
                         break;
                     }
-                    const uint32_t e0 = c * E, ne = min(E, cnt - e0);
-                    tag[s] = g;
-                    // E > 1 only for whole units (copy_bytes == unit_bytes), so the chunk is contiguous
-                    mbar_arrive_expect_tx(&full[s], ne * a.copy_bytes);
-                    bulk_load(smem + (size_t)s * L.slot_bytes, ke + (size_t)(begin + e0) * a.unit_bytes,
-                              ne * a.copy_bytes, &full[s], pol);
-                    issued = g + 1;
+                    const uint32_t bytes = min(E, cnt - e0) * a.copy_bytes;
+                    tag[s] = g++;
+                    mbar_arrive_expect_tx(&full[s], bytes);
+                    bulk_load(smem + (size_t)s * L.slot_bytes, src, bytes, &full[s], pol);
+                    if (++s == S) s = 0, round++;
                 }
-                gbase += nch;
             }
+            const uint32_t issued = g;
             allow_dependent_launch();
             if (*abort) atomicOr(a.err, kErrTimeout);
             // every issued copy lands before the CTA's shared memory is released
@@ -970,11 +1040,13 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
 
     if (a.probe && blockIdx.x == 0 && warp == 0 && !probe_wait(a.probe, a.wait_ns)) *abort = 1;
     const uint32_t grp = warp / G.g, q = warp % G.g;
-    const uint32_t rg = q / G.gc, cg = q % G.gc;
+    // rows in pairs: the first gr warps gather and scatter, all of them split the columns
+    constexpr uint32_t PG = A::kPair && NT != 0 ? wpg_pair_groups(NT) : 0u;
+    const uint32_t rg = PG ? q : q / G.gc, cg = PG ? 0u : q % G.gc;
     const uint32_t r = 32 * rg + lane;
     const bool rvalid = r < n;
     const uint32_t cb = cg * n / G.gc, ce = (cg + 1) * n / G.gc;
-    const bool gatherer = (cg == 0);
+    const bool gatherer = PG ? rvalid || 32 * rg < n : cg == 0;
     const uint32_t bar_id = 1 + grp, bar_threads = G.g * 32;
     const VT* __restrict__ u = static_cast<const VT*>(a.u);
     VO* __restrict__ v = static_cast<VO*>(a.v);
@@ -982,7 +1054,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
     // the scale was written by a launch that completed before this segment's first launch
     const int usk = load_uscale<A>(a.umax);
     unsigned char* ubuf0 = ubase + (size_t)(grp * 2) * ub;
-    const uint32_t pstride = (G.gc > 1 ? G.gc - 1 : 1) * n;
+    const uint32_t pstride = (PG ? G.g * PG : G.gc > 1 ? G.gc - 1 : 1) * n;
     Acc* pbuf0 = pbase + (size_t)(grp * 2) * pstride;
     auto ubuf = [&](uint32_t p) { return reinterpret_cast<UT*>(ubuf0 + (size_t)p * ub); };
     auto pbuf = [&](uint32_t p) { return pbuf0 + (size_t)p * pstride; };
@@ -1031,7 +1103,8 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
         if (!VE && gatherer && i < cnt && rvalid) vold_c = v_load(v + (dof_c & kDofMask));
         group_sync(bar_id, bar_threads);
         bool ok = false;  // the current chunk's slot has landed (one verdict per warp and chunk)
-        uint32_t s = 0;   // the current chunk's ring slot
+        // the current chunk's ring index, slot and round; the group's next chunk is ng further on (ng < S)
+        uint32_t g = gbase + grp, s = g % S, round = g / S;
         for (uint32_t k = 0; i < cnt; k++) {
             const uint32_t par = k & 1;
             uint32_t chnn = chn, jnn = jn;
@@ -1046,15 +1119,23 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
             }
             Acc acc = A::zero();
             // one verdict per warp and chunk: the block below synchronises the warp, so no lane may skip it alone
-            if (jc == 0) {
-                const uint32_t g = gbase + ch;
-                s = g % S;
-                ok = __all_sync(0xffffffffu, ring_wait(&full[s], &tag[s], g, (g / S) & 1, abort, a.wait_ns));
-            }
+            if (jc == 0) ok = __all_sync(0xffffffffu, ring_wait(&full[s], &tag[s], g, round & 1, abort, a.wait_ns));
             if (ok) {
                 const unsigned char* ks = smem + (size_t)s * L.slot_bytes + (size_t)jc * a.unit_bytes;
                 const UT* uu = ubuf(par);
-                if (rvalid) {
+                if constexpr (PG != 0) {
+                    constexpr uint32_t GR = (NT + 31) / 32, NG = GR * wpg_gc(GR, sizeof(UT)) * PG;  // column groups
+                    constexpr int NC = NT / NG;
+                    static_assert(NT % 2 == 0 && NT % NG == 0 && NT / 2 * PG <= 32, "rows in pairs");
+                    const uint32_t l = lane % (NT / 2), h = lane / (NT / 2), cgp = q * PG + h;
+                    if (h < PG) {
+                        const float* kh = reinterpret_cast<const float*>(ks) + cgp * NC * NT + 2 * l;
+                        f2 hi, lo;
+                        split_pair_terms<NT, NC>(hi, lo, kh, kh + a.plane, uu + cgp * NC);
+                        const float2 s = unpack2(hi), t = unpack2(lo);
+                        *reinterpret_cast<float4*>(pbuf(par) + cgp * n + 2 * l) = make_float4(s.x, t.x, s.y, t.y);
+                    }
+                } else if (rvalid) {
                     if constexpr (A::kSym && NT != 0) {
                         // the column group's terms, with compile-time bounds
                         constexpr int GR = (NT + 31) / 32;
@@ -1118,7 +1199,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
                 // the chunk's last element (a CTA's last chunk may be short) releases the slot
                 if (lane == 0 && (jc + 1 == E || i + 1 == cnt)) mbar_arrive(&empty[s]);
             }
-            if (!gatherer && rvalid) pbuf(par)[(cg - 1) * n + r] = acc;
+            if (!PG && !gatherer && rvalid) pbuf(par)[(cg - 1) * n + r] = acc;
             if (gatherer && rvalid && inext < cnt) {
                 const UT x = stage_s<A>(u_n, usk);
                 ubuf(par ^ 1)[r] = x;
@@ -1126,8 +1207,15 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
             }
             group_sync(bar_id, bar_threads);
             if (gatherer) {
-                for (uint32_t c2 = 1; c2 < G.gc; c2++) {
-                    if (rvalid) A::combine(acc, pbuf(par)[(c2 - 1) * n + r]);
+                if constexpr (PG != 0) {
+                    if (rvalid) {
+                        acc = pbuf(par)[r];
+                        for (uint32_t c2 = 1; c2 < G.g * PG; c2++) A::combine(acc, pbuf(par)[c2 * n + r]);
+                    }
+                } else {
+                    for (uint32_t c2 = 1; c2 < G.gc; c2++) {
+                        if (rvalid) A::combine(acc, pbuf(par)[(c2 - 1) * n + r]);
+                    }
                 }
                 if (rvalid && !*abort) {
                     const VO x = finish_s<A>(acc, usk);
@@ -1139,6 +1227,11 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
                 dof_c = dof_n;
                 vold_c = vold_n;
                 dof_n = dof_nn;
+            }
+            if (jn == 0) {
+                g += G.ng;
+                s += G.ng;
+                if (s >= S) s -= S, round++;
             }
             ch = chn;
             jc = jn;

@@ -35,6 +35,7 @@ void* pick_wpg(uint32_t n, bool chunked) {
             case 20: return kernel_ptr<20, true, false, true, VE>();
             case 24: return kernel_ptr<24, true, false, true, VE>();
             case 30: return kernel_ptr<30, true, false, true, VE>();
+            case 60: return kernel_ptr<60, true, false, true, VE>();
             default: return kernel_ptr<0, true, false, true, VE>();
         }
     }
@@ -48,7 +49,8 @@ void* pick_wpg(uint32_t n, bool chunked) {
 }
 
 // chunked: warp-group launches whose ring slots hold several units (small
-// elements; hex20's units fill a slot alone and keep the single-unit kernel).
+// elements, and the FP32 units of hex20; its 28.8 KB units fill a slot alone and
+// keep the single-unit kernel).
 // ve: element products to a buffer (SegArgs::ve).
 void* pick_kernel(int regime, uint32_t n, bool dup, bool chunked = false, bool ve = false) {
     if (regime == REG_TPE) {
@@ -73,10 +75,16 @@ void* pick_kernel(int regime, uint32_t n, bool dup, bool chunked = false, bool v
 // land, and each SM needs ~200 KB of copies in flight to keep HBM busy, which
 // small slots reach only with many stages.
 constexpr uint32_t kMaxStages = 32;
+// Shared memory of a segment CTA: with 8-byte staged u the 196 KB configuration
+// (with the 1 KB the system takes), which leaves L1 60 KB for the gathers (tet10
+// elasticity 32^3 x 6 split 248 -> 239 us, hex8 elasticity 48^3 92 -> 91.5, hex20
+// 42^3 307 -> 305.5); FP32 rings use the depth (tet10 elasticity 92 us, 97 with 194
+// KB).
+constexpr uint32_t kRingBudget = sizeof(typename ARITH::UT) == 8 ? 194u * 1024 : kSmemBudget;
 #ifdef LAUNCH_FN
 static uint32_t stages_for(uint32_t slot_bytes, uint32_t extra) {
-    if (extra + 32 >= kSmemBudget) return 0;
-    uint32_t st = (kSmemBudget - extra - 32) / (slot_bytes + 20);
+    if (extra + 32 >= kRingBudget) return 0;
+    uint32_t st = (kRingBudget - extra - 32) / (slot_bytes + 20);
     return st > kMaxStages ? kMaxStages : st;
 }
 
@@ -104,7 +112,8 @@ static RingLayout ring_layout(const Segment& s, uint64_t copy_bytes, uint64_t un
         G.gc = wpg_gc(G.gr, (uint32_t)ut);
         G.g = G.gr * G.gc;
         const uint32_t ub = wpg_ubuf_bytes(ARITH::kSym ? 2 * s.n : s.n, (uint32_t)ut);  // u staged twice (symmetric)
-        const uint32_t pstride = (G.gc > 1 ? G.gc - 1 : 1) * s.n;
+        const uint32_t pair = ARITH::kPair ? wpg_pair_groups(s.n) : 0u;
+        const uint32_t pstride = (pair ? G.g * pair : G.gc > 1 ? G.gc - 1 : 1) * s.n;
         // groups of one warp synchronise with __syncwarp; larger groups take one named barrier each (ids 1..15;
         // a fused launch keeps id 15 for its grid barrier)
         const uint32_t ng_max =
@@ -254,6 +263,14 @@ namespace {
 // ring slots).
 constexpr bool kF32Patch = sizeof(typename ARITH::VT) == 4;
 constexpr uint32_t kMinPatchStages = kF32Patch ? 6 : 5;  // ring slots below which fewer groups are used
+// Shared memory of a patch CTA. FP32: with the 1 KB the system takes, the 196 KB
+// configuration, which leaves L1 60 KB for the gathers instead of 28 (tet10
+// Poisson 50^3 x 6 43.6 -> 39.4 us, hex8 Poisson 80^3 28.6 -> 26.8). 8-byte entries
+// need the ring more (190 KB: tet10 Poisson 52^3 x 6 103 -> 111 us), but leave
+// room beside them for the CTAs of a CG iteration's vector launches, so that the
+// next product's CTAs are resident before those end (226 KB: FP64 CG of hex8
+// Poisson 32^3 2.53 -> 2.83 ms).
+constexpr uint32_t kPatchSmemBudget = (kF32Patch ? 194u : 200u) * 1024;
 
 // warps per group for G groups
 constexpr int patch_gw(int G) { return kF32Patch || G == 8 ? 2 : 4; }
@@ -285,8 +302,8 @@ PatchLayout patch_layout_g(const PatchPlanGeom& pg, uint32_t copy_bytes, uint32_
     L.ve_bytes = patch_r16(pg.n * pg.max_slots * (uint32_t)sizeof(typename ARITH::Acc));
     const uint32_t fixed = 16 * kPatchMaxGroups + 16 + 16 + L.groups * L.group_bytes();
     L.stages = 0;
-    if (fixed < kSmemBudget) {
-        const uint32_t st = (kSmemBudget - fixed) / (L.slot_bytes + 20);
+    if (fixed < kPatchSmemBudget) {
+        const uint32_t st = (kPatchSmemBudget - fixed) / (L.slot_bytes + 20);
         L.stages = st > kMaxStages ? kMaxStages : st;
     }
     return L;
