@@ -130,8 +130,7 @@ __global__ void __launch_bounds__(kRedThreads) k_set_constrained(T* v, const T* 
 
 // part[block]: partial sums of a.b
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_dot(const T* a, const T* b, size_t n,
-                                                     double* part) {
+__global__ void __launch_bounds__(kRedThreads) k_dot(const T* a, const T* b, size_t n, double* part) {
     __shared__ double sh[kRedThreads];
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -148,8 +147,37 @@ __global__ void __launch_bounds__(kRedThreads) k_dot(const T* a, const T* b, siz
         for (int q = 0; q < kUnroll; q++) ab.add(x[q], y[q]);
     }
     for (; i < n; i += kStride) ab.add(a[i], b[i]);
-    const double s = block_sum(ab.value(), sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    const double v[1] = {ab.value()};
+    block_partials(v, sh, part);
+}
+
+// r = b - q (r may be q), with the partials of r.r: one pass where a copy, an update and a dot product were three. A
+// mixed solve is bound by launches and host turns between its segments; with this, the update of the recursion in two
+// launches and a segment's first batch enqueued with it, hex8 Poisson 24^3 (69 iterations, 11 segments) went from 2605
+// to 2290 us.
+__global__ void __launch_bounds__(kRedThreads) k_residual(double* r, const double* b, const double* q, size_t n,
+                                                          double* part) {
+    __shared__ double sh[kRedThreads];
+    DotAcc<double> rr;
+    for (size_t i = (size_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += kUnroll * kStride) {
+        double x[kUnroll], y[kUnroll];
+#pragma unroll
+        for (int k = 0; k < kUnroll; k++) {
+            const size_t j = i + k * kStride;
+            if (j < n) x[k] = b[j], y[k] = q[j];
+        }
+#pragma unroll
+        for (int k = 0; k < kUnroll; k++) {
+            const size_t j = i + k * kStride;
+            if (j < n) {
+                const double t = x[k] - y[k];
+                r[j] = t;
+                rr.add(t, t);
+            }
+        }
+    }
+    const double v[1] = {rr.value()};
+    block_partials(v, sh, part);
 }
 
 // r = b - q, z = dinv r, p = z; partials of r.z, r.r, z.z, b.b, (dinv b).(dinv b)
@@ -193,11 +221,20 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_init_final(double* sc, const
         sc[S_ZZ] = zz;
         sc[S_BB] = bb;
         sc[S_DB] = db;
-        sc[S_FLAG] = (rz < 0.0 || rz != rz) ? 1.0 : 0.0;
-        sc[S_DONE] = 0.0;
+        const bool bad = rz < 0.0 || rz != rz;
+        sc[S_FLAG] = bad ? 1.0 : 0.0;
+        sc[S_DONE] = bad ? 1.0 : 0.0;
         sc[S_ITER] = 0.0;
     }
 }
+
+// Launches of one CG iteration follow one another with programmatic
+// dependence: each waits for the one before it in full, but is on the SMs by
+// then. What a launch before may write is read with plain loads (no
+// __restrict__ const pointers, no ld.global.nc, whose lines may have been in
+// L1 since before the write).
+__device__ __forceinline__ void wait_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // Reliable update of the FP32 recursion of the mixed-precision solve, pass 1:
 // r = fl32(sigma r64) (the FP64 true residual in the new segment's scale),
@@ -208,7 +245,8 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_reliable(const double* __res
                                                              T* __restrict__ z, const T* __restrict__ p,
                                                              const T* __restrict__ dinv, size_t n, double* part,
                                                              double sigma) {
-    __shared__ double sh[kRedThreads];
+    __shared__ double sh[4 * kRedThreads];
+    release_next();
     double rz = 0, rr = 0, zz = 0, rp = 0;
     for (size_t i = (size_t)blockIdx.x * kRedThreads + threadIdx.x; i < n; i += kStride) {
         const T ri = (T)(r64[i] * sigma);
@@ -220,66 +258,58 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_reliable(const double* __res
         zz = __fma_rn((double)zi, (double)zi, zz);
         rp = __fma_rn((double)ri, (double)p[i], rp);
     }
-    double v[4] = {rz, rr, zz, rp};
-    for (int j = 0; j < 4; j++) {
-        const double s = block_sum(v[j], sh);
-        if (threadIdx.x == 0) part[j * kRedBlocks + blockIdx.x] = s;
-    }
+    const double v[4] = {rz, rr, zz, rp};
+    block_partials(v, sh, part);
 }
 
-// pass 2 (one block): beta = r.z / (rho r_k.z_k), gamma = r.p / r.z; S_DONE,
-// S_ITER cleared. rho = sigma_new / sigma_old, the change of the residual's
-// scale: with r, z in the new scale and p, r_k.z_k in the old one,
-// p = z + beta (p - gamma z) is the scaled form of the unscaled update.
-__global__ void __launch_bounds__(kRedThreads) k_cg_reliable_final(double* sc, const double* part, uint32_t nb,
-                                                                   double rho) {
-    __shared__ double sh[kRedThreads];
-    const double rz = final_sum(part, sh, nb);
-    const double rr = final_sum(part + kRedBlocks, sh, nb);
-    const double zz = final_sum(part + 2 * kRedBlocks, sh, nb);
-    const double rp = final_sum(part + 3 * kRedBlocks, sh, nb);
-    if (threadIdx.x == 0) {
-        const double old = sc[S_RZOLD];
-        const bool bad = (rz < 0.0 || rz != rz);
-        sc[S_BETA] = (!bad && old > 0.0) ? rz / (old * rho) : 0.0;
-        sc[S_GAMMA] = (!bad && rz > 0.0) ? rp / rz : 0.0;
-        sc[S_RZ] = rz;
-        sc[S_RR] = rr;
-        sc[S_ZZ] = zz;
-        sc[S_FLAG] = bad ? 1.0 : 0.0;
-        sc[S_DONE] = 0.0;
-        sc[S_ITER] = 0.0;
-    }
-}
-
-// pass 3: p = z + beta (p - gamma z)
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// pass 2: beta = r.z / (rho r_k.z_k), gamma = r.p / r.z (every block adds up
+// the partials; the first writes the scalars and clears S_DONE, or sets it on
+// breakdown, and S_ITER), p = z + beta (p - gamma z). rho = sigma_new /
+// sigma_old, the change of the residual's scale: with r, z in the new scale and
+// p, r_k.z_k in the old one this is the scaled form of the unscaled update.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_cg_reliable_p(T* __restrict__ p, const T* __restrict__ z,
-                                                               size_t n, const double* sc) {
-    const T beta = (T)sc[S_BETA];
-    const T c = (T)(1.0 - sc[S_BETA] * sc[S_GAMMA]);
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        p[i] = fma_rn(beta, p[i], c * z[i]);
+__global__ void __launch_bounds__(kRedThreads) k_cg_reliable_p(T* p, const T* z, size_t n, double* sc,
+                                                               const double* part, uint32_t nb, double rho) {
+    __shared__ double sums[4];
+    __shared__ double coef[2];
+    wait_launch();
+    const uint32_t t = threadIdx.x;
+    if (t < 128) {
+        const double s = row_sum(part + (t >> 5) * kRedBlocks, nb);
+        if ((t & 31) == 0) sums[t >> 5] = s;
+    }
+    __syncthreads();
+    if (t == 0) {
+        const double rz = sums[0], old = sc[S_RZOLD];
+        const bool bad = rz < 0.0 || rz != rz;
+        const double beta = (!bad && old > 0.0) ? rz / (old * rho) : 0.0;
+        const double gamma = (!bad && rz > 0.0) ? sums[3] / rz : 0.0;
+        coef[0] = beta;
+        coef[1] = 1.0 - beta * gamma;
+        if (blockIdx.x == 0) {
+            sc[S_BETA] = beta;
+            sc[S_GAMMA] = gamma;
+            sc[S_RZ] = rz;
+            sc[S_RR] = sums[1];
+            sc[S_ZZ] = sums[2];
+            sc[S_FLAG] = bad ? 1.0 : 0.0;
+            sc[S_DONE] = bad ? 1.0 : 0.0;
+            sc[S_ITER] = 0.0;
+        }
+    }
+    __syncthreads();
+    const T beta = (T)coef[0], c = (T)coef[1];
+    for (size_t i = (size_t)blockIdx.x * kRedThreads + t; i < n; i += kStride) p[i] = fma_rn(beta, p[i], c * z[i]);
 }
 
-// sc[S_PQ] = sum of the partials (a plain reduction, no CG bookkeeping)
-__global__ void __launch_bounds__(kRedThreads) k_sum(double* sc, const double* part, uint32_t nb) {
-    __shared__ double sh[kRedThreads];
-    const double s = final_sum(part, sh, nb);
+// sc[S_PQ] = sum of the partials (a plain reduction, no CG bookkeeping; one warp)
+__global__ void k_sum(double* sc, const double* part, uint32_t nb) {
+    const double s = row_sum(part, nb);
     if (threadIdx.x == 0) sc[S_PQ] = s;
 }
-
-// Launches of one CG iteration follow one another with programmatic
-// dependence: each waits for the one before it in full, but is on the SMs by
-// then. What a launch before may write is read with plain loads (no
-// __restrict__ const pointers, no ld.global.nc, whose lines may have been in
-// L1 since before the write).
-__device__ __forceinline__ void wait_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // First half of an iteration: alpha = r.z / p.q (every block adds up the
 // partials of p.q itself), x += alpha p, r -= alpha q; partials of r.z, r.r,
@@ -757,18 +787,24 @@ template <typename T>
 cudaError_t launch_norm2(const T* a, size_t n, double* sc, double* part, cudaStream_t st) {
     const uint32_t nb = red_blocks(n);
     k_dot<T><<<nb, kRedThreads, 0, st>>>(a, a, n, part);
-    k_sum<<<1, kRedThreads, 0, st>>>(sc, part, nb);
+    k_sum<<<1, 32, 0, st>>>(sc, part, nb);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_residual(double* r, const double* b, const double* q, size_t n, double* sc, double* part,
+                            cudaStream_t st) {
+    const uint32_t nb = cg_blocks(n);
+    k_residual<<<nb, kRedThreads, 0, st>>>(r, b, q, n, part);
+    k_sum<<<1, 32, 0, st>>>(sc, part, nb);
     return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_cg_reliable(const double* r64, T* r, T* z, T* p, const T* dinv, size_t n, double* sc,
                                double* part, double sigma, double rho, cudaStream_t st) {
-    const uint32_t nb = red_blocks(n);
+    const uint32_t nb = cg_blocks(n);
     k_cg_reliable<T><<<nb, kRedThreads, 0, st>>>(r64, r, z, p, dinv, n, part, sigma);
-    k_cg_reliable_final<<<1, kRedThreads, 0, st>>>(sc, part, nb, rho);
-    k_cg_reliable_p<T><<<grid_for(n), kRedThreads, 0, st>>>(p, z, n, sc);
-    return cudaGetLastError();
+    return launch(k_cg_reliable_p<T>, nb, true, st, p, (const T*)z, n, sc, (const double*)part, nb, rho);
 }
 template cudaError_t launch_cg_reliable<float>(const double*, float*, float*, float*, const float*, size_t, double*,
                                                double*, double, double, cudaStream_t);

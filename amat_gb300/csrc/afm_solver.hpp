@@ -67,11 +67,15 @@ cudaError_t launch_invert(T* dinv, const double* d, size_t n, cudaStream_t st);
 // sc[S_PQ] = ||a||^2 (no CG bookkeeping)
 template <typename T>
 cudaError_t launch_norm2(const T* a, size_t n, double* sc, double* part, cudaStream_t st);
+// r = b - q (r may be q), sc[S_PQ] = ||r||^2
+cudaError_t launch_residual(double* r, const double* b, const double* q, size_t n, double* sc, double* part,
+                            cudaStream_t st);
 // Reliable update of the FP32 recursion (after a segment stopped on S_DONE,
 // p is still the last direction p_k): r = fl32(r64), z = dinv r,
 // p = z + beta (p - gamma z) with beta = r.z / r_k.z_k and gamma = r.p / r.z,
 // so that the new residual is orthogonal to the kept direction again;
-// sc[S_RZ], sc[S_RR], sc[S_ZZ] of the new residual; S_DONE and S_ITER cleared.
+// sc[S_RZ], sc[S_RR], sc[S_ZZ] of the new residual; S_ITER cleared, S_DONE too
+// (set on breakdown, with S_FLAG).
 // The recursion runs on the residual times a power of two: sigma is the new
 // segment's scale (r = fl32(sigma r64)), rho = sigma / the previous segment's.
 // T = float (the FP32 recursion) or double (the FP64-vector recursion of
