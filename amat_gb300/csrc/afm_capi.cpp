@@ -44,6 +44,8 @@ cudaError_t launch_batched_split(const Segment& s, const BatchArgs& a, int sm_co
                                  cudaStream_t st);
 cudaError_t launch_fused_split(const Segment* segs, uint32_t ncol, const SegArgs& a, unsigned* gbar, int sm_count,
                                cudaStream_t st);
+cudaError_t launch_fused_splitblk(const Segment* segs, uint32_t ncol, const SegArgs& a, unsigned* gbar, int sm_count,
+                                  cudaStream_t st);
 bool batched_tc_supported(uint32_t n, uint32_t nrhs);
 cudaError_t launch_batched_tc(const Segment& s, const BatchArgs& a, int sm_count, bool pdl, cudaStream_t stream);
 cudaError_t launch_batched_fp32(const Segment& s, const BatchArgs& a, int sm_count, int tr, int ng, bool pdl,
@@ -80,6 +82,10 @@ cudaError_t launch_patches_splitsym(const PatchPlanGeom& pg, const PatchArgs& a,
                                     cudaStream_t st);
 cudaError_t configure_kernels_splitsym();
 size_t patch_smem_splitsym(const PatchPlanGeom& pg, uint32_t copy_bytes);
+cudaError_t launch_segment_splitblk(const Segment& s, const SegArgs& a, int sm_count, bool dup, bool pdl,
+                                    cudaStream_t st);
+cudaError_t configure_kernels_splitblk();
+size_t segment_smem_splitblk(const Segment& s);
 size_t patch_smem_f32symc(const PatchPlanGeom& pg, uint32_t copy_bytes);
 size_t segment_smem_f32symc(const Segment& s);
 size_t patch_smem_splitsymx(const PatchPlanGeom& pg, uint32_t copy_bytes);
@@ -138,6 +144,7 @@ cudaError_t launch_segment(const Segment& s, int prec, const SegArgs& a, int sm_
         case kPrecF32SymX: return launch_segment_f32symx(s, a, sm_count, dup, pdl, stream);
         case kPrecSplitSymX: return launch_segment_splitsymx(s, a, sm_count, dup, pdl, stream);
         case kPrecF32SymC: return launch_segment_f32symc(s, a, sm_count, dup, pdl, stream);
+        case kPrecSplitBlk: return launch_segment_splitblk(s, a, sm_count, dup, pdl, stream);
         default: return launch_segment_fp32(s, a, sm_count, dup, pdl, stream);
     }
 }
@@ -776,21 +783,26 @@ int buffer_done(afm_operator* op, cudaStream_t st) {
 // True when every element matrix is symmetric to within 1e-6 of its largest
 // diagonal entry (exactly, for an element whose diagonal is zero). *exact:
 // every one equal to its transpose.
-bool ke_is_symmetric(const afm_operator* op, bool* exact) {
-    int sym = 1, same = 1;
-#pragma omp parallel for schedule(static) reduction(&& : sym, same)
+bool ke_is_symmetric(const afm_operator* op, bool* exact, bool* near) {
+    int sym = 1, same = 1, close = 1;
+#pragma omp parallel for schedule(static) reduction(&& : sym, same, close)
     for (int64_t e = 0; e < (int64_t)op->n_elem; e++) {
         if (!sym) continue;
         const uint32_t n = op->offsets[e + 1] - op->offsets[e];
         const double* k = op->ke.data() + op->kofs[e];
-        double dmax = 0.0;
-        for (uint32_t r = 0; r < n; r++) dmax = std::max(dmax, std::fabs(k[(size_t)r * n + r]));
+        double dmax = 0.0, dmin = 1e300;
+        for (uint32_t r = 0; r < n; r++) {
+            const double d = std::fabs(k[(size_t)r * n + r]);
+            dmax = std::max(dmax, d);
+            dmin = std::min(dmin, d);
+        }
         const double tol = 1e-6 * dmax;
         for (uint32_t r = 0; r < n && sym; r++)
             for (uint32_t c = r + 1; c < n; c++) {
                 const double x = k[(size_t)r * n + c], y = k[(size_t)c * n + r];
                 if (x == y) continue;
                 same = 0;
+                if (!(std::fabs(x - y) <= kBlockAsym * dmin)) close = 0;
                 if (!(std::fabs(x - y) <= tol)) {
                     sym = 0;
                     break;
@@ -798,6 +810,7 @@ bool ke_is_symmetric(const afm_operator* op, bool* exact) {
             }
     }
     *exact = sym && same;
+    *near = sym && close;
     return sym != 0;
 }
 
@@ -1035,6 +1048,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     float* const d_v32 = static_cast<float*>(d_v);
     if (via_vx) d_v = op->d_vx;
     const bool scaled = kprec == AFM_PREC_FP64_SPLIT || kprec == kPrecSplitSymX;
+    const bool blocks = kprec == AFM_PREC_FP64_SPLIT && !op->use_patches && op->d_packed;
     // one launch for every element plus the gather pass, which writes every entry of v
     bool gather = false;
     const bool fused = op->fused && op->fused_ok && kprec == AFM_PREC_FP64_SPLIT && !sym && !f32;
@@ -1058,12 +1072,16 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         a.copy_bytes = (uint32_t)a.unit_bytes;
         a.plane = sym ? s.sym_plane : s.plane;
         if (f32 && !sym && op->precision == AFM_PREC_FP64_SPLIT) a.copy_bytes = s.plane * 4;
+        if (blocks) {
+            a.ke = op->d_packed;
+            a.unit_bytes = a.copy_bytes = split_block_bytes(s.n);
+        }
         a.bc_mode = bc_mode;
         a.err = op->d_err;
         a.umax = op->d_usc;
         a.wait_ns = op->wait_ns;
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
-        AFM_CUDA(launch_segment(s, kprec, a, op->sm_count, false, false, st));
+        AFM_CUDA(launch_segment(s, blocks ? kPrecSplitBlk : kprec, a, op->sm_count, false, false, st));
         const int vt_bytes = f32 || kprec == AFM_PREC_FP32 ? 4 : 8;
         double* part = tail && op->n_dofs <= kFusedDotDofs ? tail->part : nullptr;
         AFM_CUDA(launch_gather_sum(ve_bytes, vt_bytes, op->gather_b, via_vx ? (void*)d_v32 : d_v, op->d_ve,
@@ -1153,7 +1171,11 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         a.wait_ns = op->wait_ns;
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
         AFM_CUDA(cudaMemsetAsync(op->d_gbar, 0, sizeof(unsigned) * op->segs.size(), st));
-        AFM_CUDA(launch_fused_split(op->segs.data(), (uint32_t)op->segs.size(), a, op->d_gbar, op->sm_count, st));
+        if (blocks) {
+            a.ke = op->d_packed;
+            a.unit_bytes = a.copy_bytes = split_block_bytes(s0.n);
+        }
+        AFM_CUDA((blocks ? launch_fused_splitblk : launch_fused_split)(op->segs.data(), (uint32_t)op->segs.size(), a, op->d_gbar, op->sm_count, st));
         return AFM_SUCCESS;
     }
     for (const Segment& s : op->segs) {
@@ -1169,13 +1191,17 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         a.copy_bytes = (uint32_t)a.unit_bytes;
         a.plane = sym ? s.sym_plane : s.plane;
         if (f32 && !sym && op->precision == AFM_PREC_FP64_SPLIT) a.copy_bytes = s.plane * 4;
+        if (blocks) {
+            a.ke = op->d_packed + s.blk_offset;
+            a.unit_bytes = a.copy_bytes = split_block_bytes(s.n);
+        }
         a.bc_mode = bc_mode;
         a.err = op->d_err;
         a.umax = op->d_usc;
         a.wait_ns = op->wait_ns;
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
         // every launch after the first may overlap its prologue with the previous one's tail
-        AFM_CUDA(launch_segment(s, kprec, a, op->sm_count, op->dup_in_element, !first, st));
+        AFM_CUDA(launch_segment(s, blocks ? kPrecSplitBlk : kprec, a, op->sm_count, op->dup_in_element, !first, st));
         first = false;
     }
     if (via_vx) AFM_CUDA(launch_to_f32(d_v32, op->d_vx, op->n_dofs, st));
@@ -2090,6 +2116,7 @@ int afm_create(afm_operator** out, int bc_method, int device) {
         configure_kernels_fp32() != cudaSuccess || configure_kernels_f32sym() != cudaSuccess ||
         configure_kernels_f32symx() != cudaSuccess || configure_kernels_splitsymx() != cudaSuccess ||
         configure_kernels_f32symc() != cudaSuccess || configure_kernels_splitsym() != cudaSuccess ||
+        configure_kernels_splitblk() != cudaSuccess ||
         configure_bpatch() != cudaSuccess)
         return fail(AFM_ERR_CUDA, "kernel configuration failed on device %d", device);
     auto* op = new afm_operator();
@@ -2693,11 +2720,12 @@ int afm_finalize(afm_operator* op) {
     // symmetric Ke, and elements that run as patches or on the warp-group kernel
     op->ke_symmetric = false;
     op->ke_sym_exact = false;
+    op->ke_sym_near = false;
     op->sym_ok = false;
     op->sym_bytes = 0;
     op->sym_built = 0;
     if (prec == AFM_PREC_FP64_SPLIT && !op->dup_in_element && op->n_elem > 0) {
-        op->ke_symmetric = ke_is_symmetric(op, &op->ke_sym_exact);
+        op->ke_symmetric = ke_is_symmetric(op, &op->ke_sym_exact, &op->ke_sym_near);
         bool covered = true;
         if (!op->use_patches)
             for (const Segment& s : op->segs)
@@ -2713,7 +2741,25 @@ int afm_finalize(afm_operator* op) {
                 AFM_CUDA(pack_split_units(op->d_ke, s.n, s.units, op->d_packed, op->sm_count, op->stream));
             }
         }
+        if (!op->use_patches && op->ke_sym_near && op->n_elem >= kBlockElemsPerSm * (uint64_t)std::max(op->sm_count, 1)) {
+            uint64_t bytes = 0;
+            for (Segment& s : op->segs) {
+                if (s.units == 0) continue;
+                if (s.regime != REG_WPE || !split_block_bytes(s.n)) covered = false;
+                s.blk_offset = bytes;
+                bytes += (uint64_t)split_block_bytes(s.n) * s.units;
+            }
+            if (covered && dalloc(op, &op->d_packed, std::max<uint64_t>(bytes, 16)) != cudaSuccess) {
+                cudaGetLastError();  // no room: as above
+                op->d_packed = nullptr;
+            } else if (covered) {
+                for (const Segment& s : op->segs)
+                    AFM_CUDA(pack_split_blocks(op->d_ke + s.ke_offset, s.unit_bytes, s.plane, s.n, s.units,
+                                               op->d_packed + s.blk_offset, op->sm_count, op->stream));
+            }
+        }
     }
+    if (op->d_packed) AFM_CUDA(cudaStreamSynchronize(op->stream));  // products may run on other streams
     op->ke_dirty = false;
     op->finalized = true;
     return ok();

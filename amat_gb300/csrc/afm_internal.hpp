@@ -49,6 +49,7 @@ struct Segment {
     uint32_t plane = 0;       // FP64_SPLIT: entries per plane of a unit (the lo plane follows the hi plane)
     uint64_t sym_offset = 0;     // byte offset of the first unit in the symmetric inner arena
     uint64_t sym_unit_bytes = 0; // its bytes per unit (0: no symmetric form)
+    uint64_t blk_offset = 0;     // byte offset of the first unit in the arena of block units
     uint32_t sym_plane = 0;      // entries of a unit's FP32 plane before its BF16 correction plane (0: none)
 };
 
@@ -216,6 +217,25 @@ constexpr int kPrecF32SymC = 19;
 
 // FP64 vectors, the split arithmetic on packed symmetric patch units (ArithSplitSym).
 constexpr int kPrecSplitSym = 20;
+// ... and on symmetric element units of 2 x 2 blocks (ArithSplitBlk).
+constexpr int kPrecSplitBlk = 21;
+// Bytes of such a unit (0: no block kernel for this size): n/4 + 1 (rounded down) wrapped diagonals of n/2 blocks with
+// 4 hi, 4 lo entries and 4 bytes each, and 16 bytes with the bytes' unit.
+constexpr uint32_t split_block_bytes(uint32_t n) {
+    return n == 60 ? (n / 4 + 1) * (n / 2) * 36 + 16 : 0u;
+}
+// Largest |K(r, c) - K(c, r)| of a block unit, relative to the element's smallest diagonal entry: its byte then holds the
+// difference to 2^-53 of that entry, half the last place of the FP64 sums that K came from, in every row of an element
+// with rows of very different sizes too (relative to the largest, rows 1e10 smaller would lose 8 digits). Matrices from
+// quadrature on this library's meshes differ by 2^-52 to 2^-50.
+constexpr double kBlockAsym = 0x1p-46;
+// Elements per SM from which a plan takes block units (24 consumer warps hold 6 elements of an SM; below about ten each
+// the longer way of one element shows): hex20 elasticity with 1000 elements 11.4 us on whole units, 13.1 on blocks; 1331
+// 13.2 and 13.6; 1440 14.2 and 14.0; 1584 15.1 and 14.0; 2744 20.2 and 19.4.
+constexpr uint32_t kBlockElemsPerSm = 10;
+// Packs a segment's split units into block units (afm_mv_splitblk.cu).
+cudaError_t pack_split_blocks(const unsigned char* ke, uint64_t unit_bytes, uint32_t plane, uint32_t n, uint32_t units,
+                              unsigned char* dst, int sm_count, cudaStream_t st);
 
 // Packs a patch plan's split units (afm_mv_splitsym.cu).
 cudaError_t pack_split_units(const unsigned char* ke, uint32_t n, uint32_t units, unsigned char* packed, int sm_count,
@@ -366,7 +386,9 @@ struct afm_operator {
     // entries stored once, built from the split arena on the first FP32 product
     bool ke_symmetric = false;      // every Ke symmetric to 1e-6 of its largest diagonal entry
     bool ke_sym_exact = false;      // every Ke equal to its transpose bit for bit
-    // the split units of a patch plan with such Ke, packed (FP64 products read them; null: they read d_ke)
+    bool ke_sym_near = false;       // ... or to kBlockAsym
+    // the split units of a patch plan with exactly symmetric Ke, packed, or of a segment plan with nearly symmetric Ke of
+    // 60 DoFs, as block units (FP64 products read them; null: they read d_ke)
     unsigned char* d_packed = nullptr;
     bool sym_ok = false;            // symmetric, split arena, and a layout the symmetric kernels cover
     int sym_mode = 1;               // afm_set_symmetric_inner: 0 off, 1 FP32, 2 FP32 + BF16 correction

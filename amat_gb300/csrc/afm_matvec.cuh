@@ -394,6 +394,17 @@ struct ArithSplitSym : ArithSplit {
     static constexpr bool kSym = true;
 };
 
+// The split arithmetic on element units of 2 x 2 blocks, each pair of a block
+// and its transpose once (split_block_terms).
+struct ArithSplitBlk : ArithSplit {
+    static constexpr bool kSym = true;  // (u staged twice in a row)
+    static constexpr uint32_t kWpgWarps = 24;  // hex20 42^3: 16 warps 290 us, 20 272 (even runs); 20 248, 24 239 (uneven)
+};
+template <typename A>
+inline constexpr bool kBlocks = false;
+template <>
+inline constexpr bool kBlocks<ArithSplitBlk> = true;
+
 // FP64 products from the corrected symmetric arena (the arena of ArithF32SymX:
 // K to about 2^-32, each pair of entries once): u and v are FP64 vectors, u is
 // staged as a scaled float pair like the split arithmetic, and each product
@@ -890,6 +901,99 @@ __device__ __forceinline__ void split_pair_terms(f2& hi, f2& lo, const float* kh
     }
 }
 
+// One product term of ArithSplit::fma for two floats at once: (hi, lo) += (k + kl)(u + ul), nu = -u. Each difference is
+// a multiply-add by -1 (exact products: the same roundings).
+__device__ __forceinline__ void split_term2(f2& hi, f2& lo, f2 k, f2 kl, f2 u, f2 nu, f2 ul) {
+    const f2 m1 = pack2(-1.0f, -1.0f);
+    const f2 np = mul2(k, nu);  // -p
+    const f2 t = fma2(k, ul, fma2(kl, u, fma2(k, u, np)));
+    const f2 s = fma2(np, m1, hi);
+    const f2 bp = fma2(hi, m1, s);
+    const f2 err = fma2(add2(np, bp), m1, fma2(fma2(bp, m1, s), m1, hi));
+    hi = s;
+    lo = add2(lo, add2(err, t));
+}
+
+// ArithSplit::combine for two sums at once.
+__device__ __forceinline__ void split_combine2(f2& hi, f2& lo, f2 bhi, f2 blo) {
+    const f2 m1 = pack2(-1.0f, -1.0f);
+    const f2 s = add2(hi, bhi);
+    const f2 bp = fma2(hi, m1, s);
+    const f2 err = add2(fma2(fma2(bp, m1, s), m1, hi), fma2(bp, m1, bhi));
+    hi = s;
+    lo = add2(lo, add2(blo, err));
+}
+
+// Block units (ArithSplitBlk; elements of 60 DoFs whose Ke is symmetric to 2^-46 of its smallest diagonal entry): NB =
+// n / 2 block rows of 2 x 2 blocks B(i, j); of each pair B(i, j), B(j, i) one is stored, by wrapped diagonals d = 0 ..
+// NB / 2: block (i, (i + d) mod NB) at d NB + i, its hi entries row by row in one float4, its lo entries in a second
+// plane. Element matrices from quadrature are symmetric only up to rounding, so a third plane holds K(c, r) - K(r, c) of
+// each entry as a biased byte times a power of two per element (the float after the plane): K(r, c) is the split
+// arena's to the bit, K(c, r) to 2^-53 of that diagonal entry. 60% of the whole matrix's bytes.
+// The operations stay those of the whole matrix but for the third plane's (a byte permutation and an add and a
+// multiply-add per entry of a transposed block) and 4 shuffles per diagonal.
+// A lane owns block row i. For each diagonal it adds B(i, j) u_j to its own sums, and B(i, j)^T u_i to the sums of
+// block row j, which travel: the lane that needs them for the next diagonal is the neighbour. The own sums are kept
+// per column parity (row 0: (k00 x0, k01 x1)), so that every operand is a pair as loaded: no packing in the loop.
+// Diagonals 0 and NB / 2 hold both blocks of a pair and have no transposed part. Warp q of the element's four takes
+// diagonals [block_run(q), block_run(q + 1)): 3, 3, 5 and 5, as the first two also gather u and scatter v, and the others
+// would wait for them at the element's barrier (42^3: 2, 2, 6 and 6 261 us, 4 each 278, this 248, with 20 warps).
+// What bounds it now is the double-float arithmetic and its latencies (0.4 to 0.6 instructions issued per cycle), so the
+// gain is below the bytes': hex20 elasticity 42^3 306 -> 239 us a product (5.4 TB/s), 56^3 715 -> 534, 14^3 20.2 -> 19.4. In
+// elements of 24 and 30 DoFs (two runs of diagonals per warp) the overhead per element outweighs it: hex8 elasticity
+// 48^3 92 -> 97 us, tet10 elasticity 32^3 x 6 240 -> 241.
+template <int NT>
+__host__ __device__ constexpr int block_run(int q) {
+    constexpr int ND = NT / 4 + 1, A = 3;  // (A: the gathering warps' diagonals)
+    return q <= 2 ? q * A : q == 3 ? 2 * A + (ND - 2 * A) / 2 : ND;
+}
+template <int NT, int Q>
+__device__ __forceinline__ void split_block_terms(f2& hi, f2& lo, const unsigned char* ks, const float4* ub, uint32_t lane) {
+    constexpr int NB = NT / 2, ND = NB / 2 + 1, D0 = block_run<NT>(Q), D1 = block_run<NT>(Q + 1);
+    static_assert(NB % 2 == 0 && NB <= 32, "block rows of a warp");
+    // (lanes past the last block row repeat the first lanes' work; nothing of theirs is used)
+    const int l = (int)lane < NB ? (int)lane : (int)lane - NB;
+    const float4* kp = reinterpret_cast<const float4*>(ks) + l;
+    const uint32_t* dp = reinterpret_cast<const uint32_t*>(ks + ND * NB * 32) + l;
+    const float4* xp = ub + l;
+    const float step = *reinterpret_cast<const float*>(ks + ND * NB * 36);
+    const f2 step2 = pack2(step, step), m1 = pack2(-1.0f, -1.0f), bias = pack2(-8388736.0f, -8388736.0f);
+    const float4 o = ub[l];
+    const f2 u0 = pack2(o.x, o.x), n0 = pack2(-o.x, -o.x), v0 = pack2(o.z, o.z);
+    const f2 u1 = pack2(o.y, o.y), n1 = pack2(-o.y, -o.y), v1 = pack2(o.w, o.w);
+    const int next = l + 1 == NB ? 0 : l + 1, home = l < D1 - 1 ? l - (D1 - 1) + NB : l - (D1 - 1);
+    auto pass = [](f2 x, int src) {
+        const float2 y = unpack2(x);
+        return pack2(__shfl_sync(0xffffffffu, y.x, src), __shfl_sync(0xffffffffu, y.y, src));
+    };
+    f2 w0h = 0, w0l = 0, w1h = 0, w1l = 0, th = 0, tl = 0;
+#pragma unroll
+    for (int d = D0; d < D1; d++) {
+        const float4 a = kp[d * NB], b = kp[d * NB + ND * NB], x = xp[d];
+        const f2 k0 = pack2(a.x, a.y), k1 = pack2(a.z, a.w), l0 = pack2(b.x, b.y), l1 = pack2(b.z, b.w);
+        const f2 xh = pack2(x.x, x.y), xl = pack2(x.z, x.w), xn = mul2(xh, m1);
+        split_term2(w0h, w0l, k0, l0, xh, xn, xl);
+        split_term2(w1h, w1l, k1, l1, xh, xn, xl);
+        if (d != 0 && d != ND - 1) {
+            const uint32_t w = dp[d * NB];
+            auto byte = [&](uint32_t i) { return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u | i)); };  // 2^23 + byte
+            const f2 e0 = fma2(add2(pack2(byte(0), byte(1)), bias), step2, l0);
+            const f2 e1 = fma2(add2(pack2(byte(2), byte(3)), bias), step2, l1);
+            split_term2(th, tl, k0, e0, u0, n0, v0);
+            split_term2(th, tl, k1, e1, u1, n1, v1);
+        }
+        if (d != 0) {  // (else still zero)
+            th = pass(th, d + 1 < D1 ? next : home);
+            tl = pass(tl, d + 1 < D1 ? next : home);
+        }
+    }
+    const float2 ah = unpack2(w0h), al = unpack2(w0l), bh = unpack2(w1h), bl = unpack2(w1l);
+    hi = pack2(ah.x, bh.x);
+    lo = pack2(al.x, bl.x);
+    split_combine2(hi, lo, pack2(ah.y, bh.y), pack2(al.y, bl.y));
+    split_combine2(hi, lo, th, tl);
+}
+
 // Synchronises an element group: a one-warp group with __syncwarp, a larger
 // one with its named barrier (ids 1..15).
 __device__ __forceinline__ void group_sync(uint32_t id, uint32_t threads) {
@@ -1058,6 +1162,17 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
     Acc* pbuf0 = pbase + (size_t)(grp * 2) * pstride;
     auto ubuf = [&](uint32_t p) { return reinterpret_cast<UT*>(ubuf0 + (size_t)p * ub); };
     auto pbuf = [&](uint32_t p) { return pbuf0 + (size_t)p * pstride; };
+    // row r's staged u; blocks: (u_2i, u_2i+1) hi, then lo, twice in a row like every symmetric unit's u
+    auto put_u = [&](uint32_t p, UT x) {
+        if constexpr (kBlocks<A>) {
+            float* f = reinterpret_cast<float*>(ubuf(p)) + (r >> 1) * 4 + (r & 1);
+            f[0] = f[2 * n] = x.x;
+            f[2] = f[2 * n + 2] = x.y;
+        } else {
+            ubuf(p)[r] = x;
+            if constexpr (A::kSym) ubuf(p)[r + n] = x;
+        }
+    };
 
     const uint64_t keep = l2_evict_last_policy(), stream_pol = l2_evict_first_policy();
     // v written by other CTAs in an earlier colour of a fused launch is read past L1
@@ -1089,11 +1204,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
         uint32_t i = ch * E, inext = chn * E + jn;
         if (gatherer && i < cnt) {
             dof_c = map_at(i);
-            if (rvalid) {
-                const UT x = stage_s<A>(load_u_hint(u, dof_c, a.bc_mode, keep), usk);
-                ubuf(0)[r] = x;
-                if constexpr (A::kSym) ubuf(0)[r + n] = x;
-            }
+            if (rvalid) put_u(0, stage_s<A>(load_u_hint(u, dof_c, a.bc_mode, keep), usk));
             if (inext < cnt) dof_n = map_at(inext);
         }
         if (!FU || col == 0)
@@ -1128,10 +1239,20 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
                     constexpr int NC = NT / NG;
                     static_assert(NT % 2 == 0 && NT % NG == 0 && NT / 2 * PG <= 32, "rows in pairs");
                     const uint32_t l = lane % (NT / 2), h = lane / (NT / 2), cgp = q * PG + h;
+                    f2 hi, lo;
+                    if constexpr (kBlocks<A>)  // (shuffles: every lane)
+                    {
+                        const float4* ub = reinterpret_cast<const float4*>(uu);
+                        if (q == 0) split_block_terms<NT, 0>(hi, lo, ks, ub, lane);
+                        else if (q == 1) split_block_terms<NT, 1>(hi, lo, ks, ub, lane);
+                        else if (q == 2) split_block_terms<NT, 2>(hi, lo, ks, ub, lane);
+                        else split_block_terms<NT, 3>(hi, lo, ks, ub, lane);
+                    }
                     if (h < PG) {
-                        const float* kh = reinterpret_cast<const float*>(ks) + cgp * NC * NT + 2 * l;
-                        f2 hi, lo;
-                        split_pair_terms<NT, NC>(hi, lo, kh, kh + a.plane, uu + cgp * NC);
+                        if constexpr (!kBlocks<A>) {
+                            const float* kh = reinterpret_cast<const float*>(ks) + cgp * NC * NT + 2 * l;
+                            split_pair_terms<NT, NC>(hi, lo, kh, kh + a.plane, uu + cgp * NC);
+                        }
                         const float2 s = unpack2(hi), t = unpack2(lo);
                         *reinterpret_cast<float4*>(pbuf(par) + cgp * n + 2 * l) = make_float4(s.x, t.x, s.y, t.y);
                     }
@@ -1200,11 +1321,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
                 if (lane == 0 && (jc + 1 == E || i + 1 == cnt)) mbar_arrive(&empty[s]);
             }
             if (!PG && !gatherer && rvalid) pbuf(par)[(cg - 1) * n + r] = acc;
-            if (gatherer && rvalid && inext < cnt) {
-                const UT x = stage_s<A>(u_n, usk);
-                ubuf(par ^ 1)[r] = x;
-                if constexpr (A::kSym) ubuf(par ^ 1)[r + n] = x;
-            }
+            if (gatherer && rvalid && inext < cnt) put_u(par ^ 1, stage_s<A>(u_n, usk));
             group_sync(bar_id, bar_threads);
             if (gatherer) {
                 if constexpr (PG != 0) {

@@ -1,7 +1,8 @@
 // Instantiation and dispatch of the matvec kernels for one arithmetic policy
 // (included by the afm_mv_*.cu files, which define ARITH and LAUNCH_FN so that
 // they compile in parallel; BATCH_FN is left undefined where there is no
-// batched product, LAUNCH_FN where the arithmetic runs on patches only).
+// batched product, LAUNCH_FN where the arithmetic runs on patches only,
+// PATCH_FN where it does not run on them).
 #include <algorithm>
 
 #include "afm_batched.cuh"
@@ -16,8 +17,8 @@ namespace {
 // or <= kMaxN (WPE) runs the run-time-n instance (template argument 0).
 template <int NT, bool WPE, bool DUP, bool CH = false, bool VE = false>
 void* kernel_ptr() {
-    if constexpr (ARITH::kSym && (!WPE || DUP)) {
-        return nullptr;  // the symmetric arena has element units for the warp-group kernel only
+    if constexpr (ARITH::kSym && (!WPE || DUP || (kBlocks<ARITH> && (CH || split_block_bytes(NT) == 0)))) {
+        return nullptr;  // the symmetric arena has element units for the warp-group kernel only (blocks: of one size)
     } else if constexpr (WPE) {
         if constexpr (DUP)
             return (void*)afm_wpe_kernel<NT, ARITH, true>;
@@ -253,6 +254,7 @@ cudaError_t BATCH_FN(const Segment& s, const BatchArgs& a, int sm_count, int ct,
 
 #endif  // LAUNCH_FN
 
+#ifdef PATCH_FN
 // ---- patch path (small elements) -----------------------------------------
 
 namespace {
@@ -343,6 +345,7 @@ size_t PATCH_SMEM_FN(const PatchPlanGeom& pg, uint32_t copy_bytes) {
     const PatchLayout L = patch_layout(pg, copy_bytes);
     return L.stages >= 2 ? L.total() : 0;
 }
+#endif  // PATCH_FN
 
 #ifdef LAUNCH_FN
 size_t SMEM_FN(const Segment& s) { return ring_layout(s, s.unit_bytes, s.unit_bytes, false, nullptr).total(); }
@@ -351,7 +354,10 @@ size_t SMEM_FN(const Segment& s) { return ring_layout(s, s.unit_bytes, s.unit_by
 namespace {
 template <int NT, bool CH>
 void* fused_ptr() {
-    return (void*)afm_wpg_fused_kernel<NT, ARITH, CH>;
+    if constexpr (kBlocks<ARITH> && (CH || split_block_bytes(NT) == 0))
+        return nullptr;
+    else
+        return (void*)afm_wpg_fused_kernel<NT, ARITH, CH>;
 }
 void* pick_fused_kernel(uint32_t n, bool chunked) {
     if (chunked) {
@@ -382,12 +388,13 @@ cudaError_t FUSED_FN(const Segment* segs, uint32_t ncol, const SegArgs& a, unsig
     const RingLayout L = ring_layout(segs[0], a.copy_bytes, a.unit_bytes, false, &G, true);
     if (L.stages < 2) return cudaErrorInvalidConfiguration;
     void* fn = pick_fused_kernel(segs[0].n, L.chunk > 1);
+    if (!fn) return cudaErrorInvalidValue;
     ColourTable T{};
     T.ncol = ncol;
     T.gbar = gbar;
     for (uint32_t c = 0; c < ncol; c++) {
         if (segs[c].n != segs[0].n || segs[c].regime != REG_WPE) return cudaErrorInvalidValue;
-        T.ke_off[c] = segs[c].ke_offset;
+        T.ke_off[c] = kBlocks<ARITH> ? segs[c].blk_offset : segs[c].ke_offset;
         T.map_off[c] = segs[c].map_offset;
         T.units[c] = segs[c].units;
     }
@@ -441,17 +448,21 @@ cudaError_t CONFIG_FN() {
                     if (e != cudaSuccess) return e;
                 }
 #endif
+#ifdef PATCH_FN
     for (uint32_t nn : {4u, 8u, 10u, 0u})
         for (uint32_t gg : {2u, 4u, 8u}) {
             cudaError_t e = cudaFuncSetAttribute(pick_patch_kernel(nn, gg),
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemBudget + 1024));
             if (e != cudaSuccess) return e;
         }
+#endif
 #ifdef FUSED_FN
     for (uint32_t nn : {24u, 30u, 60u, 7u})
         for (int ch = 0; ch < 2; ch++) {
-            cudaError_t e = cudaFuncSetAttribute(pick_fused_kernel(nn, ch != 0),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemBudget + 1024));
+            void* f = pick_fused_kernel(nn, ch != 0);
+            if (!f) continue;
+            cudaError_t e =
+                cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemBudget + 1024));
             if (e != cudaSuccess) return e;
         }
 #endif

@@ -79,7 +79,7 @@ double now_s() {
 
 // Device bytes a request holds once admitted: element matrices (8 bytes per
 // entry in every arena but FP32, plus the symmetric inner copy of at most 6
-// bytes per stored pair, and the packed FP64 units of small elements), maps or
+// bytes per stored pair, and the packed FP64 units), maps or
 // patch index blocks, diagonal, the solver's
 // FP64 and FP32 work vectors (and the FP64 inner vectors of formats 3 to 5),
 // b and x; 10% and 1 MB of slack.
@@ -87,7 +87,7 @@ uint64_t estimate_bytes(const afm_operator* op) {
     uint64_t ke = 0;
     for (uint32_t e = 0; e < op->n_elem; e++) {
         const uint64_t n = op->offsets[e + 1] - op->offsets[e];
-        ke += n * n * 8 + 8 * n + 6 * n * (n / 2 + 1) + (n <= afm::kPatchMaxN ? 4 * n * (n + 1) : 0);
+        ke += n * n * 8 + 8 * n + 6 * n * (n / 2 + 1) + (n <= afm::kPatchMaxN ? 4 * n * (n + 1) : afm::split_block_bytes((uint32_t)n));
     }
     const uint64_t vec = (uint64_t)op->n_dofs * (8 * 8 + 7 * 4 + 8 * 8 + 3 * 8);
     return (ke + vec) * 11 / 10 + (1u << 20);
