@@ -217,6 +217,7 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
 struct ArithF64 {
     static constexpr bool kSym = false;
     static constexpr bool kPair = false;  // rows in pairs in the warp-group kernel (wpg_pair_groups)
+    static constexpr bool kPairTerms = false;  // terms in pairs (sym_terms)
     static constexpr bool kScaled = false;  // u scaled by a power of two per launch (stage_s, finish_s)
     static constexpr uint32_t kWpgWarps = 16;  // consumer warps of the warp-group kernel
     using KT = double;
@@ -243,6 +244,7 @@ struct ArithF64 {
 struct ArithSplit {
     static constexpr bool kSym = false;
     static constexpr bool kPair = true;
+    static constexpr bool kPairTerms = false;
     static constexpr bool kScaled = true;
     static constexpr uint32_t kWpgWarps = 16;
     using KT = float2;
@@ -285,6 +287,7 @@ struct ArithSplit {
 struct ArithF32 {
     static constexpr bool kSym = false;
     static constexpr bool kPair = false;
+    static constexpr bool kPairTerms = false;
     static constexpr bool kScaled = false;
     static constexpr uint32_t kWpgWarps = 24;  // more elements in flight: see wpg_gc
     using KT = float;
@@ -327,6 +330,7 @@ struct ArithF32Sym : ArithF32 {
 struct ArithF32SymX {
     static constexpr bool kSym = true;
     static constexpr bool kPair = false;
+    static constexpr bool kPairTerms = true;
     static constexpr bool kScaled = false;
     static constexpr uint32_t kWpgWarps = 24;
     using KT = float2;  // (hi, lo)
@@ -370,6 +374,7 @@ struct ArithF32SymX {
 struct ArithF32SymC {
     static constexpr bool kSym = true;
     static constexpr bool kPair = false;
+    static constexpr bool kPairTerms = false;
     static constexpr bool kScaled = false;
     static constexpr uint32_t kWpgWarps = 24;
     using KT = float2;  // (hi, lo)
@@ -416,6 +421,7 @@ inline constexpr bool kBlocks<ArithSplitBlk> = true;
 struct ArithSplitSymX {
     static constexpr bool kSym = true;
     static constexpr bool kPair = false;
+    static constexpr bool kPairTerms = true;
     static constexpr bool kScaled = true;
     static constexpr uint32_t kWpgWarps = 16;
     using KT = float2;  // (hi, lo)
@@ -843,6 +849,35 @@ __host__ __device__ constexpr uint32_t wpg_gc(uint32_t gr, uint32_t ut_bytes) {
     return gr == 2 && ut_bytes == 8 ? 2u : 1u;
 }
 
+// One product term of ArithSplit::fma for two floats at once: (hi, lo) += (k + kl)(u + ul), nu = -u. Each difference is
+// a multiply-add by -1 (exact products: the same roundings).
+template <bool UL = true>
+__device__ __forceinline__ void split_term2(f2& hi, f2& lo, f2 k, f2 kl, f2 u, f2 nu, f2 ul) {
+    const f2 m1 = pack2(-1.0f, -1.0f);
+    const f2 np = mul2(k, nu);  // -p
+    f2 t = fma2(kl, u, fma2(k, u, np));
+    if constexpr (UL) t = fma2(k, ul, t);
+    const f2 s = fma2(np, m1, hi);
+    const f2 bp = fma2(hi, m1, s);
+    const f2 err = fma2(add2(np, bp), m1, fma2(fma2(bp, m1, s), m1, hi));
+    hi = s;
+    lo = add2(lo, add2(err, t));
+}
+// ... with u a single float (ArithF32SymX::fma).
+__device__ __forceinline__ void split_term2(f2& hi, f2& lo, f2 k, f2 kl, f2 u, f2 nu) {
+    split_term2<false>(hi, lo, k, kl, u, nu, 0);
+}
+
+// ArithSplit::combine for two sums at once.
+__device__ __forceinline__ void split_combine2(f2& hi, f2& lo, f2 bhi, f2 blo) {
+    const f2 m1 = pack2(-1.0f, -1.0f);
+    const f2 s = add2(hi, bhi);
+    const f2 bp = fma2(hi, m1, s);
+    const f2 err = add2(fma2(fma2(bp, m1, s), m1, hi), fma2(bp, m1, bhi));
+    hi = s;
+    lo = add2(lo, add2(blo, err));
+}
+
 // Terms [T0, T1) of row r of a symmetric element in the wrapped-diagonal
 // layout (D[d][j] = K(j, (j + d) mod n) at d n + j): term t <= n/2 is
 // D[t][r] u[r + t], term t > n/2 (d = t - n/2) is K(r, r - d) =
@@ -850,18 +885,42 @@ __host__ __device__ constexpr uint32_t wpg_gc(uint32_t gr, uint32_t ut_bytes) {
 // where u is staged twice in a row (u[j + n] = u[j]) so that no u index
 // wraps. Every offset is a compile-time constant but the wrap of the
 // transposed read (one select).
+// The double-float arithmetics take the terms in pairs, one sum for the even and one for the odd ones, on packed
+// instructions: these products are bound by issued instructions, and a term's arithmetic is most of them (one by one, then in
+// pairs: inner product of format 4 on hex20 elasticity 32^3 92 -> 87 us, hex8 elasticity 48^3 80 -> 74.5, tet10 elasticity
+// 20^3 x 6 58 -> 50).
 template <typename A, int NT, int T0, int T1>
 __device__ __forceinline__ void sym_terms(typename A::Acc& acc, const unsigned char* ks, uint32_t plane,
                                           const typename A::UT* ur, uint32_t r) {
     constexpr int H = NT / 2;
+    auto entry = [&](int t) {
+        const int d = t - H;
+        return t <= H ? r + t * NT : r + d * NT - d + ((int)r < d ? NT : 0);
+    };
+    auto at = [&](int t) { return ur[t <= H ? t : NT - (t - H)]; };
+    if constexpr (A::kPairTerms) {
+        static_assert((T1 - T0) % 2 == 0, "terms in pairs");
+        const f2 m1 = pack2(-1.0f, -1.0f);
+        f2 hi = 0, lo = 0;
 #pragma unroll
-    for (int t = T0; t < T1; t++) {
-        if (t <= H) {
-            A::fma(acc, A::kload(ks, r + t * NT, plane), ur[t]);
-        } else {
-            const int d = t - H;
-            A::fma(acc, A::kload(ks, r + d * NT - d + ((int)r < d ? NT : 0), plane), ur[NT - d]);
+        for (int t = T0; t < T1; t += 2) {
+            const float2 a = A::kload(ks, entry(t), plane), b = A::kload(ks, entry(t + 1), plane);
+            const typename A::UT x = at(t), y = at(t + 1);
+            const f2 k = pack2(a.x, b.x), kl = pack2(a.y, b.y);
+            if constexpr (sizeof(typename A::UT) == 8) {
+                const f2 u = pack2(x.x, y.x);
+                split_term2(hi, lo, k, kl, u, mul2(u, m1), pack2(x.y, y.y));
+            } else {
+                const f2 u = pack2(x, y);
+                split_term2(hi, lo, k, kl, u, mul2(u, m1));
+            }
         }
+        const float2 h = unpack2(hi), l = unpack2(lo);
+        acc = {h.x, l.x};
+        A::combine(acc, {h.y, l.y});
+    } else {
+#pragma unroll
+        for (int t = T0; t < T1; t++) A::fma(acc, A::kload(ks, entry(t), plane), at(t));
     }
 }
 
@@ -899,29 +958,6 @@ __device__ __forceinline__ void split_pair_terms(f2& hi, f2& lo, const float* kh
         hi = s;
         lo = add2(lo, fma2(nt, m1, err));
     }
-}
-
-// One product term of ArithSplit::fma for two floats at once: (hi, lo) += (k + kl)(u + ul), nu = -u. Each difference is
-// a multiply-add by -1 (exact products: the same roundings).
-__device__ __forceinline__ void split_term2(f2& hi, f2& lo, f2 k, f2 kl, f2 u, f2 nu, f2 ul) {
-    const f2 m1 = pack2(-1.0f, -1.0f);
-    const f2 np = mul2(k, nu);  // -p
-    const f2 t = fma2(k, ul, fma2(kl, u, fma2(k, u, np)));
-    const f2 s = fma2(np, m1, hi);
-    const f2 bp = fma2(hi, m1, s);
-    const f2 err = fma2(add2(np, bp), m1, fma2(fma2(bp, m1, s), m1, hi));
-    hi = s;
-    lo = add2(lo, add2(err, t));
-}
-
-// ArithSplit::combine for two sums at once.
-__device__ __forceinline__ void split_combine2(f2& hi, f2& lo, f2 bhi, f2 blo) {
-    const f2 m1 = pack2(-1.0f, -1.0f);
-    const f2 s = add2(hi, bhi);
-    const f2 bp = fma2(hi, m1, s);
-    const f2 err = add2(fma2(fma2(bp, m1, s), m1, hi), fma2(bp, m1, bhi));
-    hi = s;
-    lo = add2(lo, add2(blo, err));
 }
 
 // Block units (ArithSplitBlk; elements of 60 DoFs whose Ke is symmetric to 2^-46 of its smallest diagonal entry): NB =
