@@ -684,7 +684,9 @@ void build_segments(afm_operator* op, int prec) {
 // 248. FP32 products and inner formats, whose element launches are shorter:
 // hex20 42^3 FP32 122 -> 98 us, format 4 225 -> 195 (0.56 M), 56^3 232 -> 236 and
 // 462 -> 458 (1.3 M); hex8 elasticity 72^3 159 -> 126 us (1.1 M), 90^3 258 -> 242
-// (2.2 M); tet10 elasticity 44^3 x 6 FP32 339 -> 242.
+// (2.2 M); tet10 elasticity 44^3 x 6 FP32 339 -> 242. The split products on block
+// units go with these: hex20 30^3 109 -> 90 us, 42^3 238 -> 227 (0.56 M), 54^3 477 ->
+// 470 (1.2 M).
 bool gather_pays(const afm_operator* op, bool wide, uint32_t ve_bytes) {
     const uint64_t entries = (uint64_t)op->n_elem * op->nmax;
     const uint64_t most = op->nmax > 32 ? (wide ? 200000u : 1200000u) : (wide ? 900000u : 2200000u);
@@ -1054,7 +1056,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     const bool fused = op->fused && op->fused_ok && kprec == AFM_PREC_FP64_SPLIT && !sym && !f32;
     const int ve_bytes = (f32 || kprec == AFM_PREC_FP32) && !symx ? 4 : 8;
     if (!fused)
-        if (int s = gather_ready(op, scaled || kprec == AFM_PREC_FP64, ve_bytes, st, &gather)) return s;
+        if (int s = gather_ready(op, (scaled || kprec == AFM_PREC_FP64) && !blocks, ve_bytes, st, &gather)) return s;
     if (gather) {
         if (scaled)
             AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs, nullptr,
@@ -3456,7 +3458,7 @@ int afm_get_info(afm_operator* op, afm_info* info) {
     } else if (op->use_patches) {
         launches += op->patch_one_launch ? 1u + (op->n_shared ? 1u : 0u) : (uint32_t)op->patch_color_first.size() - 1;
     } else {
-        if (op->gather_b && gather_pays(op, op->precision != AFM_PREC_FP32, op->precision == AFM_PREC_FP32 ? 4 : 8) && !(op->fused && op->fused_ok))
+        if (op->gather_b && gather_pays(op, op->precision != AFM_PREC_FP32 && !op->d_packed, op->precision == AFM_PREC_FP32 ? 4 : 8) && !(op->fused && op->fused_ok))
             launches += 2;  // one launch for every element and the gather pass
         else
             for (const Segment& s : op->segs)

@@ -975,7 +975,8 @@ __device__ __forceinline__ void split_pair_terms(f2& hi, f2& lo, const float* kh
 // diagonals [block_run(q), block_run(q + 1)): 3, 3, 5 and 5, as the first two also gather u and scatter v, and the others
 // would wait for them at the element's barrier (42^3: 2, 2, 6 and 6 261 us, 4 each 278, this 248, with 20 warps).
 // What bounds it now is the double-float arithmetic and its latencies (0.4 to 0.6 instructions issued per cycle), so the
-// gain is below the bytes': hex20 elasticity 42^3 306 -> 239 us a product (5.4 TB/s), 56^3 715 -> 534, 14^3 20.2 -> 19.4. In
+// gain is below the bytes': hex20 elasticity 42^3 306 -> 239 us a product (5.4 TB/s; 227 in one launch with
+// the gather pass), 56^3 715 -> 534, 14^3 20.2 -> 19.4. In
 // elements of 24 and 30 DoFs (two runs of diagonals per warp) the overhead per element outweighs it: hex8 elasticity
 // 48^3 92 -> 97 us, tet10 elasticity 32^3 x 6 240 -> 241.
 template <int NT>
