@@ -149,8 +149,9 @@ int afm_set_element_kind(afm_operator* op, int kind, double E, double nu, uint32
  * into xe, e.g. examples/src/example07a.cpp:54-71). With
  * afm_set_matfree_type(op, 2) (MATFREE_TYPE::FREE, include/aMatFree.hpp:
  * 2241-2745) every product integrates each element's stiffness from these
- * coordinates on the device instead of reading stored Ke: one warp per
- * element, one launch per colour, FP64 for afm_matvec(_device), FP32 for the
+ * coordinates on the device instead of reading stored Ke: 8 to 32 lanes per
+ * element, one launch and a gather pass or one launch per colour, FP64 for
+ * afm_matvec(_device), FP32 for the
  * _f32 products and the inner CG of afm_solve_cg_mixed; the Jacobi diagonal
  * and trace come from the same kernels on the host at afm_finalize. */
 int afm_set_element_coords(afm_operator* op, uint32_t first, uint32_t count, const double* xe);
@@ -201,9 +202,10 @@ int afm_set_symmetric_inner(afm_operator* op, int format);
  * (warp-group regime, up to 48 colours) runs every colour in one cooperative
  * launch, a grid barrier between colours, outside stream capture (captured
  * solve iterations keep one launch per colour); same results bit for bit.
- * 0 (default): one launch per colour, which measured faster (hex20 elasticity
- * 64^3: 1.359 against 1.438 ms; the grid barriers cost more than the launch
- * boundaries they replace). */
+ * 0 (default): one launch per colour, or one launch for every element and a
+ * pass that sums the element products, which measured faster (hex20 elasticity
+ * 64^3 with whole matrices: 1.359 against 1.438 ms; the grid barriers cost more
+ * than the launch boundaries they replace). */
 int afm_set_fused_colours(afm_operator* op, int enable);
 /* Limit of each wait inside the operator's element kernels (no counterpart
  * in the reference, which ends the process on a device error:
