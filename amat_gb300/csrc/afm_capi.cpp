@@ -239,6 +239,24 @@ void dfree(afm_operator* op, T*& p) {
     p = nullptr;
 }
 
+// The packed arena of FP64 products (bytes), where the device has room for it beside what the operator may allocate
+// later (inner arenas, vectors, batched and assembled forms): as much again as the element matrices take and 512 bytes
+// per DoF must stay free, so that nothing that fits without the packed arena fails with it. Small ones are not worth the
+// question. False: there is none, and the products read the whole matrices.
+bool alloc_packed(afm_operator* op, uint64_t bytes) {
+    if (bytes > (256ull << 20)) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < bytes + op->ke_bytes + 512ull * op->n_dofs) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    if (dalloc(op, &op->d_packed, std::max<uint64_t>(bytes, 16)) == cudaSuccess) return true;
+    cudaGetLastError();
+    op->d_packed = nullptr;
+    return false;
+}
+
 void drop_graph(afm_operator::CgGraph& g);
 
 void free_device(afm_operator* op) {
@@ -732,7 +750,11 @@ int build_gather(afm_operator* op, uint32_t n, const std::vector<uint32_t>& colo
     }
     // one allocation: the products, then the lists and their offsets
     const size_t ve_bytes = ((gather_pays(op, false, 8) ? 8 : 4) * entries + 15) / 16 * 16;
-    AFM_CUDA(dalloc(op, &op->d_ve, ve_bytes + sizeof(uint32_t) * (idx.size() + off.size())));
+    if (dalloc(op, &op->d_ve, ve_bytes + sizeof(uint32_t) * (idx.size() + off.size())) != cudaSuccess) {
+        cudaGetLastError();  // no room: colour launches
+        op->d_ve = nullptr;
+        return AFM_SUCCESS;
+    }
     op->d_gather_idx = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(op->d_ve) + ve_bytes);
     op->d_gather_off = op->d_gather_idx + idx.size();
     AFM_CUDA(cudaMemcpyAsync(op->d_gather_off, off.data(), sizeof(uint32_t) * off.size(), cudaMemcpyHostToDevice,
@@ -2735,13 +2757,8 @@ int afm_finalize(afm_operator* op) {
         op->sym_ok = op->ke_symmetric && covered;
         if (op->use_patches && op->ke_sym_exact) {
             const Segment& s = op->segs[0];
-            const size_t bytes = (size_t)s.units * s.n * (s.n + 1) * kTpeWidth * 4;
-            if (dalloc(op, &op->d_packed, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-                cudaGetLastError();  // no room: FP64 products read the whole matrices
-                op->d_packed = nullptr;
-            } else {
+            if (alloc_packed(op, (uint64_t)s.units * s.n * (s.n + 1) * kTpeWidth * 4))
                 AFM_CUDA(pack_split_units(op->d_ke, s.n, s.units, op->d_packed, op->sm_count, op->stream));
-            }
         }
         if (!op->use_patches && op->ke_sym_near && op->n_elem >= kBlockElemsPerSm * (uint64_t)std::max(op->sm_count, 1)) {
             uint64_t bytes = 0;
@@ -2751,10 +2768,7 @@ int afm_finalize(afm_operator* op) {
                 s.blk_offset = bytes;
                 bytes += (uint64_t)split_block_bytes(s.n) * s.units;
             }
-            if (covered && dalloc(op, &op->d_packed, std::max<uint64_t>(bytes, 16)) != cudaSuccess) {
-                cudaGetLastError();  // no room: as above
-                op->d_packed = nullptr;
-            } else if (covered) {
+            if (covered && alloc_packed(op, bytes)) {
                 for (const Segment& s : op->segs)
                     AFM_CUDA(pack_split_blocks(op->d_ke + s.ke_offset, s.unit_bytes, s.plane, s.n, s.units,
                                                op->d_packed + s.blk_offset, op->sm_count, op->stream));
