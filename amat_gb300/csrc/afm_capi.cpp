@@ -760,7 +760,7 @@ int build_gather(afm_operator* op, uint32_t n, const std::vector<uint32_t>& colo
     AFM_CUDA(cudaMemcpyAsync(op->d_gather_off, off.data(), sizeof(uint32_t) * off.size(), cudaMemcpyHostToDevice,
                              op->stream));
     AFM_CUDA(cudaMemcpyAsync(op->d_gather_idx, idx.data(), sizeof(uint32_t) * idx.size(), cudaMemcpyHostToDevice,
-                             op->stream));  // (pageable memory: staged before the call returns)
+                             op->stream));  // (pageable memory: read before the call returns; finalize waits for the copies)
     op->gather_b = b;
     return AFM_SUCCESS;
 }
@@ -2507,6 +2507,7 @@ int finalize_free(afm_operator* op) {
     AFM_CUDA(cudaStreamSynchronize(st));
     if (!op->dup_in_element)
         if (int s = build_gather(op, n, op->free_color_first)) return s;
+    AFM_CUDA(cudaStreamSynchronize(st));  // products may run on other streams
     op->ke_dirty = false;
     op->finalized = true;
     return ok();
@@ -2775,7 +2776,8 @@ int afm_finalize(afm_operator* op) {
             }
         }
     }
-    if (op->d_packed) AFM_CUDA(cudaStreamSynchronize(op->stream));  // products may run on other streams
+    // products may run on other streams: the gather lists, packed units and stream-ordered allocations are there
+    AFM_CUDA(cudaStreamSynchronize(op->stream));
     op->ke_dirty = false;
     op->finalized = true;
     return ok();
