@@ -259,7 +259,15 @@ bool alloc_packed(afm_operator* op, uint64_t bytes) {
 
 void drop_graph(afm_operator::CgGraph& g);
 
+// Orders the operator's stream after its last product (take_turn), before device memory that a product on a caller's
+// stream may still use is freed or written there.
+void own_turn(afm_operator* op) {
+    if (op->turn_id) cudaStreamWaitEvent(op->stream, op->turn_event, 0);
+    op->turn_id = 0;
+}
+
 void free_device(afm_operator* op) {
+    own_turn(op);
     drop_graph(op->cg64);
     drop_graph(op->cg32);
     drop_graph(op->cg64i);
@@ -287,7 +295,6 @@ void free_device(afm_operator* op) {
     dfree(op, op->d_gbar);
     dfree(op, op->d_ve);  // (and the gather lists)
     op->gather_b = 0;
-    op->ve_stream = nullptr;
     op->fused_ok = false;
     dfree(op, op->d_work);
     dfree(op, op->d_work32);
@@ -765,42 +772,43 @@ int build_gather(afm_operator* op, uint32_t n, const std::vector<uint32_t>& colo
     return AFM_SUCCESS;
 }
 
-// Whether a product enqueued on st may use the element-product (or batched combine) buffer, which
-// the operator's products share. A product on another stream than the one
-// before waits for that one's end; inside a caller's own capture, whose graph
-// may be replayed beside other products, the colour launches (no shared
-// buffer) run instead.
-int buffer_ready(afm_operator* op, cudaStream_t st, bool* use) {
-    *use = false;
+// An operator's products share its device memory beside Ke and the maps (element products, combine buffers, u scales,
+// the staging vectors of the inner formats), so they run in turn, whichever streams they are enqueued on: a product
+// waits for the one before if that ran on another stream, and a solve, whose iterations are captured once and replayed,
+// takes its turn with the product that it starts with. *captured: st records a caller's graph, which may be replayed
+// beside other products and can wait for nothing outside: the launches per colour, with u scales of their own, run then.
+// Streams are told apart by their ids: a new stream may have the handle of one that is gone, and one handle
+// (cudaStreamPerThread) stands for several.
+int take_turn(afm_operator* op, cudaStream_t st, bool* captured) {
+    *captured = false;
+    // (patch products take the same launches in a capture; the question costs the smallest of them 2%)
+    if (st == op->stream && (op->own_capture || (op->use_patches && !op->turn_id))) return AFM_SUCCESS;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     AFM_CUDA(cudaStreamIsCapturing(st, &cap));
-    const bool own = op->own_capture && st == op->stream;  // after a product of the same solve on this stream
-    if (cap != cudaStreamCaptureStatusNone && !own) return AFM_SUCCESS;
-    if (st != op->ve_stream && op->ve_stream && !own) {
-        if (op->ve_stream == op->stream) {
-            // (a caller's stream may be gone by now: its event was recorded after its product)
-            if (!op->ve_event) AFM_CUDA(cudaEventCreateWithFlags(&op->ve_event, cudaEventDisableTiming));
-            AFM_CUDA(cudaStreamIsCapturing(op->stream, &cap));
-            if (cap != cudaStreamCaptureStatusNone) return AFM_SUCCESS;
-            AFM_CUDA(cudaEventRecord(op->ve_event, op->stream));
-        }
-        AFM_CUDA(cudaStreamWaitEvent(st, op->ve_event, 0));
+    *captured = cap != cudaStreamCaptureStatusNone;
+    if (*captured) return AFM_SUCCESS;
+    if (st == op->stream) {
+        own_turn(op);
+        return AFM_SUCCESS;
     }
-    op->ve_stream = st;
-    *use = true;
+    unsigned long long id = 0;
+    AFM_CUDA(cudaStreamGetId(st, &id));
+    if (op->turn_id == id + 1) return AFM_SUCCESS;
+    if (!op->turn_event) AFM_CUDA(cudaEventCreateWithFlags(&op->turn_event, cudaEventDisableTiming));
+    if (!op->turn_id) {  // (a caller's stream may be gone by now: its event was recorded after its product)
+        AFM_CUDA(cudaStreamIsCapturing(op->stream, &cap));
+        *captured = cap != cudaStreamCaptureStatusNone;
+        if (*captured) return AFM_SUCCESS;
+        AFM_CUDA(cudaEventRecord(op->turn_event, op->stream));
+    }
+    AFM_CUDA(cudaStreamWaitEvent(st, op->turn_event, 0));
+    op->turn_id = id + 1;
     return AFM_SUCCESS;
 }
 
-int gather_ready(afm_operator* op, bool wide, uint32_t ve_bytes, cudaStream_t st, bool* use) {
-    *use = false;
-    if (!op->gather_b || !gather_pays(op, wide, ve_bytes)) return AFM_SUCCESS;
-    return buffer_ready(op, st, use);
-}
-
-int buffer_done(afm_operator* op, cudaStream_t st) {
-    if (st == op->stream) return AFM_SUCCESS;
-    if (!op->ve_event) AFM_CUDA(cudaEventCreateWithFlags(&op->ve_event, cudaEventDisableTiming));
-    AFM_CUDA(cudaEventRecord(op->ve_event, st));
+// After the product's last launch.
+int end_turn(afm_operator* op, cudaStream_t st, bool captured) {
+    if (st != op->stream && !captured) AFM_CUDA(cudaEventRecord(op->turn_event, st));
     return AFM_SUCCESS;
 }
 
@@ -875,6 +883,7 @@ int ensure_sym(afm_operator* op, cudaStream_t st) {
     const int fmt = sym_arena(op);
     if (!fmt) return AFM_SUCCESS;
     if (op->d_sym && op->sym_built == fmt) return AFM_SUCCESS;
+    own_turn(op);
     dfree(op, op->d_sym);
     dfree(op, op->d_vx);
     op->sym_built = 0;
@@ -968,6 +977,7 @@ int ensure_work(afm_operator* op, size_t vectors) {
 int ensure_work64i(afm_operator* op, size_t vectors) {
     const size_t need = vectors * (size_t)std::max<uint32_t>(op->n_dofs, 1);
     if (op->work64i_elems >= need) return AFM_SUCCESS;
+    own_turn(op);
     dfree(op, op->d_work64i);
     op->work64i_elems = 0;
     AFM_CUDA(dalloc(op, &op->d_work64i, need * sizeof(double)));
@@ -1006,7 +1016,7 @@ struct ProductTail {
 
 // Matrix-free product (method 2): one launch and the gather pass, or one launch per colour.
 int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32,
-                 ProductTail* tail) {
+                 ProductTail* tail, bool captured) {
     const double E = op->elem_E, nu = op->elem_nu;
     FreeArgs a;
     a.xe = f32 ? (const void*)op->d_free_xe32 : (const void*)op->d_free_xe64;
@@ -1018,10 +1028,8 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
     a.bc_mode = bc_mode;
     a.lam = E * nu / (1.0 + nu) / (1.0 - 2.0 * nu);
     a.mu = 0.5 * E / (1.0 + nu);
-    bool gather = false;
     const int vb = f32 ? 4 : 8;
-    if (int s = gather_ready(op, false, vb, st, &gather)) return s;
-    if (gather) {
+    if (!captured && op->gather_b && gather_pays(op, false, vb)) {
         a.ve = op->d_ve;
         a.first = 0;
         a.count = op->n_elem;
@@ -1030,7 +1038,7 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
         AFM_CUDA(launch_gather_sum(vb, vb, op->gather_b, d_v, op->d_ve, op->d_gather_off, op->d_gather_idx, op->n_dofs,
                                    d_u, tail ? op->d_bcmask : nullptr, part, tail ? &tail->nb : nullptr, st));
         if (tail) tail->bc_done = true;
-        return buffer_done(op, st);
+        return AFM_SUCCESS;
     }
     AFM_CUDA(cudaMemsetAsync(d_v, 0, (size_t)op->n_dofs * vb, st));
     for (size_t c = 0; c + 1 < op->free_color_first.size(); c++) {
@@ -1041,12 +1049,10 @@ int enqueue_free(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cuda
     return AFM_SUCCESS;
 }
 
-// v = K u (bc_mode 0) or the product of MatMult_mf without the final v_c = u_c
-// (bc_mode 1: constrained columns of u read as zero), device arrays.
-// tail: MatMult_mf callers (bc_mode 1).
-int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32 = false,
-                   bool inner64 = false, ProductTail* tail = nullptr) {
-    if (op->matfree_type == 2) return enqueue_free(op, d_v, d_u, bc_mode, st, f32, tail);
+// The launches of enqueue_matvec, whose turn it is (take_turn).
+int enqueue_launches(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32, bool inner64,
+                     ProductTail* tail, bool captured) {
+    if (op->matfree_type == 2) return enqueue_free(op, d_v, d_u, bc_mode, st, f32, tail, captured);
     const void* const d_u_in = d_u;
     // f32: FP32 product on float vectors, from the symmetric inner arena once
     // built, else from an FP32 arena or the hi plane of a split arena (half of
@@ -1074,15 +1080,14 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     const bool scaled = kprec == AFM_PREC_FP64_SPLIT || kprec == kPrecSplitSymX;
     const bool blocks = kprec == AFM_PREC_FP64_SPLIT && !op->use_patches && op->d_packed;
     // one launch for every element plus the gather pass, which writes every entry of v
-    bool gather = false;
     const bool fused = op->fused && op->fused_ok && kprec == AFM_PREC_FP64_SPLIT && !sym && !f32;
     const int ve_bytes = (f32 || kprec == AFM_PREC_FP32) && !symx ? 4 : 8;
-    if (!fused)
-        if (int s = gather_ready(op, (scaled || kprec == AFM_PREC_FP64) && !blocks, ve_bytes, st, &gather)) return s;
-    if (gather) {
+    unsigned long long* const usc = op->d_usc + (captured ? kUscWords : 0);
+    if (!fused && !captured && op->gather_b &&
+        gather_pays(op, (scaled || kprec == AFM_PREC_FP64) && !blocks, ve_bytes)) {
         if (scaled)
             AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs, nullptr,
-                                 0, op->d_usc, op->own_capture && !inner_f32u, st));
+                                 0, usc, op->own_capture && !inner_f32u, st));
         Segment s = op->segs[0];
         s.count = s.units = op->n_elem;
         SegArgs a;
@@ -1102,7 +1107,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         }
         a.bc_mode = bc_mode;
         a.err = op->d_err;
-        a.umax = op->d_usc;
+        a.umax = usc;
         a.wait_ns = op->wait_ns;
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
         AFM_CUDA(launch_segment(s, blocks ? kPrecSplitBlk : kprec, a, op->sm_count, false, false, st));
@@ -1112,7 +1117,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
                                    op->d_gather_off, op->d_gather_idx, op->n_dofs, d_u_in,
                                    tail ? op->d_bcmask : nullptr, part, tail ? &tail->nb : nullptr, st));
         if (tail) tail->bc_done = true;
-        return buffer_done(op, st);
+        return AFM_SUCCESS;
     }
     // one launch over every patch and its combine pass write every DoF that an element lists; else v = 0, and
     // for a segment plan max|u| for the launches' power-of-two u scale, in one launch before the first element
@@ -1120,7 +1125,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     const bool one_patch = op->use_patches && op->patch_one_launch;
     if (scaled && !op->use_patches)
         AFM_CUDA(launch_umax(static_cast<const double*>(d_u), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
-                             static_cast<double*>(d_v), op->n_dofs, op->d_usc, false, st));
+                             static_cast<double*>(d_v), op->n_dofs, usc, false, st));
     else if (!one_patch || op->n_unlisted)
         AFM_CUDA(cudaMemsetAsync(d_v, 0, via_vx ? (size_t)op->n_dofs * 8 : vbytes, st));
     bool first = true;
@@ -1176,8 +1181,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     }
     // split products of a plan with one element size: every colour in one cooperative launch (outside
     // stream capture: captured solve iterations keep the colour launches)
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (fused && cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    if (fused && !captured && !op->own_capture) {
         const Segment& s0 = op->segs[0];
         SegArgs a;
         a.ke = op->d_ke;
@@ -1191,7 +1195,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         a.plane = s0.plane;
         a.bc_mode = bc_mode;
         a.err = op->d_err;
-        a.umax = op->d_usc;
+        a.umax = usc;
         a.wait_ns = op->wait_ns;
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
         AFM_CUDA(cudaMemsetAsync(op->d_gbar, 0, sizeof(unsigned) * op->segs.size(), st));
@@ -1221,7 +1225,7 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
         }
         a.bc_mode = bc_mode;
         a.err = op->d_err;
-        a.umax = op->d_usc;
+        a.umax = usc;
         a.wait_ns = op->wait_ns;
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
         // every launch after the first may overlap its prologue with the previous one's tail
@@ -1230,6 +1234,18 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
     }
     if (via_vx) AFM_CUDA(launch_to_f32(d_v32, op->d_vx, op->n_dofs, st));
     return AFM_SUCCESS;
+}
+
+// v = K u (bc_mode 0) or the product of MatMult_mf without the final v_c = u_c
+// (bc_mode 1: constrained columns of u read as zero), device arrays.
+// tail: MatMult_mf callers (bc_mode 1).
+int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cudaStream_t st, bool f32 = false,
+                   bool inner64 = false, ProductTail* tail = nullptr) {
+    bool captured = false;
+    if (int s = take_turn(op, st, &captured)) return s;
+    const int s = enqueue_launches(op, d_v, d_u, bc_mode, st, f32, inner64, tail, captured);
+    const int e = end_turn(op, st, captured);
+    return s ? s : e;
 }
 
 // MatMult_mf: the product with constrained columns read as zero, then v_c = u_c.
@@ -1297,9 +1313,7 @@ int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, cudaStream_t st, bo
     if (!bpatch_supported(op->bp_n, f32)) return AFM_SUCCESS;
     const size_t bytes = std::max<size_t>((size_t)op->bp_pv_rows * nrhs * (f32 ? 4 : 8), 16);
     if (op->bp_pv_bytes < bytes) {
-        // products on other streams may still read the old buffer
-        if (op->ve_stream && op->ve_stream != op->stream && op->ve_event)
-            AFM_CUDA(cudaStreamWaitEvent(op->stream, op->ve_event, 0));
+        own_turn(op);
         dfree(op, op->d_bp_pv);
         op->bp_pv_bytes = 0;
         if (cudaMallocAsync((void**)&op->d_bp_pv, bytes, op->stream) != cudaSuccess) {
@@ -1315,19 +1329,18 @@ int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, cudaStream_t st, bo
     return AFM_SUCCESS;
 }
 
-// tr = kPatchTile: the patch plan (ensure_bpatch), in the arithmetic it was made usable for.
-int enqueue_matvec_batched(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, uint32_t ld, int bc_mode,
-                           cudaStream_t st, bool f32, int tr, int ng) {
+// The launches of enqueue_matvec_batched, whose turn it is (take_turn).
+int enqueue_launches_batched(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, uint32_t ld, int bc_mode,
+                             cudaStream_t st, bool f32, int tr, int ng, bool captured) {
     const int kprec = f32 ? AFM_PREC_FP32 : op->precision;
     const size_t vb = (kprec == AFM_PREC_FP32 ? 4 : 8);
+    unsigned long long* const cols = op->d_usc + (captured ? kUscWords : 0) + kUscColsOffset;
     if (tr == kPatchTile) {
-        bool use = false;
-        if (int s = buffer_ready(op, st, &use)) return s;
-        if (use) {
+        if (!captured) {
             if (op->n_unlisted) AFM_CUDA(cudaMemsetAsync(d_V, 0, (size_t)op->n_dofs * ld * vb, st));
             if (!f32)
                 AFM_CUDA(launch_umax_cols(static_cast<const double*>(d_U), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
-                                          nrhs, ld, op->d_usc + kUscColsOffset, st));
+                                          nrhs, ld, cols, st));
             BPatchGeom g;
             g.n = op->bp_n;
             g.patches = op->bp_patches;
@@ -1346,9 +1359,9 @@ int enqueue_matvec_batched(afm_operator* op, void* d_V, const void* d_U, uint32_
             a.nrhs = nrhs;
             a.ld = ld;
             a.bc_mode = bc_mode;
-            a.umax = op->d_usc + kUscColsOffset;
+            a.umax = cols;
             AFM_CUDA(launch_bpatch(g, a, f32, op->d_bp_dof, op->d_bp_off, op->d_bp_idx, op->sm_count, st));
-            return buffer_done(op, st);
+            return AFM_SUCCESS;
         }
         // a caller's capture: the launches per colour, with the tile tuned for them
         tr = nrhs % 8 == 0 ? 8 : 4;
@@ -1358,7 +1371,7 @@ int enqueue_matvec_batched(afm_operator* op, void* d_V, const void* d_U, uint32_
     // split arithmetic: max|U(:, j)| of every column for the per-column u scale
     if (kprec == AFM_PREC_FP64_SPLIT)
         AFM_CUDA(launch_umax_cols(static_cast<const double*>(d_U), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
-                                  nrhs, ld, op->d_usc + kUscColsOffset, st));
+                                  nrhs, ld, cols, st));
     bool first = true;
     for (const Segment& s : op->segs) {
         if (s.units == 0) continue;
@@ -1378,7 +1391,7 @@ int enqueue_matvec_batched(afm_operator* op, void* d_V, const void* d_U, uint32_
         a.bc_mode = bc_mode;
         a.err = op->d_err;
         a.n_dofs = op->n_dofs;
-        a.umax = op->d_usc + kUscColsOffset;
+        a.umax = cols;
         a.wait_ns = op->wait_ns;
         a.probe = op->wait_probe ? op->d_err + (kErrWords - 1) : nullptr;
         cudaError_t e;
@@ -1395,6 +1408,16 @@ int enqueue_matvec_batched(afm_operator* op, void* d_V, const void* d_U, uint32_
         first = false;
     }
     return AFM_SUCCESS;
+}
+
+// tr = kPatchTile: the patch plan (ensure_bpatch), in the arithmetic it was made usable for.
+int enqueue_matvec_batched(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, uint32_t ld, int bc_mode,
+                           cudaStream_t st, bool f32, int tr, int ng) {
+    bool captured = false;
+    if (int s = take_turn(op, st, &captured)) return s;
+    const int s = enqueue_launches_batched(op, d_V, d_U, nrhs, ld, bc_mode, st, f32, tr, ng, captured);
+    const int e = end_turn(op, st, captured);
+    return s ? s : e;
 }
 
 int check_batched(afm_operator* op, uint32_t nrhs, uint32_t ld) {
@@ -2080,7 +2103,6 @@ int afm::set_stream_priority(afm_operator* op, int priority) {
     }
     cudaStreamDestroy(op->stream);
     op->stream = st;
-    op->ve_stream = nullptr;  // (its work has finished)
     drop_graph(op->cg64);  // no captured iteration keeps the old stream's work order
     drop_graph(op->cg32);
     drop_graph(op->cg64i);
@@ -2149,14 +2171,14 @@ int afm_create(afm_operator** out, int bc_method, int device) {
     op->sm_count = prop.multiProcessorCount;
     if (cudaStreamCreateWithFlags(&op->stream, cudaStreamNonBlocking) != cudaSuccess ||
         dalloc(op, &op->d_err, sizeof(int) * kErrWords) != cudaSuccess ||
-        dalloc(op, &op->d_usc, sizeof(unsigned long long) * kUscWords) != cudaSuccess ||
+        dalloc(op, &op->d_usc, sizeof(unsigned long long) * 2 * kUscWords) != cudaSuccess ||
         dalloc(op, &op->d_scalars, sizeof(double) * (kScalarSets * kScalarSlots + kPartialSlots)) != cudaSuccess ||
         cudaMallocHost((void**)&op->h_scalars, sizeof(double) * kScalarSlots) != cudaSuccess) {
         afm_destroy(op);
         return fail(AFM_ERR_CUDA, "afm_create: stream or buffer allocation failed");
     }
     cudaMemsetAsync(op->d_err, 0, sizeof(int) * kErrWords, op->stream);
-    cudaMemsetAsync(op->d_usc, 0, sizeof(unsigned long long) * kUscWords, op->stream);
+    cudaMemsetAsync(op->d_usc, 0, sizeof(unsigned long long) * 2 * kUscWords, op->stream);
     cudaStreamSynchronize(op->stream);
     *out = op;
     return ok();
@@ -2177,7 +2199,7 @@ int afm_destroy(afm_operator* op) {
         }
         if (op->h_scalars) cudaFreeHost(op->h_scalars);
         if (op->h_bremain) cudaFreeHost(op->h_bremain);
-        if (op->ve_event) cudaEventDestroy(op->ve_event);
+        if (op->turn_event) cudaEventDestroy(op->turn_event);
         if (op->stream) cudaStreamDestroy(op->stream);
     }
     delete op;
@@ -2242,6 +2264,7 @@ int afm_set_symmetric_inner(afm_operator* op, int format) {
     op->sym_mode = format;
     if (op->d_sym && op->sym_built != sym_arena(op)) {
         DeviceGuard g(op->device);
+        own_turn(op);
         dfree(op, op->d_sym);
         dfree(op, op->d_vx);
         op->sym_built = 0;

@@ -355,7 +355,8 @@ struct afm_operator {
     int* d_err = nullptr;
     unsigned long long wait_ns = 4000000000ull;  // limit of each kernel pipeline wait (afm_set_wait_limit)
     bool wait_probe = false;         // afm_set_wait_probe
-    unsigned long long* d_usc = nullptr;  // u-scale words of the split products (kUscWords, afm_solver.hpp)
+    unsigned long long* d_usc = nullptr;  // u-scale words of the split products (kUscWords, afm_solver.hpp), and as
+                                          // many for products recorded in callers' graphs
     uint8_t* d_bcmask = nullptr;     // 1 per constrained DoF (null without constraints)
     // one cooperative launch for every colour of a split product (segment plans of one element size)
     bool fused_ok = false;           // the plan allows it (decided at finalize)
@@ -442,8 +443,10 @@ struct afm_operator {
     double* d_ve = nullptr;            // owns the lists too
     uint32_t* d_gather_idx = nullptr;
     uint32_t* d_gather_off = nullptr;
-    cudaStream_t ve_stream = nullptr;  // stream of the last product that used d_ve or d_bp_pv
-    cudaEvent_t ve_event = nullptr;    // its end, where that stream is not the operator's own
+    // order of products on several streams (take_turn): 1 + the id of the stream of the last product (0: the operator's
+    // own stream, or none yet), and the end of that product where the stream is a caller's
+    unsigned long long turn_id = 0;
+    cudaEvent_t turn_event = nullptr;
     bool own_capture = false;          // the operator's solver is capturing its iterations on `stream`
 
     // batched (multi right-hand side) state

@@ -15,7 +15,13 @@
  *  - Host pointers are copied; nothing passed in is retained after the call
  *    returns (unlike Maps::set_map, which keeps dofs_per_element,
  *    include/maps.hpp:423).
- *  - All work for one operator is serialised on that operator's CUDA stream.
+ *  - All work for one operator is serialised: on that operator's CUDA stream,
+ *    and a product enqueued on a caller's stream waits for the operator's
+ *    product or solve before it, as the next one does for it. Products that a
+ *    caller records into a graph are not part of that order: replays must not
+ *    run beside other replays of the same operator's products, nor beside
+ *    other calls of an operator with patches (elements of up to 16 DoFs) or a
+ *    symmetric inner format of 2 or more.
  *    Calls on one operator are not re-entrant (same as aMatFree,
  *    include/aMatFree.hpp:75-84); different operators may be used from
  *    different threads.
