@@ -76,16 +76,16 @@ void* pick_kernel(int regime, uint32_t n, bool dup, bool chunked = false, bool v
 // land, and each SM needs ~200 KB of copies in flight to keep HBM busy, which
 // small slots reach only with many stages.
 constexpr uint32_t kMaxStages = 32;
-// Shared memory of a segment CTA: with 8-byte staged u the 196 KB configuration
+// Shared memory of a single-vector segment CTA: with 8-byte staged u the 196 KB configuration
 // (with the 1 KB the system takes), which leaves L1 60 KB for the gathers (tet10
 // elasticity 32^3 x 6 split 248 -> 239 us, hex8 elasticity 48^3 92 -> 91.5, hex20
 // 42^3 307 -> 305.5); FP32 rings use the depth (tet10 elasticity 92 us, 97 with 194
 // KB).
 constexpr uint32_t kRingBudget = sizeof(typename ARITH::UT) == 8 ? 194u * 1024 : kSmemBudget;
 #ifdef LAUNCH_FN
-static uint32_t stages_for(uint32_t slot_bytes, uint32_t extra) {
-    if (extra + 32 >= kRingBudget) return 0;
-    uint32_t st = (kRingBudget - extra - 32) / (slot_bytes + 20);
+static uint32_t stages_for(uint32_t slot_bytes, uint32_t extra, uint32_t budget = kRingBudget) {
+    if (extra + 32 >= budget) return 0;
+    uint32_t st = (budget - extra - 32) / (slot_bytes + 20);
     return st > kMaxStages ? kMaxStages : st;
 }
 
@@ -228,7 +228,8 @@ cudaError_t BATCH_FN(const Segment& s, const BatchArgs& a, int sm_count, int ct,
     // two stages more than there are consumer warps (as ring_layout does).
     for (L.warps = 8; L.warps >= 1; L.warps--) {
         L.extra_bytes = L.warps * 2 * L.ubuf_bytes;
-        L.stages = stages_for(L.slot_bytes, L.extra_bytes);
+        // (the columns of U take most of it: all there is, or elements of 60 DoFs run out of it at 120 columns)
+        L.stages = stages_for(L.slot_bytes, L.extra_bytes, kSmemBudget);
         if (L.stages >= L.warps + 2) break;
     }
     if (L.warps == 0 || L.stages < L.warps + 2) return cudaErrorInvalidConfiguration;

@@ -354,7 +354,9 @@ int afm_matmult_bc_device_f32(afm_operator* op, float* d_v, const float* d_u, vo
 /* ---- batched: many right-hand sides at once -------------------------------
  * Blocks are n_dofs x ld row-major device arrays (the nrhs values of one DoF
  * are contiguous), 16-byte aligned; nrhs is a multiple of 4, at most 256, ld
- * >= nrhs a multiple of 4; every element must have more than 16 DoFs. Each
+ * >= nrhs a multiple of 4; every element must have more than 16 DoFs, and on
+ * double blocks three of its matrices and 2 n_e nrhs doubles must fit in 226
+ * KB (n_e = 60: up to 144 columns; 81: 48). Each
  * element matrix is streamed once per call and applied to all columns (for
  * example hex8 elasticity with 64 right-hand sides): over patches of elements
  * of one size (24, 30 or 60 DoFs; not in AFM_PREC_FP64), whose rows of V a
