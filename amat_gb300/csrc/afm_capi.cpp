@@ -308,6 +308,11 @@ void free_device(afm_operator* op) {
     dfree(op, op->d_shared_pos);
     dfree(op, op->d_sym);
     dfree(op, op->d_packed);
+    dfree(op, op->d_loose_row);
+    dfree(op, op->d_loose_off);
+    dfree(op, op->d_loose_col);
+    dfree(op, op->d_loose_val);
+    op->n_loose_rows = 0;
     dfree(op, op->d_vx);
     dfree(op, op->d_csr_rp);
     dfree(op, op->d_csr_cols);
@@ -710,8 +715,7 @@ void build_segments(afm_operator* op, int prec) {
 // hex20 42^3 FP32 122 -> 98 us, format 4 225 -> 195 (0.56 M), 56^3 232 -> 236 and
 // 462 -> 458 (1.3 M); hex8 elasticity 72^3 159 -> 126 us (1.1 M), 90^3 258 -> 242
 // (2.2 M); tet10 elasticity 44^3 x 6 FP32 339 -> 242. The split products on block
-// units go with these: hex20 30^3 109 -> 90 us, 42^3 238 -> 227 (0.56 M), 54^3 477 ->
-// 470 (1.2 M).
+// units go with these: hex20 20^3 58 -> 31 us, 30^3 114 -> 88, 42^3 254 -> 246 (0.56 M), 54^3 514 -> 520 (1.2 M).
 bool gather_pays(const afm_operator* op, bool wide, uint32_t ve_bytes) {
     const uint64_t entries = (uint64_t)op->n_elem * op->nmax;
     const uint64_t most = op->nmax > 32 ? (wide ? 200000u : 1200000u) : (wide ? 900000u : 2200000u);
@@ -812,38 +816,110 @@ int end_turn(afm_operator* op, cudaStream_t st, bool captured) {
     return AFM_SUCCESS;
 }
 
+// Calls f(r, c) for each pair of element e's matrix k, of n DoFs, that a block unit does not hold; (r, c) is the entry
+// that the unit would store.
+template <typename F>
+void for_loose_pairs(const double* k, uint32_t n, const F& f) {
+    for (uint32_t a = 0; a < n; a++)
+        for (uint32_t b = a + 1; b < n; b++) {
+            const double x = k[(size_t)a * n + b], y = k[(size_t)b * n + a];
+            const int side = x == y ? 0 : block_side(a, b, n);
+            if (!side) continue;
+            const float h = (float)(side > 0 ? x : y), th = (float)(side > 0 ? y : x);
+            const float tl = (float)((side > 0 ? y : x) - (double)th);
+            if (!block_holds(h, th, tl)) side > 0 ? f(a, b) : f(b, a);
+        }
+}
+
 // True when every element matrix is symmetric to within 1e-6 of its largest
 // diagonal entry (exactly, for an element whose diagonal is zero). *exact:
-// every one equal to its transpose.
-bool ke_is_symmetric(const afm_operator* op, bool* exact, bool* near) {
-    int sym = 1, same = 1, close = 1;
-#pragma omp parallel for schedule(static) reduction(&& : sym, same, close)
+// every one equal to its transpose. *pairs: the pairs of elements of 60 DoFs
+// that block units do not hold (counted until they are too many for block
+// units), loose: their elements.
+bool ke_is_symmetric(const afm_operator* op, bool* exact, uint64_t* pairs, std::vector<uint32_t>& loose) {
+    int sym = 1, same = 1, many = 0;
+    *pairs = 0;
+    loose.clear();
+#pragma omp parallel for schedule(static) reduction(&& : sym, same) firstprivate(many)
     for (int64_t e = 0; e < (int64_t)op->n_elem; e++) {
         if (!sym) continue;
         const uint32_t n = op->offsets[e + 1] - op->offsets[e];
         const double* k = op->ke.data() + op->kofs[e];
-        double dmax = 0.0, dmin = 1e300;
-        for (uint32_t r = 0; r < n; r++) {
-            const double d = std::fabs(k[(size_t)r * n + r]);
-            dmax = std::max(dmax, d);
-            dmin = std::min(dmin, d);
-        }
+        double dmax = 0.0;
+        for (uint32_t r = 0; r < n; r++) dmax = std::max(dmax, std::fabs(k[(size_t)r * n + r]));
         const double tol = 1e-6 * dmax;
         for (uint32_t r = 0; r < n && sym; r++)
             for (uint32_t c = r + 1; c < n; c++) {
                 const double x = k[(size_t)r * n + c], y = k[(size_t)c * n + r];
                 if (x == y) continue;
                 same = 0;
-                if (!(std::fabs(x - y) <= kBlockAsym * dmin)) close = 0;
                 if (!(std::fabs(x - y) <= tol)) {
                     sym = 0;
                     break;
                 }
             }
+        if (sym && !many && split_block_bytes(n)) {
+            uint32_t found = 0;
+            for_loose_pairs(k, n, [&](uint32_t, uint32_t) { found++; });
+            if (found) {
+#pragma omp critical
+                {
+                    *pairs += found;
+                    loose.push_back((uint32_t)e);
+                    many = *pairs * kElemsPerLoosePair > op->n_elem;
+                }
+            }
+        }
     }
     *exact = sym && same;
-    *near = sym && close;
     return sym != 0;
+}
+
+// The entries of the pairs that block units leave out, row by row, on the device. No room: no block units.
+int build_loose(afm_operator* op, std::vector<uint32_t> elems, const std::vector<uint8_t>& is_bc) {
+    struct Entry {
+        uint32_t row, col;
+        double val;
+    };
+    std::vector<Entry> all;
+    std::sort(elems.begin(), elems.end());
+    for (uint32_t e : elems) {
+        const uint32_t n = op->offsets[e + 1] - op->offsets[e];
+        const double* k = op->ke.data() + op->kofs[e];
+        const uint32_t* m = op->map.data() + op->offsets[e];
+        for_loose_pairs(k, n, [&](uint32_t r, uint32_t c) {
+            all.push_back({m[r], m[c], k[(size_t)r * n + c]});
+            all.push_back({m[c], m[r], k[(size_t)c * n + r]});
+        });
+    }
+    std::stable_sort(all.begin(), all.end(), [](const Entry& x, const Entry& y) { return x.row < y.row; });
+    std::vector<uint32_t> row, off, col;
+    std::vector<double> val;
+    for (const Entry& x : all) {
+        if (row.empty() || row.back() != x.row) {
+            row.push_back(x.row);
+            off.push_back((uint32_t)col.size());
+        }
+        col.push_back(x.col | (is_bc[x.col] ? kBcFlag : 0u));
+        val.push_back(x.val);
+    }
+    off.push_back((uint32_t)col.size());
+    if (dalloc(op, &op->d_loose_row, sizeof(uint32_t) * row.size()) != cudaSuccess ||
+        dalloc(op, &op->d_loose_off, sizeof(uint32_t) * off.size()) != cudaSuccess ||
+        dalloc(op, &op->d_loose_col, sizeof(uint32_t) * col.size()) != cudaSuccess ||
+        dalloc(op, &op->d_loose_val, sizeof(double) * val.size()) != cudaSuccess) {
+        cudaGetLastError();  // no room: whole matrices
+        dfree(op, op->d_packed);
+        return AFM_SUCCESS;
+    }
+    cudaStream_t st = op->stream;
+    AFM_CUDA(cudaMemcpyAsync(op->d_loose_row, row.data(), sizeof(uint32_t) * row.size(), cudaMemcpyHostToDevice, st));
+    AFM_CUDA(cudaMemcpyAsync(op->d_loose_off, off.data(), sizeof(uint32_t) * off.size(), cudaMemcpyHostToDevice, st));
+    AFM_CUDA(cudaMemcpyAsync(op->d_loose_col, col.data(), sizeof(uint32_t) * col.size(), cudaMemcpyHostToDevice, st));
+    AFM_CUDA(cudaMemcpyAsync(op->d_loose_val, val.data(), sizeof(double) * val.size(), cudaMemcpyHostToDevice, st));
+    AFM_CUDA(cudaStreamSynchronize(st));
+    op->n_loose_rows = (uint32_t)row.size();
+    return AFM_SUCCESS;
 }
 
 // Layout of the symmetric inner arena in format `mode` (1: FP32, 2: FP32 +
@@ -1203,7 +1279,8 @@ int enqueue_launches(afm_operator* op, void* d_v, const void* d_u, int bc_mode, 
             a.ke = op->d_packed;
             a.unit_bytes = a.copy_bytes = split_block_bytes(s0.n);
         }
-        AFM_CUDA((blocks ? launch_fused_splitblk : launch_fused_split)(op->segs.data(), (uint32_t)op->segs.size(), a, op->d_gbar, op->sm_count, st));
+        AFM_CUDA((blocks ? launch_fused_splitblk : launch_fused_split)(op->segs.data(), (uint32_t)op->segs.size(), a,
+                                                                       op->d_gbar, op->sm_count, st));
         return AFM_SUCCESS;
     }
     for (const Segment& s : op->segs) {
@@ -1243,7 +1320,13 @@ int enqueue_matvec(afm_operator* op, void* d_v, const void* d_u, int bc_mode, cu
                    bool inner64 = false, ProductTail* tail = nullptr) {
     bool captured = false;
     if (int s = take_turn(op, st, &captured)) return s;
-    const int s = enqueue_launches(op, d_v, d_u, bc_mode, st, f32, inner64, tail, captured);
+    // (with pairs to add, v is not complete when the product's own last pass ends)
+    const bool loose = op->n_loose_rows && !f32 && !inner64;
+    int s = enqueue_launches(op, d_v, d_u, bc_mode, st, f32, inner64, loose ? nullptr : tail, captured);
+    if (!s && loose &&
+        launch_add_pairs(static_cast<double*>(d_v), static_cast<const double*>(d_u), op->d_loose_row, op->d_loose_off,
+                         op->d_loose_col, op->d_loose_val, op->n_loose_rows, bc_mode, st) != cudaSuccess)
+        s = fail(AFM_ERR_CUDA, "loose pairs: %s", cudaGetErrorString(cudaGetLastError()));
     const int e = end_turn(op, st, captured);
     return s ? s : e;
 }
@@ -2768,12 +2851,13 @@ int afm_finalize(afm_operator* op) {
     // symmetric Ke, and elements that run as patches or on the warp-group kernel
     op->ke_symmetric = false;
     op->ke_sym_exact = false;
-    op->ke_sym_near = false;
+    op->loose_pairs = 0;
     op->sym_ok = false;
     op->sym_bytes = 0;
     op->sym_built = 0;
     if (prec == AFM_PREC_FP64_SPLIT && !op->dup_in_element && op->n_elem > 0) {
-        op->ke_symmetric = ke_is_symmetric(op, &op->ke_sym_exact, &op->ke_sym_near);
+        std::vector<uint32_t> loose;
+        op->ke_symmetric = ke_is_symmetric(op, &op->ke_sym_exact, &op->loose_pairs, loose);
         bool covered = true;
         if (!op->use_patches)
             for (const Segment& s : op->segs)
@@ -2784,7 +2868,8 @@ int afm_finalize(afm_operator* op) {
             if (alloc_packed(op, (uint64_t)s.units * s.n * (s.n + 1) * kTpeWidth * 4))
                 AFM_CUDA(pack_split_units(op->d_ke, s.n, s.units, op->d_packed, op->sm_count, op->stream));
         }
-        if (!op->use_patches && op->ke_sym_near && op->n_elem >= kBlockElemsPerSm * (uint64_t)std::max(op->sm_count, 1)) {
+        if (!op->use_patches && op->ke_symmetric && op->loose_pairs * kElemsPerLoosePair <= op->n_elem &&
+            op->n_elem >= kBlockElemsPerSm * (uint64_t)std::max(op->sm_count, 1)) {
             uint64_t bytes = 0;
             for (Segment& s : op->segs) {
                 if (s.units == 0) continue;
@@ -2796,6 +2881,8 @@ int afm_finalize(afm_operator* op) {
                 for (const Segment& s : op->segs)
                     AFM_CUDA(pack_split_blocks(op->d_ke + s.ke_offset, s.unit_bytes, s.plane, s.n, s.units,
                                                op->d_packed + s.blk_offset, op->sm_count, op->stream));
+                if (op->loose_pairs)
+                    if ((st = build_loose(op, loose, is_bc))) return st;
             }
         }
     }

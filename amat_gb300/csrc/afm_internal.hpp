@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -220,18 +221,42 @@ constexpr int kPrecSplitSym = 20;
 // ... and on symmetric element units of 2 x 2 blocks (ArithSplitBlk).
 constexpr int kPrecSplitBlk = 21;
 // Bytes of such a unit (0: no block kernel for this size): n/4 + 1 (rounded down) wrapped diagonals of n/2 blocks with
-// 4 hi, 4 lo entries and 4 bytes each, and 16 bytes with the bytes' unit.
+// 4 hi and 4 lo entries each, and for all but the first and the last the 4 lo entries of the transposed block.
 constexpr uint32_t split_block_bytes(uint32_t n) {
-    return n == 60 ? (n / 4 + 1) * (n / 2) * 36 + 16 : 0u;
+    return n == 60 ? ((n / 4 + 1) * 32 + (n / 4 - 1) * 16) * (n / 2) : 0u;
 }
-// Largest |K(r, c) - K(c, r)| of a block unit, relative to the element's smallest diagonal entry: its byte then holds the
-// difference to 2^-53 of that entry, half the last place of the FP64 sums that K came from, in every row of an element
-// with rows of very different sizes too (relative to the largest, rows 1e10 smaller would lose 8 digits). Matrices from
-// quadrature on this library's meshes differ by 2^-52 to 2^-50.
-constexpr double kBlockAsym = 0x1p-46;
-// Elements per SM from which a plan takes block units (24 consumer warps hold 6 elements of an SM; below about ten each
-// the longer way of one element shows): hex20 elasticity with 1000 elements 11.4 us on whole units, 13.1 on blocks; 1331
-// 13.2 and 13.6; 1440 14.2 and 14.0; 1584 15.1 and 14.0; 2744 20.2 and 19.4.
+// The lo part of K(c, r) in a block unit, beside the hi part of K(r, c) (h): what is left of the split pair (th, tl) of
+// K(c, r), which is tl itself where the two hi parts agree.
+AFM_HD inline float split_transposed(float h, float th, float tl) {
+    return (float)(((double)th - (double)h) + (double)tl);
+}
+// Whether such a unit holds K(c, r) as the split pair does: to 2^-48 of itself, and as a leading part with a low part
+// below its last place (2^-23 of it: the products round a low part to 24 bits and leave out its product with u's low
+// part). Not where the rounding of the quadrature sums (2^-57 of the diagonal) is no small part of the entry: entries
+// below 2^-34 of the diagonal, the zeros of regular meshes above all, and in jittered ones (15 x of the entries are below
+// x of the diagonal) one in 1e9 or so. Such pairs are left out of the units and added by a pass of their own
+// (launch_add_pairs).
+AFM_HD inline bool block_holds(float h, float th, float tl) {
+    if (h == th) return true;
+    const double t = ((double)th - (double)h) + (double)tl;
+    const float l = (float)t;
+    return fabs(t - (double)l) <= 0x1p-49 * fabs((double)th) && fabs((double)l) <= 0x1p-23 * fabs((double)th);
+}
+// Whether a block unit stores entry (r, c) itself, its transpose beside it (1), as the transpose of (c, r) (-1), or both
+// (0: the first and the last wrapped diagonal).
+inline int block_side(uint32_t r, uint32_t c, uint32_t n) {
+    const uint32_t nb = n / 2, d = (c / 2 + nb - r / 2) % nb;
+    return d == 0 || d == nb / 2 ? 0 : d < nb / 2 ? 1 : -1;
+}
+// Pairs left out of block units, at most one in this many elements (a regular mesh has 84 an element: whole matrices).
+constexpr uint32_t kElemsPerLoosePair = 8;
+// v[row[i]] += the sum over k in [off[i], off[i + 1]) of val[k] u[col[k]], in order (bc_mode: constrained columns, kBcFlag
+// in col, as zero).
+cudaError_t launch_add_pairs(double* v, const double* u, const uint32_t* row, const uint32_t* off, const uint32_t* col,
+                             const double* val, uint32_t rows, int bc_mode, cudaStream_t st);
+// Elements per SM from which a plan takes block units (20 consumer warps hold 5 elements of an SM, so that below about ten
+// each the ramps are most of the time): hex20 elasticity with 1000 elements 10.9 us on whole units, 10.9 on blocks; 1331
+// 13.5 and 13.0; 1440 14.2 and 13.3; 1584 15.3 and 14.0; 2744 20.2 and 16.9.
 constexpr uint32_t kBlockElemsPerSm = 10;
 // Packs a segment's split units into block units (afm_mv_splitblk.cu).
 cudaError_t pack_split_blocks(const unsigned char* ke, uint64_t unit_bytes, uint32_t plane, uint32_t n, uint32_t units,
@@ -387,9 +412,15 @@ struct afm_operator {
     // entries stored once, built from the split arena on the first FP32 product
     bool ke_symmetric = false;      // every Ke symmetric to 1e-6 of its largest diagonal entry
     bool ke_sym_exact = false;      // every Ke equal to its transpose bit for bit
-    bool ke_sym_near = false;       // ... or to kBlockAsym
-    // the split units of a patch plan with exactly symmetric Ke, packed, or of a segment plan with nearly symmetric Ke of
-    // 60 DoFs, as block units (FP64 products read them; null: they read d_ke)
+    uint64_t loose_pairs = 0;       // pairs of symmetric Ke of 60 DoFs that block units do not hold (block_holds)
+    // ... and their entries, where the plan has block units: per row (DoF) its columns and values, row by row
+    uint32_t n_loose_rows = 0;
+    uint32_t* d_loose_row = nullptr;
+    uint32_t* d_loose_off = nullptr;
+    uint32_t* d_loose_col = nullptr;
+    double* d_loose_val = nullptr;
+    // the split units of a patch plan with exactly symmetric Ke, packed, or of a segment plan with Ke of 60 DoFs symmetric
+    // up to rounding, as block units (FP64 products read them; null: they read d_ke)
     unsigned char* d_packed = nullptr;
     bool sym_ok = false;            // symmetric, split arena, and a layout the symmetric kernels cover
     int sym_mode = 1;               // afm_set_symmetric_inner: 0 off, 1 FP32, 2 FP32 + BF16 correction

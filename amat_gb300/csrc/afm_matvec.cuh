@@ -403,7 +403,7 @@ struct ArithSplitSym : ArithSplit {
 // and its transpose once (split_block_terms).
 struct ArithSplitBlk : ArithSplit {
     static constexpr bool kSym = true;  // (u staged twice in a row)
-    static constexpr uint32_t kWpgWarps = 24;  // hex20 42^3: 16 warps 290 us, 20 272 (even runs); 20 248, 24 239 (uneven)
+    static constexpr uint32_t kWpgWarps = 24;  // (hex20: 20, with 7 ring slots in 194 KB; 42^3 246 us, 16 283; 24 in 226 KB 261)
 };
 template <typename A>
 inline constexpr bool kBlocks = false;
@@ -960,25 +960,25 @@ __device__ __forceinline__ void split_pair_terms(f2& hi, f2& lo, const float* kh
     }
 }
 
-// Block units (ArithSplitBlk; elements of 60 DoFs whose Ke is symmetric to 2^-46 of its smallest diagonal entry): NB =
-// n / 2 block rows of 2 x 2 blocks B(i, j); of each pair B(i, j), B(j, i) one is stored, by wrapped diagonals d = 0 ..
-// NB / 2: block (i, (i + d) mod NB) at d NB + i, its hi entries row by row in one float4, its lo entries in a second
-// plane. Element matrices from quadrature are symmetric only up to rounding, so a third plane holds K(c, r) - K(r, c) of
-// each entry as a biased byte times a power of two per element (the float after the plane): K(r, c) is the split
-// arena's to the bit, K(c, r) to 2^-53 of that diagonal entry. 60% of the whole matrix's bytes.
-// The operations stay those of the whole matrix but for the third plane's (a byte permutation and an add and a
-// multiply-add per entry of a transposed block) and 4 shuffles per diagonal.
+// Block units (ArithSplitBlk; elements of 60 DoFs whose Ke is symmetric up to rounding: block_holds): NB = n / 2 block
+// rows of 2 x 2 blocks B(i, j); of each pair B(i, j), B(j, i) one is stored, by wrapped diagonals d = 0 .. NB / 2: block
+// (i, (i + d) mod NB) at d NB + i, its hi entries row by row in one float4, its lo entries in a second plane. Element
+// matrices from quadrature are symmetric only up to rounding, so a third plane (no first and last diagonal) holds the lo
+// parts of the transposed block, beside the same hi parts: both entries of a pair are the split arena's to 2^-48 of
+// each (the few pairs that this does not hold are zero here and added by a pass of their own). 77% of the whole matrix's
+// bytes.
+// The operations stay those of the whole matrix, and 4 shuffles per diagonal.
 // A lane owns block row i. For each diagonal it adds B(i, j) u_j to its own sums, and B(i, j)^T u_i to the sums of
 // block row j, which travel: the lane that needs them for the next diagonal is the neighbour. The own sums are kept
 // per column parity (row 0: (k00 x0, k01 x1)), so that every operand is a pair as loaded: no packing in the loop.
 // Diagonals 0 and NB / 2 hold both blocks of a pair and have no transposed part. Warp q of the element's four takes
 // diagonals [block_run(q), block_run(q + 1)): 3, 3, 5 and 5, as the first two also gather u and scatter v, and the others
-// would wait for them at the element's barrier (42^3: 2, 2, 6 and 6 261 us, 4 each 278, this 248, with 20 warps).
-// What bounds it now is the double-float arithmetic and its latencies (0.4 to 0.6 instructions issued per cycle), so the
-// gain is below the bytes': hex20 elasticity 42^3 306 -> 239 us a product (5.4 TB/s; 227 in one launch with
-// the gather pass), 56^3 715 -> 534, 14^3 20.2 -> 19.4. In
+// would wait for them at the element's barrier (42^3 246 us, 28^3 72; with 2, 2, 6 and 6 247 and 73, 4 each 251 and 76).
+// What bounds it is HBM where the products are long (42^3 6.7 TB/s of units) and the latencies of the double-float
+// arithmetic where they are short. Whole matrices with rows in pairs -> this: hex20 elasticity 14^3 20.3 -> 17.0 us a
+// product, 28^3 100 -> 72, 42^3 304 -> 246, 56^3 722 -> 578. In
 // elements of 24 and 30 DoFs (two runs of diagonals per warp) the overhead per element outweighs it: hex8 elasticity
-// 48^3 92 -> 97 us, tet10 elasticity 32^3 x 6 240 -> 241.
+// 48^3 92 -> 97 us, tet10 elasticity 32^3 x 6 240 -> 241 (measured with a byte in place of the third plane's floats).
 template <int NT>
 __host__ __device__ constexpr int block_run(int q) {
     constexpr int ND = NT / 4 + 1, A = 3;  // (A: the gathering warps' diagonals)
@@ -991,10 +991,8 @@ __device__ __forceinline__ void split_block_terms(f2& hi, f2& lo, const unsigned
     // (lanes past the last block row repeat the first lanes' work; nothing of theirs is used)
     const int l = (int)lane < NB ? (int)lane : (int)lane - NB;
     const float4* kp = reinterpret_cast<const float4*>(ks) + l;
-    const uint32_t* dp = reinterpret_cast<const uint32_t*>(ks + ND * NB * 32) + l;
     const float4* xp = ub + l;
-    const float step = *reinterpret_cast<const float*>(ks + ND * NB * 36);
-    const f2 step2 = pack2(step, step), m1 = pack2(-1.0f, -1.0f), bias = pack2(-8388736.0f, -8388736.0f);
+    const f2 m1 = pack2(-1.0f, -1.0f);
     const float4 o = ub[l];
     const f2 u0 = pack2(o.x, o.x), n0 = pack2(-o.x, -o.x), v0 = pack2(o.z, o.z);
     const f2 u1 = pack2(o.y, o.y), n1 = pack2(-o.y, -o.y), v1 = pack2(o.w, o.w);
@@ -1012,10 +1010,8 @@ __device__ __forceinline__ void split_block_terms(f2& hi, f2& lo, const unsigned
         split_term2(w0h, w0l, k0, l0, xh, xn, xl);
         split_term2(w1h, w1l, k1, l1, xh, xn, xl);
         if (d != 0 && d != ND - 1) {
-            const uint32_t w = dp[d * NB];
-            auto byte = [&](uint32_t i) { return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u | i)); };  // 2^23 + byte
-            const f2 e0 = fma2(add2(pack2(byte(0), byte(1)), bias), step2, l0);
-            const f2 e1 = fma2(add2(pack2(byte(2), byte(3)), bias), step2, l1);
+            const float4 t = kp[(2 * ND + d - 1) * NB];
+            const f2 e0 = pack2(t.x, t.y), e1 = pack2(t.z, t.w);
             split_term2(th, tl, k0, e0, u0, n0, v0);
             split_term2(th, tl, k1, e1, u1, n1, v1);
         }
