@@ -1357,7 +1357,7 @@ constexpr int kPatchTile = -1;  // "columns of the lane tile" of the patch plan
 // The patch plan of the batched product, where the elements have one size that
 // its kernel takes in this arithmetic and list no DoF twice; and its combine
 // buffer for nrhs columns. Call outside stream capture.
-int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, cudaStream_t st, bool* usable) {
+int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, bool* usable) {
     *usable = false;
     if (op->bp_state < 0 || (!f32 && op->precision != AFM_PREC_FP64_SPLIT)) return AFM_SUCCESS;
     if (op->bp_state == 0) {
@@ -1407,8 +1407,7 @@ int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, cudaStream_t st, bo
         op->bp_pv_bytes = bytes;
         op->generation++;  // captured iterations hold the old buffer
     }
-    if (st != op->stream) AFM_CUDA(cudaStreamSynchronize(op->stream));  // (the plan and the buffer are there)
-    *usable = true;
+    *usable = true;  // (a product on st takes its turn after the work enqueued here)
     return AFM_SUCCESS;
 }
 
@@ -1543,12 +1542,12 @@ int batch_tuning(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, ui
                 cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
                 AFM_CUDA(cudaStreamIsCapturing(st, &cap));
                 if (cap == cudaStreamCaptureStatusNone)
-                    if (int s = ensure_bpatch(op, nrhs, f32, st, &patch)) return s;
+                    if (int s = ensure_bpatch(op, nrhs, f32, &patch)) return s;
                 if (!patch) *tr = t.tr;
             }
             return AFM_SUCCESS;
         }
-    if (int s = ensure_bpatch(op, nrhs, f32, st, &patch)) return s;
+    if (int s = ensure_bpatch(op, nrhs, f32, &patch)) return s;
     // (columns, rows) of the lane tile; (0, 0): the tensor-core kernel (FP32 products)
     std::vector<std::pair<int, int>> cand = {{8, 6}, {8, 4}, {8, 2}, {4, 4}};
     if (f32 && allow_tc && batched_tc_all(op, nrhs)) cand.insert(cand.begin(), {0, 0});
