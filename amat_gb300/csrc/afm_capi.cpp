@@ -231,6 +231,11 @@ uint64_t round16(uint64_t b) { return (b + 15) / 16 * 16; }
 // its own streams with this operator must be ordered before such a release.
 template <typename T>
 cudaError_t dalloc(afm_operator* op, T** p, size_t bytes) {
+    if (op->fail_allocs && op->fail_skip-- <= 0) {
+        op->fail_allocs--;
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
     return cudaMallocAsync((void**)p, bytes, op->stream);
 }
 template <typename T>
@@ -266,6 +271,16 @@ void own_turn(afm_operator* op) {
     op->turn_id = 0;
 }
 
+// The patch plan of the batched products and its combine buffer.
+void drop_bpatch(afm_operator* op) {
+    dfree(op, op->d_bp_hdr);
+    dfree(op, op->d_bp_dof);
+    dfree(op, op->d_bp_off);
+    dfree(op, op->d_bp_idx);
+    dfree(op, op->d_bp_pv);
+    op->bp_pv_bytes = 0;
+}
+
 void free_device(afm_operator* op) {
     own_turn(op);
     drop_graph(op->cg64);
@@ -274,13 +289,8 @@ void free_device(afm_operator* op) {
     drop_graph(op->bcg64);
     drop_graph(op->bcg32);
     op->batch_tune.clear();
-    dfree(op, op->d_bp_hdr);
-    dfree(op, op->d_bp_dof);
-    dfree(op, op->d_bp_off);
-    dfree(op, op->d_bp_idx);
-    dfree(op, op->d_bp_pv);
+    drop_bpatch(op);
     op->bp_state = 0;
-    op->bp_pv_bytes = 0;
     dfree(op, op->d_bwork);
     dfree(op, op->d_bsc);
     op->bwork_elems = 0;
@@ -1356,7 +1366,8 @@ constexpr int kPatchTile = -1;  // "columns of the lane tile" of the patch plan
 
 // The patch plan of the batched product, where the elements have one size that
 // its kernel takes in this arithmetic and list no DoF twice; and its combine
-// buffer for nrhs columns. Call outside stream capture.
+// buffer for nrhs columns. Without room for them the launches per colour, which
+// need none, go on. Call outside stream capture.
 int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, bool* usable) {
     *usable = false;
     if (op->bp_state < 0 || (!f32 && op->precision != AFM_PREC_FP64_SPLIT)) return AFM_SUCCESS;
@@ -1374,10 +1385,14 @@ int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, bool* usable) {
         for (uint32_t d : op->bc_unique) is_bc[d] = 1;
         BPatchPlanHost plan;
         build_bpatch_plan(op->n_elem, op->n_dofs, n, op->map.data(), op->perm.data(), first, is_bc.data(), plan);
-        AFM_CUDA(dalloc(op, &op->d_bp_hdr, std::max<size_t>(plan.hdr.size(), 16)));
-        AFM_CUDA(dalloc(op, &op->d_bp_dof, sizeof(uint32_t) * std::max<size_t>(plan.shared_dof.size(), 1)));
-        AFM_CUDA(dalloc(op, &op->d_bp_off, sizeof(uint32_t) * plan.shared_off.size()));
-        AFM_CUDA(dalloc(op, &op->d_bp_idx, sizeof(uint32_t) * std::max<size_t>(plan.shared_idx.size(), 1)));
+        if (dalloc(op, &op->d_bp_hdr, std::max<size_t>(plan.hdr.size(), 16)) != cudaSuccess ||
+            dalloc(op, &op->d_bp_dof, sizeof(uint32_t) * std::max<size_t>(plan.shared_dof.size(), 1)) != cudaSuccess ||
+            dalloc(op, &op->d_bp_off, sizeof(uint32_t) * plan.shared_off.size()) != cudaSuccess ||
+            dalloc(op, &op->d_bp_idx, sizeof(uint32_t) * std::max<size_t>(plan.shared_idx.size(), 1)) != cudaSuccess) {
+            cudaGetLastError();
+            drop_bpatch(op);
+            return AFM_SUCCESS;
+        }
         auto up = [&](void* d, const void* h, size_t bytes) {
             return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, op->stream);
         };
@@ -1399,8 +1414,8 @@ int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, bool* usable) {
         own_turn(op);
         dfree(op, op->d_bp_pv);
         op->bp_pv_bytes = 0;
-        if (cudaMallocAsync((void**)&op->d_bp_pv, bytes, op->stream) != cudaSuccess) {
-            cudaGetLastError();  // no room: the launches per colour need none
+        if (dalloc(op, &op->d_bp_pv, bytes) != cudaSuccess) {
+            cudaGetLastError();
             op->d_bp_pv = nullptr;
             return AFM_SUCCESS;
         }
@@ -3142,6 +3157,14 @@ int afm_solve_cg_mixed_device(afm_operator* op, const double* d_b, double* d_x, 
     }
     const int st = mixed_end(m, stats);
     return s != AFM_SUCCESS ? s : st;
+}
+
+int afm_debug_fail_allocations(afm_operator* op, int skip, int count) {
+    AFM_CHECK_OP(op);
+    if (skip < 0 || count < 0) return fail(AFM_ERR_INVALID_ARG, "skip %d, count %d", skip, count);
+    op->fail_skip = skip;
+    op->fail_allocs = count;
+    return ok();
 }
 
 int afm_debug_segment_geometry(int kind, uint32_t n, uint32_t* out) {

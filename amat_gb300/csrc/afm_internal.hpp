@@ -380,6 +380,7 @@ struct afm_operator {
     int* d_err = nullptr;
     unsigned long long wait_ns = 4000000000ull;  // limit of each kernel pipeline wait (afm_set_wait_limit)
     bool wait_probe = false;         // afm_set_wait_probe
+    int fail_skip = 0, fail_allocs = 0;  // afm_debug_fail_allocations
     unsigned long long* d_usc = nullptr;  // u-scale words of the split products (kUscWords, afm_solver.hpp), and as
                                           // many for products recorded in callers' graphs
     uint8_t* d_bcmask = nullptr;     // 1 per constrained DoF (null without constraints)

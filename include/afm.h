@@ -325,6 +325,9 @@ int afm_solve_cg_device(afm_operator* op, const double* d_b, double* d_x, double
  * consumer warps, element groups, column groups, dynamic shared memory bytes,
  * unit bytes, bytes copied per unit. */
 int afm_debug_segment_geometry(int kind, uint32_t n, uint32_t* out);
+/* Test hook: of the operator's device allocations from now on, the `count` that
+ * follow the next `skip` fail, as if the device had no room. */
+int afm_debug_fail_allocations(afm_operator* op, int skip, int count);
 /* The last mixed-precision solve of the operator (afm_solve_cg_mixed*): at
  * each FP64 residual, the inner iterations done so far and ||b - A x|| / ||b||.
  * *n = the count; up to cap entries are written. */
