@@ -13,7 +13,8 @@ namespace afm {
 
 constexpr uint32_t kBPatchElems = 8;  // elements per patch, at most
 // rows (local DoFs) per patch, at most: 2 x 2 x 2 linear bricks have 81; one hex20 element has 60
-AFM_HD inline uint32_t bpatch_max_rows(uint32_t n) { return n <= 32 ? 96u : 128u; }
+constexpr uint32_t kBPatchRows = 128;
+AFM_HD inline uint32_t bpatch_max_rows(uint32_t n) { return n <= 32 ? 96u : kBPatchRows; }
 
 // One patch's block in the plan (hdr_bytes apart, 16-byte aligned):
 //   uint32 {elements, rows, rows of this patch alone, first row of the others in the combine buffer}, 4 words free,

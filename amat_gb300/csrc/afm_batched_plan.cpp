@@ -1,6 +1,7 @@
 // Host side of the batched product's patch plan (afm_batched_patch.hpp).
 #include <algorithm>
 #include <cstring>
+#include <utility>
 
 #include "afm_batched_patch.hpp"
 
@@ -115,45 +116,44 @@ void build_bpatch_plan(uint32_t n_elem, uint32_t n_dofs, uint32_t n, const uint3
     out.hdr.assign((size_t)P * out.geom.hdr_bytes, 0);
     // headers, and the combine lists' entries: entry r of a shared node is its row in its r-th patch
     out.shared_idx.assign((size_t)soff[nodes] * b, 0);
-#pragma omp parallel
-    {
-        std::vector<uint32_t> place(nodes);  // of the patch's nodes
-#pragma omp for schedule(static)
-        for (int64_t p = 0; p < (int64_t)P; p++) {
-            unsigned char* h = out.hdr.data() + (size_t)p * out.geom.hdr_bytes;
-            uint32_t* w = reinterpret_cast<uint32_t*>(h);
-            const uint32_t ne = first[p + 1] - first[p], nn = nfirst[p + 1] - nfirst[p];
-            uint32_t* ep = w + 8;
-            uint32_t* rows = reinterpret_cast<uint32_t*>(h + bpatch_rows_off());
-            unsigned char* loc = h + bpatch_loc_off(out.geom.max_rows);
-            // the patch's own nodes first
-            uint32_t own = 0, k = 0;
-            for (int shared = 0; shared < 2; shared++) {
-                for (uint32_t q = nfirst[p]; q < nfirst[p + 1]; q++) {
-                    const uint32_t m = pnodes[q];
-                    if ((cnt[m] > 1) != (shared == 1)) continue;
-                    place[m] = k;
-                    for (uint32_t c = 0; c < b; c++) {
-                        const uint32_t d = m * b + c;
-                        rows[k * b + c] = d | (is_bc[d] ? kBcFlag : 0u);
-                        if (shared)  // the node's DoFs have lists of equal length one after another
-                            out.shared_idx[(size_t)soff[m] * b + c * cnt[m] + rank[q]] = pv0[p] + (k - own) * b + c;
-                    }
-                    k++;
+#pragma omp parallel for schedule(static)
+    for (int64_t p = 0; p < (int64_t)P; p++) {
+        unsigned char* h = out.hdr.data() + (size_t)p * out.geom.hdr_bytes;
+        uint32_t* w = reinterpret_cast<uint32_t*>(h);
+        const uint32_t ne = first[p + 1] - first[p], nn = nfirst[p + 1] - nfirst[p];
+        uint32_t* ep = w + 8;
+        uint32_t* rows = reinterpret_cast<uint32_t*>(h + bpatch_rows_off());
+        unsigned char* loc = h + bpatch_loc_off(out.geom.max_rows);
+        std::pair<uint32_t, uint32_t> place[kBPatchRows];  // the patch's nodes and their places, by node
+        // the patch's own nodes first
+        uint32_t own = 0, k = 0;
+        for (int shared = 0; shared < 2; shared++) {
+            for (uint32_t q = nfirst[p]; q < nfirst[p + 1]; q++) {
+                const uint32_t m = pnodes[q];
+                if ((cnt[m] > 1) != (shared == 1)) continue;
+                place[k] = {m, k};
+                for (uint32_t c = 0; c < b; c++) {
+                    const uint32_t d = m * b + c;
+                    rows[k * b + c] = d | (is_bc[d] ? kBcFlag : 0u);
+                    if (shared)  // the node's DoFs have lists of equal length one after another
+                        out.shared_idx[(size_t)soff[m] * b + c * cnt[m] + rank[q]] = pv0[p] + (k - own) * b + c;
                 }
-                if (!shared) own = k;
+                k++;
             }
-            w[0] = ne;
-            w[1] = nn * b;
-            w[2] = own * b;
-            w[3] = pv0[p];
-            for (uint32_t q = 0; q < ne; q++) {
-                const uint32_t e = elems[first[p] + q];
-                ep[q] = pos[e];
-                for (uint32_t j = 0; j < per; j++) {
-                    const uint32_t at = place[map[(uint64_t)e * n + j * b] / b];
-                    for (uint32_t c = 0; c < b; c++) loc[q * n + j * b + c] = (unsigned char)(at * b + c);
-                }
+            if (!shared) own = k;
+        }
+        std::sort(place, place + nn);
+        w[0] = ne;
+        w[1] = nn * b;
+        w[2] = own * b;
+        w[3] = pv0[p];
+        for (uint32_t q = 0; q < ne; q++) {
+            const uint32_t e = elems[first[p] + q];
+            ep[q] = pos[e];
+            for (uint32_t j = 0; j < per; j++) {
+                const std::pair<uint32_t, uint32_t> m(map[(uint64_t)e * n + j * b] / b, 0);
+                const uint32_t at = std::lower_bound(place, place + nn, m)->second;
+                for (uint32_t c = 0; c < b; c++) loc[q * n + j * b + c] = (unsigned char)(at * b + c);
             }
         }
     }

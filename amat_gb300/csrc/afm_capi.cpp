@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <new>
 #include <numeric>
 #include <string>
 #include <type_traits>
@@ -1384,7 +1385,11 @@ int ensure_bpatch(afm_operator* op, uint32_t nrhs, bool f32, bool* usable) {
         std::vector<uint8_t> is_bc(op->n_dofs, 0);
         for (uint32_t d : op->bc_unique) is_bc[d] = 1;
         BPatchPlanHost plan;
-        build_bpatch_plan(op->n_elem, op->n_dofs, n, op->map.data(), op->perm.data(), first, is_bc.data(), plan);
+        try {
+            build_bpatch_plan(op->n_elem, op->n_dofs, n, op->map.data(), op->perm.data(), first, is_bc.data(), plan);
+        } catch (const std::bad_alloc&) {
+            return AFM_SUCCESS;
+        }
         if (dalloc(op, &op->d_bp_hdr, std::max<size_t>(plan.hdr.size(), 16)) != cudaSuccess ||
             dalloc(op, &op->d_bp_dof, sizeof(uint32_t) * std::max<size_t>(plan.shared_dof.size(), 1)) != cudaSuccess ||
             dalloc(op, &op->d_bp_off, sizeof(uint32_t) * plan.shared_off.size()) != cudaSuccess ||
@@ -3450,6 +3455,83 @@ int afm_solve_cg_batched_mixed_device(afm_operator* op, const double* d_B, doubl
         stats->refinements = outer;
     }
     if (status != AFM_SUCCESS) return fail(status, "batched refinement stopped after %d steps", outer);
+    return ok();
+}
+
+int afm_batched_plan_host_matvec(uint32_t n_elem, uint32_t n_dofs, uint32_t n, const uint32_t* map, const double* ke,
+                                 const uint8_t* fixed, const double* u, double* v, uint32_t* n_patches) {
+    if (!map || !ke || !fixed || !u || !v || n_elem == 0) return fail(AFM_ERR_INVALID_ARG, "bad arguments");
+    if (!bpatch_supported(n, true)) return fail(AFM_NOT_IMPLEMENTED, "n = %u", n);
+    std::vector<uint32_t> offsets(n_elem + 1), m(map, map + (size_t)n_elem * n), colors, perm(n_elem);
+    for (uint32_t e = 0; e <= n_elem; e++) offsets[e] = e * n;
+    for (uint32_t d : m)
+        if (d >= n_dofs) return fail(AFM_INDEX_OUT_OF_BOUNDS, "DoF %u", d);
+    const uint32_t ncol = color_elements(n_dofs, n_elem, offsets, m, colors);
+    std::iota(perm.begin(), perm.end(), 0u);
+    std::stable_sort(perm.begin(), perm.end(), [&](uint32_t a, uint32_t b) { return colors[a] < colors[b]; });
+    std::vector<uint32_t> first(ncol + 1, 0);
+    for (uint32_t c : colors) first[c + 1]++;
+    for (uint32_t c = 0; c < ncol; c++) first[c + 1] += first[c];
+    BPatchPlanHost plan;
+    build_bpatch_plan(n_elem, n_dofs, n, m.data(), perm.data(), first, fixed, plan);
+    const BPatchGeom& g = plan.geom;
+    std::fill(v, v + n_dofs, 0.0);
+    std::vector<uint32_t> seen(n_elem, 0), rows_of(n_dofs, 0);
+    std::vector<uint8_t> filled(g.pv_rows, 0);
+    std::vector<double> pv(g.pv_rows, 0.0), vacc;
+    for (uint32_t p = 0; p < g.patches; p++) {
+        const unsigned char* h = plan.hdr.data() + (size_t)p * g.hdr_bytes;
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(h);
+        const uint32_t* rows = reinterpret_cast<const uint32_t*>(h + bpatch_rows_off());
+        const unsigned char* loc = h + bpatch_loc_off(g.max_rows);
+        const uint32_t ne = w[0], nr = w[1], own = w[2], pv0 = w[3];
+        if (ne == 0 || ne > kBPatchElems || nr > g.max_rows || nr > kBPatchRows || own > nr || pv0 + nr - own > g.pv_rows ||
+            bpatch_loc_off(g.max_rows) + ne * n > g.hdr_bytes)
+            return fail(AFM_ERR_INTERNAL, "patch %u header", p);
+        vacc.assign(nr, 0.0);
+        for (uint32_t q = 0; q < ne; q++) {
+            if (w[8 + q] >= n_elem) return fail(AFM_ERR_INTERNAL, "patch %u element %u", p, q);
+            const uint32_t e = perm[w[8 + q]];
+            seen[e]++;
+            for (uint32_t r = 0; r < n; r++) {
+                const uint32_t l = loc[q * n + r];
+                if (l >= nr || (rows[l] & kDofMask) != m[(size_t)e * n + r])
+                    return fail(AFM_ERR_INTERNAL, "patch %u element %u row %u", p, q, r);
+                double s = 0.0;
+                for (uint32_t c = 0; c < n; c++) {
+                    const uint32_t d = rows[loc[q * n + c]];
+                    if (!(d & kBcFlag)) s += ke[((size_t)e * n + r) * n + c] * u[d & kDofMask];
+                }
+                vacc[l] += s;
+            }
+        }
+        for (uint32_t r = 0; r < nr; r++) {
+            const uint32_t d = rows[r] & kDofMask;
+            if (((rows[r] & kBcFlag) != 0) != (fixed[d] != 0)) return fail(AFM_ERR_INTERNAL, "patch %u row %u flag", p, r);
+            if (r < own) {
+                if (rows_of[d]++) return fail(AFM_ERR_INTERNAL, "DoF %u is not of patch %u alone", d, p);
+                v[d] = vacc[r];
+            } else {
+                if (filled[pv0 + r - own]++) return fail(AFM_ERR_INTERNAL, "combine row %u twice", pv0 + r - own);
+                pv[pv0 + r - own] = vacc[r];
+            }
+        }
+    }
+    for (uint32_t e = 0; e < n_elem; e++)
+        if (seen[e] != 1) return fail(AFM_ERR_INTERNAL, "element %u in %u patches", e, seen[e]);
+    for (uint32_t i = 0; i < g.shared; i++) {
+        const uint32_t d = plan.shared_dof[i];
+        if (rows_of[d]++) return fail(AFM_ERR_INTERNAL, "DoF %u written twice", d);
+        double s = 0.0;
+        for (uint32_t k = plan.shared_off[i]; k < plan.shared_off[i + 1]; k++) {
+            const uint32_t x = plan.shared_idx[k];
+            if (x >= g.pv_rows || !filled[x] || (k > plan.shared_off[i] && x <= plan.shared_idx[k - 1]))
+                return fail(AFM_ERR_INTERNAL, "combine list of DoF %u", d);
+            s += pv[x];
+        }
+        v[d] = s;
+    }
+    if (n_patches) *n_patches = g.patches;
     return ok();
 }
 

@@ -421,6 +421,12 @@ int afm_patch_plan_host_matvec(uint32_t n_elem, uint32_t n_dofs, const uint32_t*
                                const double* ke, const double* u, double* v, uint32_t* n_patches,
                                uint32_t* n_patch_colors);
 
+/* The same for the patch plan of the batched products (elements of n = 24, 30
+ * or 60 DoFs, one column): fixed[d] != 0 marks constrained DoFs, whose columns
+ * read as zero. */
+int afm_batched_plan_host_matvec(uint32_t n_elem, uint32_t n_dofs, uint32_t n, const uint32_t* map, const double* ke,
+                                 const uint8_t* fixed, const double* u, double* v, uint32_t* n_patches);
+
 /* ---- assembled operator (par::aMatBased) ----------------------------------
  * The matrix aMatBased assembles through PETSc, as CSR (row_ptr[n_dofs + 1],
  * cols ascending per row, FP64 values): set_element_matrix with ADD_VALUES in
