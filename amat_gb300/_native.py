@@ -133,6 +133,8 @@ AFM_SIGNATURES = {
     "afm_matmult_bc_batched_device": (I, [P, P, P, U32, U32, P]),
     "afm_matmult_bc_batched_device_f32": (I, [P, P, P, U32, U32, P]),
     "afm_get_batch_tuning": (I, [P, U32, U32, I, P, P, P]),
+    "afm_set_batch_patches": (I, [P, I]),
+    "afm_get_batch_patches": (I, [P, U32, U32, I, P]),
     "afm_set_batch_tuning": (I, [P, U32, U32, I, I, I]),
     "afm_solve_cg_batched_device": (I, [P, P, P, U32, D, D, I, P]),
     "afm_solve_cg_batched_mixed_device": (I, [P, P, P, U32, D, D, I, D, I, P]),

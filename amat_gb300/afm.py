@@ -364,6 +364,17 @@ class aMatFree:
         check(self._lib.afm_set_batch_tuning(self._h, int(nrhs), int(ld), int(bool(f32)), int(cols_per_thread),
                                              int(rows_per_thread)), "afm_set_batch_tuning")
 
+    def set_batch_patches(self, mode):
+        """Batched products over patches: 0 never, 1 where the autotuner finds them faster, 2 wherever there is a plan."""
+        check(self._lib.afm_set_batch_patches(self._h, int(mode)), "afm_set_batch_patches")
+
+    def batch_patches(self, nrhs, ld=None, f32=False, solve=False):
+        """Whether products of this width take the patches (solve=True: those of the batched mixed solve)."""
+        p = C.c_int()
+        check(self._lib.afm_get_batch_patches(self._h, int(nrhs), int(nrhs if ld is None else ld),
+                                              2 if solve else int(bool(f32)), C.byref(p)), "afm_get_batch_patches")
+        return bool(p.value)
+
     def batch_tuning(self, nrhs, ld=None, f32=False, solve=False):
         """(columns, rows, ms) the autotuner chose; solve=True: the FP32 products of the batched mixed solve."""
         ld = nrhs if ld is None else ld

@@ -1544,6 +1544,9 @@ bool batched_tc_all(afm_operator* op, uint32_t nrhs) {
 // The project's autotuner: the first batched call for (nrhs, ld, arithmetic)
 // times every (columns per thread tile, element groups per CTA) candidate on
 // the caller's data, three runs each, and keeps the fastest for the operator.
+// With a patch plan, which beats every tile by half or more as a rule, one run
+// each; where its one run is above 7/10 of the best tile's, both are timed
+// again over several.
 // allow_tc = false leaves the tensor-core kernel out: the mixed block CG's
 // FP32 recursion takes the CUDA-core kernels, whose products are IEEE FP32
 // (the 3xTF32 products drop the lo x lo term and accumulate in the tensor
@@ -1567,7 +1570,8 @@ int batch_tuning(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, ui
             }
             return AFM_SUCCESS;
         }
-    if (int s = ensure_bpatch(op, nrhs, f32, &patch)) return s;
+    if (op->bp_mode)
+        if (int s = ensure_bpatch(op, nrhs, f32, &patch)) return s;
     // (columns, rows) of the lane tile; (0, 0): the tensor-core kernel (FP32 products)
     std::vector<std::pair<int, int>> cand = {{8, 6}, {8, 4}, {8, 2}, {4, 4}};
     if (f32 && allow_tc && batched_tc_all(op, nrhs)) cand.insert(cand.begin(), {0, 0});
@@ -1576,10 +1580,8 @@ int batch_tuning(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, ui
     cudaEventCreate(&e1);
     float best = 1e30f;
     int btr = 4, bng = 2;
-    // products of a candidate after others of it (its status); *ms is lowered to the time of one
-    // (one after one where the patch plan will most likely beat them all)
-    const int warm = patch ? 1 : 2, runs = patch ? 1 : 3;
-    auto time = [&](int ct, int rt, float* ms) {
+    // the time of one of `runs` products after `warm` others of the candidate, to *ms (its status)
+    auto time = [&](int ct, int rt, int warm, int runs, float* ms) {
         for (int r = 0; r < warm; r++)
             if (int s = enqueue_matvec_batched(op, d_V, d_U, nrhs, ld, 0, st, f32, ct, rt)) return s;
         cudaEventRecord(e0, st);
@@ -1588,25 +1590,36 @@ int batch_tuning(afm_operator* op, void* d_V, const void* d_U, uint32_t nrhs, ui
         cudaEventSynchronize(e1);
         float t = 0.f;
         cudaEventElapsedTime(&t, e0, e1);
-        *ms = std::min(*ms, t / (float)runs);
+        *ms = t / (float)runs;
         return (int)AFM_SUCCESS;
     };
     for (auto c : cand) {
         if (c.first != 0 && nrhs % (uint32_t)c.first) continue;  // a lane tile must divide the columns
-        const float before = best;
-        if (time(c.first, c.second, &best)) {
+        float ms = 0.f;
+        if (time(c.first, c.second, patch ? 1 : 2, patch ? 1 : 3, &ms)) {
             g_last_error.clear();
             continue;
         }
-        if (best < before) {
+        if (ms < best) {
+            best = ms;
             btr = c.first;
             bng = c.second;
         }
     }
     if (patch) {
-        const float tile = best;
-        if (time(kPatchTile, 0, &best)) return AFM_ERR_CUDA;
-        patch = best < tile;
+        float ms = 0.f;
+        int s = time(kPatchTile, 0, 1, 1, &ms);
+        if (!s && best < 1e30f && ms > 0.7f * best && op->bp_mode == 1) {
+            s = time(btr, bng, 1, 5, &best);
+            if (!s) s = time(kPatchTile, 0, 1, 5, &ms);
+        }
+        if (s) {
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
+            return s;
+        }
+        patch = ms < best || op->bp_mode == 2;
+        if (patch) best = ms;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -3254,21 +3267,25 @@ int afm_matmult_bc_batched_device_f32(afm_operator* op, float* d_V, const float*
     return batched_product<float>(op, d_V, d_U, nrhs, ld, 1, stream);
 }
 
+// The kept choice of afm_get_batch_tuning's (nrhs, ld, f32), or null.
+static const afm_operator::BatchTune* find_tune(const afm_operator* op, uint32_t nrhs, uint32_t ld, int f32) {
+    const int kprec = f32 ? AFM_PREC_FP32 : op->precision;
+    const uint64_t key = ((uint64_t)nrhs << 40) | ((uint64_t)ld << 8) | (uint64_t)kprec | (f32 == 2 ? 0x80u : 0u);
+    for (const auto& t : op->batch_tune)
+        if (t.key == key) return &t;
+    return nullptr;
+}
+
 int afm_get_batch_tuning(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, int* cols_per_thread,
                          int* rows_per_thread, float* ms) {
     AFM_CHECK_OP(op);
     if (f32 < 0 || f32 > 2) return fail(AFM_ERR_INVALID_ARG, "f32 %d: 0, 1 or 2", f32);
-    const int kprec = f32 ? AFM_PREC_FP32 : op->precision;
-    const uint64_t key =
-        ((uint64_t)nrhs << 40) | ((uint64_t)ld << 8) | (uint64_t)kprec | (f32 == 2 ? 0x80u : 0u);
-    for (const auto& t : op->batch_tune)
-        if (t.key == key) {
-            if (cols_per_thread) *cols_per_thread = t.tr;
-            if (rows_per_thread) *rows_per_thread = t.ng;
-            if (ms) *ms = t.ms;
-            return ok();
-        }
-    return fail(AFM_ERR_STATE, "no batched call with nrhs %u yet", nrhs);
+    const afm_operator::BatchTune* t = find_tune(op, nrhs, ld, f32);
+    if (!t) return fail(AFM_ERR_STATE, "no batched call with nrhs %u yet", nrhs);
+    if (cols_per_thread) *cols_per_thread = t->tr;
+    if (rows_per_thread) *rows_per_thread = t->ng;
+    if (ms) *ms = t->ms;
+    return ok();
 }
 
 int afm_set_batch_tuning(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, int cols_per_thread,
@@ -3293,6 +3310,23 @@ int afm_set_batch_tuning(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, 
             return ok();
         }
     op->batch_tune.push_back({key, cols_per_thread, groups_per_cta, 0.0f});
+    return ok();
+}
+
+int afm_set_batch_patches(afm_operator* op, int mode) {
+    AFM_CHECK_OP(op);
+    if (mode < 0 || mode > 2) return fail(AFM_ERR_INVALID_ARG, "batch patches mode %d (0 to 2)", mode);
+    op->bp_mode = mode;
+    op->batch_tune.clear();
+    return ok();
+}
+
+int afm_get_batch_patches(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, int* patches) {
+    AFM_CHECK_OP(op);
+    if (f32 < 0 || f32 > 2 || !patches) return fail(AFM_ERR_INVALID_ARG, "f32 %d: 0, 1 or 2", f32);
+    const afm_operator::BatchTune* t = find_tune(op, nrhs, ld, f32);
+    if (!t) return fail(AFM_ERR_STATE, "no batched call with nrhs %u yet", nrhs);
+    *patches = t->patch;
     return ok();
 }
 

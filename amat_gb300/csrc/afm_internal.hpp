@@ -495,6 +495,7 @@ struct afm_operator {
         bool patch = false;  // the patch plan beats every tile (ms is its time then)
     };
     // patch plan of the batched product (afm_batched_patch.hpp), built by the first batched call that can use it
+    int bp_mode = 1;                // afm_set_batch_patches
     int bp_state = 0;               // 0 not looked at, 1 built, -1 none
     uint32_t bp_n = 0, bp_patches = 0, bp_max_rows = 0, bp_pv_rows = 0, bp_shared = 0;
     unsigned char* d_bp_hdr = nullptr;

@@ -393,6 +393,15 @@ int afm_get_batch_tuning(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, 
  * apart from these. */
 int afm_set_batch_tuning(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, int cols_per_thread,
                          int rows_per_thread);
+/* Whether batched products may take the patches: 0 never, 1 (default) where the
+ * autotuner finds them faster than every lane tile, 2 wherever the operator has
+ * the plan. Forgets the choices made and pinned so far. Patches and launches per
+ * colour add the element products in different orders, so that a choice by time
+ * can change the last bits of a result from one run of a program to the next;
+ * 0, 2 and a pinned tile do not. */
+int afm_set_batch_patches(afm_operator* op, int mode);
+/* *patches: whether (nrhs, ld, f32), as in afm_get_batch_tuning, takes them. */
+int afm_get_batch_patches(afm_operator* op, uint32_t nrhs, uint32_t ld, int f32, int* patches);
 /* Batched Jacobi-PCG: one CG per column (own scalars and stopping test
  * ||b_j - A x_j|| <= max(rtol ||b_j||, atol)), all advanced together, the
  * iterations captured in CUDA graphs. FP64 arithmetic of the operator. ld =
