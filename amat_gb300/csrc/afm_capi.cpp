@@ -1439,7 +1439,13 @@ int enqueue_launches_batched(afm_operator* op, void* d_V, const void* d_U, uint3
     unsigned long long* const cols = op->d_usc + (captured ? kUscWords : 0) + kUscColsOffset;
     if (tr == kPatchTile) {
         if (!captured) {
-            if (op->n_unlisted) AFM_CUDA(cudaMemsetAsync(d_V, 0, (size_t)op->n_dofs * ld * vb, st));
+            // every entry that an element lists is written: zero are the rows that none lists, and padding columns (as
+            // after the launches per colour)
+            if (op->n_unlisted)
+                AFM_CUDA(cudaMemsetAsync(d_V, 0, (size_t)op->n_dofs * ld * vb, st));
+            else if (ld > nrhs)
+                AFM_CUDA(cudaMemset2DAsync(static_cast<unsigned char*>(d_V) + nrhs * vb, ld * vb, 0, (ld - nrhs) * vb,
+                                           op->n_dofs, st));
             if (!f32)
                 AFM_CUDA(launch_umax_cols(static_cast<const double*>(d_U), bc_mode ? op->d_bcmask : nullptr, op->n_dofs,
                                           nrhs, ld, cols, st));
