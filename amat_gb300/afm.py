@@ -406,6 +406,12 @@ class aMatFree:
         check(self._lib.afm_get_info(self._h, C.byref(i)), "afm_get_info")
         return {f: getattr(i, f) for f, _ in AfmInfo._fields_}
 
+    def product_cost(self):
+        """(kernels, bytes) of one product: launches, and the bytes of matrices as stored, maps and vectors."""
+        k, b = C.c_uint32(), C.c_uint64()
+        check(self._lib.afm_get_product_cost(self._h, C.byref(k), C.byref(b)), "afm_get_product_cost")
+        return k.value, b.value
+
     def colors(self):
         c = np.empty(self.info()["n_elements"], dtype=np.uint32)
         check(self._lib.afm_get_colors(self._h, _ptr(c)), "afm_get_colors")

@@ -3697,6 +3697,47 @@ int afm_patch_plan_host_matvec(uint32_t n_elem, uint32_t n_dofs, const uint32_t*
     return ok();
 }
 
+// Whether the operator's plain product (afm_matvec_device, FP32 operators: _f32) runs in one launch and the gather pass.
+static bool product_gathers(const afm_operator* op) {
+    const bool f32 = op->precision == AFM_PREC_FP32;
+    return op->gather_b && gather_pays(op, op->matfree_type != 2 && !f32 && !op->d_packed, f32 ? 4 : 8) &&
+           !(op->fused && op->fused_ok && op->precision == AFM_PREC_FP64_SPLIT);
+}
+
+int afm_get_product_cost(afm_operator* op, uint32_t* kernels, uint64_t* bytes) {
+    AFM_CHECK_OP(op);
+    if (!op->finalized) return fail(AFM_ERR_STATE, "before finalize");
+    if (!kernels || !bytes) return fail(AFM_ERR_INVALID_ARG, "null argument");
+    const bool split = op->precision == AFM_PREC_FP64_SPLIT;
+    uint32_t k = 0;
+    uint64_t ke = op->ke_bytes;
+    if (op->matfree_type == 2) {
+        k = product_gathers(op) ? 2 : (uint32_t)op->free_color_first.size() - 1;
+        ke = (uint64_t)op->n_elem * op->elem_nodes * 24;
+    } else if (op->use_patches) {
+        k = op->patch_one_launch ? 1u + (op->n_shared ? 1u : 0u) : (uint32_t)op->patch_color_first.size() - 1;
+        const Segment& s = op->segs[0];
+        if (op->d_packed) ke = (uint64_t)s.units * s.n * (s.n + 1) * kTpeWidth * 4;
+    } else {
+        const bool one = op->fused && op->fused_ok;
+        if (split) k++;  // max|u|
+        if (product_gathers(op))
+            k += 2;
+        else if (one)
+            k++;
+        if (op->d_packed) ke = 0;
+        for (const Segment& s : op->segs) {
+            if (s.units && !product_gathers(op) && !one) k++;
+            if (op->d_packed) ke += (uint64_t)s.units * split_block_bytes(s.n);
+        }
+        if (op->n_loose_rows) k++;
+    }
+    *kernels = k;
+    *bytes = ke + op->map_bytes + (op->use_patches ? op->patch_idx_bytes : 0) +
+             2ull * op->n_dofs * (op->precision == AFM_PREC_FP32 ? 4 : 8);
+    return ok();
+}
+
 int afm_get_info(afm_operator* op, afm_info* info) {
     AFM_CHECK_OP(op);
     if (!info) return fail(AFM_ERR_INVALID_ARG, "null info");
@@ -3719,7 +3760,7 @@ int afm_get_info(afm_operator* op, afm_info* info) {
     }
     info->algorithmic_bytes = alg + 2 * vb * (uint64_t)op->n_dofs;
     info->algorithmic_flops = fl;
-    uint32_t launches = 1;  // the zero fill of v, where there is one
+    uint32_t launches = 1;  // the pass before the elements (zero fill of v, max|u|), also where there is none
     if (op->matfree_type == 2 && op->finalized) {
         // matrix-free: node coordinates and the map per element instead of Ke
         info->algorithmic_bytes = (uint64_t)op->n_elem * (op->elem_nodes * 3 * 8 + (uint64_t)op->nmax * 4) +
@@ -3728,7 +3769,7 @@ int afm_get_info(afm_operator* op, afm_info* info) {
     } else if (op->use_patches) {
         launches += op->patch_one_launch ? 1u + (op->n_shared ? 1u : 0u) : (uint32_t)op->patch_color_first.size() - 1;
     } else {
-        if (op->gather_b && gather_pays(op, op->precision != AFM_PREC_FP32 && !op->d_packed, op->precision == AFM_PREC_FP32 ? 4 : 8) && !(op->fused && op->fused_ok))
+        if (product_gathers(op))
             launches += 2;  // one launch for every element and the gather pass
         else
             for (const Segment& s : op->segs)

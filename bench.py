@@ -77,15 +77,6 @@ def measured_peak():
     return 6800.0, "fallback"
 
 
-def ncu_traffic(key):
-    """DRAM bytes per matvec of the dominant kernel from the committed ncu summary, or None."""
-    p = os.path.join(ROOT, "profiles", "ncu_traffic.json")
-    if not os.path.exists(p):
-        return None
-    with open(p) as f:
-        return json.load(f).get(key)
-
-
 class ClockSampler:
     """nvidia-smi clocks and throttle reasons sampled every 200 ms."""
 
@@ -402,6 +393,7 @@ def run_ours(args, w, rank, world, local_rank):
     n = m.n_dofs
     info, ms, u_host, v, clk = measure_device(A, n, args.steps, args.warmup, world, dev, rank, True)
     ms_step = ms / args.steps
+    kernels, moved = A.product_cost()
     alg = info["algorithmic_bytes"]
     value = alg * world * args.steps / (ms * 1e-3) / 1e9
     f32 = info["precision"] == 2
@@ -425,10 +417,8 @@ def run_ours(args, w, rank, world, local_rank):
     if rank != 0:
         return None
     peak, peak_kind = measured_peak()
-    key = "%s_%s" % (args.workload, PREC_KEYS[info["precision"]])
     # the roofline counts the bytes that a product moves: symmetric element matrices are read in a packed form, so
-    # these are fewer than the whole matrices' that the metric counts
-    moved = min(alg, ncu_traffic(key) or alg)
+    # these are fewer than the whole matrices' that the metric counts (the operator says what it reads)
     achieved = moved / (ms_step * 1e-3) / 1e9
     out = {
         "metric": "AFM matvec GB/s", "value": value, "unit": "GB/s", "n_gpus": world, "steps": args.steps,
@@ -438,16 +428,14 @@ def run_ours(args, w, rank, world, local_rank):
                    "precision": PREC_KEYS[info["precision"]], "parallelism": "replicas x%d" % world,
                    "l2": l2_note(info)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": ncu_traffic(key), "peak_kind": peak_kind,
-                     "kernel": ("afm_patch_kernel, one launch per patch colour + v zero fill (%d launches/step)"
-                                if info["n_patches"] else
-                                ("afm_wpg_kernel, one launch per colour + v zero fill (%d launches/step)"
-                                 if info["n_launches"] > 3 else
-                                 "afm_wpg_kernel, one launch + gather pass (%d launches/step)"))
-                               % info["n_launches"],
+                     "frac": achieved / peak, "peak_kind": peak_kind,
+                     "kernel": "%s (%d launches/step)"
+                               % ("afm_patch_kernel" if info["n_patches"] else
+                                  "afm_wpg_kernel, one launch per colour" if kernels >= info["n_colors"] else
+                                  "afm_wpg_kernel, one launch + gather pass", kernels),
                      "algorithmic_bytes_per_step": alg, "moved_bytes_per_step": moved},
         "e2e": e2e,
-        "gpu_launches": (info["n_launches"] - 1) * args.steps,
+        "gpu_launches": kernels * args.steps,
     }
     if native:
         out["fp64_native"] = native

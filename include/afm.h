@@ -104,7 +104,9 @@ typedef struct afm_info {
     uint64_t algorithmic_bytes; /* per matvec: sum_e (n_e^2 * entry + 4 n_e) + 16 n_dofs (matrix-free:
                                    sum_e (24 nodes_e + 4 n_e) + 16 n_dofs) */
     double algorithmic_flops;   /* per matvec: sum_e 2 n_e^2 */
-    uint32_t n_launches;        /* kernel launches per matvec */
+    uint32_t n_launches;        /* launches per matvec, one pass before the elements (zero fill of v,
+                                   max|u|) counted whether the plan has it or not; see
+                                   afm_get_product_cost */
     int device;
     uint32_t n_patches;         /* small-element patches (0: colour segments) */
     uint32_t n_patch_colors;    /* colours of the patch conflict graph */
@@ -549,6 +551,11 @@ int afm_solve_cg_device_noalloc(afm_operator* op, const double* d_b, double* d_x
 /* ---- introspection ------------------------------------------------------ */
 
 int afm_get_info(afm_operator* op, afm_info* info);
+/* What one product afm_matvec_device (FP32 operators: afm_matvec_device_f32)
+ * takes: the kernels it launches, and the bytes it cannot do without as the
+ * operator stores them: element matrices in the form that it reads (whole, or
+ * packed where they are symmetric), maps or patch indices, u and v once. */
+int afm_get_product_cost(afm_operator* op, uint32_t* kernels, uint64_t* bytes);
 /* Colour of each element (n_elements entries), for checking determinism. */
 int afm_get_colors(afm_operator* op, uint32_t* colors);
 /* The operator's CUDA stream (cudaStream_t). */

@@ -58,6 +58,8 @@ def test_pairs_of_rounding(gpu, loose):
     A.set_precision(PRECISION.FP64_SPLIT)
     A.set_element_matrices(0, ke)
     A.finalize()
+    per = (A.product_cost()[1] - 16 * n_dofs) // n_elem
+    assert per == 4 * n + (22080 if loose <= 200 else 28800)
     pr = oracle.Problem(n_dofs, emap, ke, fixed, np.zeros(len(fixed)))
     size = oracle.Problem(n_dofs, emap, np.abs(ke), fixed, np.zeros(len(fixed)))
     full = torch.tensor(rng.uniform(-1, 1, n_dofs), device="cuda")
