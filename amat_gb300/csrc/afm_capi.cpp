@@ -86,7 +86,6 @@ size_t patch_smem_splitsym(const PatchPlanGeom& pg, uint32_t copy_bytes);
 cudaError_t launch_segment_splitblk(const Segment& s, const SegArgs& a, int sm_count, bool dup, bool pdl,
                                     cudaStream_t st);
 cudaError_t configure_kernels_splitblk();
-size_t segment_smem_splitblk(const Segment& s);
 size_t patch_smem_f32symc(const PatchPlanGeom& pg, uint32_t copy_bytes);
 size_t segment_smem_f32symc(const Segment& s);
 size_t patch_smem_splitsymx(const PatchPlanGeom& pg, uint32_t copy_bytes);
@@ -1801,7 +1800,7 @@ int cg_step(afm_operator* op, const CgVectors<T>& V, int k, bool inner64, cudaSt
     double* part = op->d_scalars + kScalarSets * kScalarSlots;
     uint32_t nb = 0;
     if (int s = enqueue_matmult(op, V.q, V.p, st, inner64, part, &nb)) return s;
-    if (!nb) AFM_CUDA(launch_dot(V.p, V.q, op->n_dofs, part, &nb, false, st));
+    if (!nb) AFM_CUDA(launch_dot(V.p, V.q, op->n_dofs, part, &nb, st));
     AFM_CUDA(launch_cg_iteration(V.x, V.r, V.p, V.q, V.dinv, op->n_dofs, in, out, part, nb, st));
     return AFM_SUCCESS;
 }

@@ -1225,7 +1225,7 @@ __device__ __forceinline__ void wpg_run(const SegArgs& a, const RingLayout& L, c
 
         // The group's elements in order: element ch E + jc of chunk ch, the chunks
         // grp, grp + ng, ...; positions advance by increments (no division in
-        // the loop but the slot of a new chunk).
+        // the loop).
         auto advance = [&](uint32_t& c, uint32_t& j) {
             if (++j == E) {
                 j = 0;

@@ -2,7 +2,8 @@
 // (included by the afm_mv_*.cu files, which define ARITH and LAUNCH_FN so that
 // they compile in parallel; BATCH_FN is left undefined where there is no
 // batched product, LAUNCH_FN where the arithmetic runs on patches only,
-// PATCH_FN where it does not run on them).
+// PATCH_FN where it does not run on them, SMEM_FN where nothing asks for the
+// shared memory of its segments).
 #include <algorithm>
 
 #include "afm_batched.cuh"
@@ -349,7 +350,9 @@ size_t PATCH_SMEM_FN(const PatchPlanGeom& pg, uint32_t copy_bytes) {
 #endif  // PATCH_FN
 
 #ifdef LAUNCH_FN
+#ifdef SMEM_FN
 size_t SMEM_FN(const Segment& s) { return ring_layout(s, s.unit_bytes, s.unit_bytes, false, nullptr).total(); }
+#endif
 
 #ifdef FUSED_FN
 namespace {
@@ -417,6 +420,7 @@ cudaError_t FUSED_FN(const Segment* segs, uint32_t ncol, const SegArgs& a, unsig
 }
 #endif  // FUSED_FN
 
+#ifdef SMEM_FN
 #define AFM_CAT2(a, b) a##b
 #define AFM_CAT(a, b) AFM_CAT2(a, b)
 // Launch geometry of a warp-group segment (host checks): out = chunk,
@@ -432,6 +436,7 @@ void AFM_CAT(SMEM_FN, _geom)(const Segment& s, uint64_t copy_bytes, uint64_t uni
     out[4] = G.gc;
     out[5] = L.total();
 }
+#endif  // SMEM_FN
 #endif  // LAUNCH_FN
 
 // Raises the dynamic shared-memory limit of every kernel instance on the

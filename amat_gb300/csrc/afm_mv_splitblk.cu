@@ -3,7 +3,6 @@
 // split arena.
 #define ARITH ArithSplitBlk
 #define LAUNCH_FN launch_segment_splitblk
-#define SMEM_FN segment_smem_splitblk
 #define CONFIG_FN configure_kernels_splitblk
 #define FUSED_FN launch_fused_splitblk
 #include "afm_mv_launch.inl"

@@ -121,7 +121,7 @@ extern "C" int afm_solve_cg_device_noalloc(afm_operator* op, const double* d_b, 
         double* in = sc + (it % 2) * kScalarSlots;
         double* out = sc + ((it + 1) % 2) * kScalarSlots;
         uint32_t nb = 0;
-        NA_CUDA(launch_dot(p, q, n, part, &nb, false, st));
+        NA_CUDA(launch_dot(p, q, n, part, &nb, st));
         NA_CUDA(launch_cg_iteration(d_x, r, p, q, dinv, n, in, out, part, nb, st));
         NA_CUDA(cudaMemcpyAsync(h, out, sizeof(double) * kScalarSlots, cudaMemcpyDeviceToHost, st));
         NA_CUDA(cudaStreamSynchronize(st));

@@ -763,9 +763,9 @@ uint32_t cg_blocks(size_t n) {
 }  // namespace
 
 template <typename T>
-cudaError_t launch_dot(const T* a, const T* b, size_t n, double* part, uint32_t* nb, bool pdl, cudaStream_t st) {
+cudaError_t launch_dot(const T* a, const T* b, size_t n, double* part, uint32_t* nb, cudaStream_t st) {
     *nb = red_blocks(n);
-    return launch(k_dot<T>, *nb, pdl, st, a, b, n, part);
+    return launch(k_dot<T>, *nb, false, st, a, b, n, part);
 }
 
 template <typename T>
@@ -907,7 +907,7 @@ cudaError_t launch_umax_cols(const double* U, const uint8_t* mask, size_t rows, 
     template cudaError_t launch_set_constrained<T>(T*, const T*, const uint32_t*, uint32_t, cudaStream_t);            \
     template cudaError_t launch_cg_init<T>(const T*, const T*, const T*, T*, T*, T*, size_t, double*, double*,        \
                                            cudaStream_t);                                                             \
-    template cudaError_t launch_dot<T>(const T*, const T*, size_t, double*, uint32_t*, bool, cudaStream_t);           \
+    template cudaError_t launch_dot<T>(const T*, const T*, size_t, double*, uint32_t*, cudaStream_t);                 \
     template cudaError_t launch_cg_iteration<T>(T*, T*, T*, const T*, const T*, size_t, const double*, double*,       \
                                                 double*, uint32_t, cudaStream_t);                                     \
     template cudaError_t launch_invert<T>(T*, const double*, size_t, cudaStream_t);                                   \

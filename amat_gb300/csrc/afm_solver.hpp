@@ -52,7 +52,7 @@ cudaError_t launch_cg_init(const T* b, const T* q, const T* dinv, T* r, T* z, T*
                            double* part, cudaStream_t st);
 // Partial sums of a.b, one per block (returned in *nb), for launch_cg_iteration.
 template <typename T>
-cudaError_t launch_dot(const T* a, const T* b, size_t n, double* part, uint32_t* nb, bool pdl, cudaStream_t st);
+cudaError_t launch_dot(const T* a, const T* b, size_t n, double* part, uint32_t* nb, cudaStream_t st);
 // The rest of a CG iteration after the product q = A p and the nb_pq partials
 // of p.q in part: x += alpha p, r -= alpha q, p = dinv r + beta p, in two
 // launches whose blocks each add up the partials of the launch before (so that
