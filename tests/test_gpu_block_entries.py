@@ -100,3 +100,5 @@ def test_pairs_of_rounding(gpu, loose):
     b = A.apply_bc(rng.standard_normal(n_dofs))
     sol, st = A.solve(b, rtol=1e-12, atol=0.0)[:2]
     assert np.linalg.norm(pr.matmult_bc(sol) - b) <= 1e-11 * np.linalg.norm(b)
+    sol = A.solve_mixed(b, rtol=1e-12, inner_rtol=0.1, max_outer=40)[0]
+    assert np.linalg.norm(pr.matmult_bc(sol) - b) <= 1e-11 * np.linalg.norm(b)

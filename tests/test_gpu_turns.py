@@ -128,6 +128,33 @@ def test_streams_that_come_and_go(gpu):
         assert torch.equal(o, refs[k % 2])
 
 
+@pytest.mark.parametrize("again", [False, True])
+@pytest.mark.parametrize("n", [10, 24])
+def test_product_pending_at_the_end(gpu, n, again):
+    """An operator is finalized again or destroyed while a product waits on a caller's stream: its memory is given back
+    after the product, so that what other operators put there in the meantime is not read."""
+    import torch
+    emap, ke, n_dofs, A = chain(n, 3000)
+    u = torch.tensor(np.random.default_rng(n).uniform(-1, 1, n_dofs), device="cuda")
+    ref, v = torch.empty_like(u), torch.empty_like(u)
+    A.matvec_device(ref.data_ptr(), u.data_ptr())
+    A.synchronize()
+    caller = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(caller):
+        torch.cuda._sleep(100_000_000)
+    A.matvec_device(v.data_ptr(), u.data_ptr(), caller.cuda_stream)
+    if again:
+        A.set_element_matrices(0, 2.0 * ke)
+        A.finalize()
+    else:
+        A.close()
+    other = chain(n, 3000 + n)[3]
+    other.synchronize()
+    torch.cuda.synchronize()
+    assert torch.equal(v, ref)
+
+
 @pytest.mark.parametrize("n", [24, 60])
 def test_recorded_product_beside_others(gpu, n):
     """A recorded product has u scales of its own: replayed beside products of u of another size, it keeps its bits."""
